@@ -496,21 +496,14 @@ def main():
                 "algorithmic_flops_per_call": flops, "kernel_ms_total": r_ms, "kernel_calls": r_n,
                 "share_of_step": r_ms / prof_ms if prof_ms > 0 else None}
     else:
-        # finest-level coloured y-line relaxation, FP32 complex (8 B): per
-        # sweep (4 launches) every interior point reads r once, writes e once
-        # and its e is read by the lines of the two other colours (2 x 8 B)
-        bytes_per_launch = 32.0 * cfg.kfour * cfg.ny * (cfg.nx - 2) / 4.0
+        # the finest level's way up, FP32 complex (8 B): e and r read, half as
+        # many coarse corrections read, e written
+        bytes_per_launch = 28.0 * cfg.kfour * cfg.ny * (cfg.nx - 2)
         r_ms, r_n = fam["relax0"]
-        kernel = "k_relax (finest level, one warp per y-line and mode)"
+        kernel = "k_up (finest level: prolongation and two line-relaxation sweeps of strips held in registers)"
         achieved = bytes_per_launch / (r_ms * 1e-3 / max(r_n, 1)) / 1e9 if r_n else 0.0
-        # DRAM bytes (read + write) per launch, averaged over a finest-level
-        # sweep's 4 launches like the algorithmic bytes, from an ncu capture of
-        # this workload: 1.0 MB (border lines) + 3 x 53.6 MB (centre colours) per
-        # sweep = 0.80 of the algorithmic bytes (the lines the previous colour
-        # wrote are still in L2)
-        traffic = 0.80 * bytes_per_launch if WORKLOAD["name"] == "config2" else None
         roof = {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
-                "traffic": traffic, "peak_source": peak_kind, "kernel": kernel,
+                "traffic": None, "peak_source": peak_kind, "kernel": kernel,
                 "algorithmic_bytes_per_launch": bytes_per_launch, "kernel_ms_total": r_ms, "kernel_launches": r_n,
                 "share_of_step": r_ms / prof_ms if prof_ms > 0 else None}
     line = {"metric": METRIC, "value": value, "unit": "Mpt-steps/s", "n_gpus": world, "steps": args.steps,

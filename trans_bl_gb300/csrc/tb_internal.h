@@ -224,11 +224,8 @@ int tb_plain_setup(tb_ctx* c);
 int tb_plain_tune(tb_ctx* c, int l, int itera, const int* gis, int ngis, int* best, float* best_ms);
 int tb_poisson_setup(tb_ctx* c);
 int tb_poisson_begin(tb_ctx* c, const cplx* dwzdx);
-int tb_poisson_defect_f32(tb_ctx* c, float2* r32, float2* e32, size_t elems32, unsigned long long* maxsq);
+int tb_poisson_defect_f32(tb_ctx* c, float2* r32, size_t elems32, int T, int np, unsigned long long* maxsq);
 int tb_poisson_end(tb_ctx* c);
-void tb_chunk_tables(int n, int ny, int S, const double* L1, const double* L2, const double* U1, const double* U2,
-                     const double* ID, double* out);
-__host__ __device__ inline size_t tb_poi_blk_size(int ny) { return (size_t)9 * ny + 1280; }
 int tb_poi_uy_mixed(tb_ctx* c, const cplx* dwzdx, double erro);
 // Learned first correction of the mixed solve (tb_learn.cu owns the network
 // and buffers, tb_mixed.cu the solver-side kernels).
@@ -250,7 +247,7 @@ struct LearnSolve {
     int probe = 32;              // a stage evaluates the network at least every `probe` solves
     int* gate = nullptr;         // (4, 8) and a host-read flag
 };
-// The fine-level FP32 operator of the mixed form (the operator of k_resid at
+// The fine-level FP32 operator of the mixed form (the operator of fine_resid at
 // level 0): device tables and scalars.
 struct FineOp {
     const float* coef;     // sp(7) cp(8) pp(4) lp(5) of the finest level

@@ -33,7 +33,7 @@
 // position.  The loss is what the solver judges: the defect left by the
 // correction e (the output times the output scale, on the grid's interior),
 //   mean over the crop interiors of (w_k (d0 / s - L e))^2,
-// with L the finest FP32 operator of the mixed form (k_resid's) and w_k the
+// with L the finest FP32 operator of the mixed form (fine_resid's) and w_k the
 // smallest 1/|D| of the mode, so that rows with the largest diagonal, where
 // the max defect sits, weigh most.  Adam.  Forward, backward-data and weight-gradient kernels are FP32 on the
 // CUDA cores.
@@ -262,7 +262,7 @@ __global__ void k_crops(const float* __restrict__ X, const cplx* __restrict__ fc
 }
 
 // Visit the terms (i', j', coefficient) of the finest FP32 operator at
-// interior point (i, j) of mode k, term by term as k_resid evaluates it
+// interior point (i, j) of mode k, term by term as fine_resid evaluates it
 // (defect, poisson_par.f:543-793): L e = b den + cc q2 + d ify - top e.
 template <class V>
 __device__ __forceinline__ void fine_terms(const FineOp& F, int k, int i, int j, V&& visit) {

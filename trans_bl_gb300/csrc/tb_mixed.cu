@@ -19,18 +19,13 @@
 // (1/4, 1/2, 1/4) restriction, linear prolongation) until a level has at most
 // DIRECT_MAX unknowns, which is solved exactly: its operator is inverted per
 // mode at set-up (FP64 Gauss-Jordan, stored in FP32) and applied as one
-// batched matrix-vector product.  The smoother relaxes y-lines in four
+// matrix-vector product.  The smoother relaxes y-lines in four
 // groups: the two border lines, then the centre lines by colour i mod 3.  The
 // centre stencil reaches i+-2 and the border stencil reaches 4 lines inwards,
 // so the lines of one group never read each other and a whole group is solved
-// at once, one warp per (line, mode).
-//
-// Layout: FP32 levels are stored per mode with each y-line contiguous
-// (element (i, j) of level l at off[l] + i*ptsy[l] + j), so a warp reads
-// a line and its x-neighbours with unit stride.  At 1025 x 193 x 32 modes one
-// FP32 level-0 field is 51 MB: the three FP32 arrays of the fine level fit in
-// the 129 MB L2 between sweeps.
+// at once (tb_cycle.cuh: the V-cycle's kernels and the layout of its levels).
 #include "tb_internal.h"
+#include "tb_cycle.cuh"
 #include <cmath>
 #include <cstring>
 #include <algorithm>
@@ -55,18 +50,12 @@ namespace {
 #define TB_MG_SEMI_FIRST 1
 #endif
 constexpr int NU_PRE = TB_MG_NU_PRE, NU_POST = TB_MG_NU_POST, INNER_VCYCLES = TB_MG_INNER;
-constexpr int RELAX_THREADS = 128;   // 4 warps, one line each
-#ifndef TB_RELAX_MIN_BLOCKS
-#define TB_RELAX_MIN_BLOCKS 8
-#endif
-constexpr int RELAX_MIN_BLOCKS = TB_RELAX_MIN_BLOCKS;   // resident blocks per SM the register budget allows
-constexpr int MG_MAX = 16;           // levels of the FP32 hierarchy
+constexpr int MG_MAX = mg::MAX_LEVELS;   // levels of the FP32 hierarchy
 constexpr int DIRECT_MAX = 400;      // unknowns per mode below which coarsening stops
-constexpr int DIRECT_LIMIT = 2048;   // largest directly solved level accepted
 
 struct Mixed {
-    float2 *e = nullptr, *r = nullptr, *rr = nullptr;   // per mode blocks of `elems` (line-contiguous)
-    float* tab = nullptr;     // [type][level][k] blocks of tb_poi_blk_size(ny): L1 L2 U1 U2 ID h1 h2 k1 k2 Pf Pb
+    float2 *ea = nullptr, *eb = nullptr, *r = nullptr;   // per mode blocks of `elems` (layout: tb_cycle.cuh)
+    float4* tab = nullptr;    // per mode: line-solve and residual rows of every level (mg::Cycle::tab)
     float* coef = nullptr;    // sp(7) cp(8) pp(4) lp(5) per reference level
     float* qdy2 = nullptr;    // (ny, msh)
     float* ainv = nullptr;    // (K, N, N) inverse of the coarsest operator per mode
@@ -81,189 +70,40 @@ struct Mixed {
     int* lkeep = nullptr;            // (K, 2) learned correction kept per mode, in the layout of pstate
     int* iter = nullptr;      // corrections tested so far in a recorded solve loop
     int NL = 0, N = 0;
-    int ptsx[MG_MAX], ptsy[MG_MAX], ylvl[MG_MAX], semi[MG_MAX], S[MG_MAX];
+    int ptsx[MG_MAX], ptsy[MG_MAX], ylvl[MG_MAX], semi[MG_MAX];
     double dx2[MG_MAX];
-    size_t off[MG_MAX], elems = 0;
+    size_t elems = 0;
+    mg::Cycle cyc;            // launch arguments of the V-cycle kernel
 };
 
-struct MgDev {
-    float2 *e, *r, *rr;
-    const float* tab;
+// The finest FP32 level for the kernels outside the V-cycle.
+struct FineDev {
+    float2 *e, *r;
     const float* coef;
     const float* qdy2;
-    const float* ainv;
     const double* k2b2;
     const int* state;
-    int ny, K, NL, N;
-    int ptsx[MG_MAX], ptsy[MG_MAX], ylvl[MG_MAX];
-    size_t off[MG_MAX], elems, bs;
-    float qx[MG_MAX];       // 1 / (12 dx_l^2 fac_y)
+    mg::Level L;
+    int nx, ny, K;
+    size_t elems;
+    float den;              // 1 / (12 dx^2 fac_y)
     float ify, alpha2;      // 1 / fac_y, alpha^2
 };
 
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 
-// x-stencil of the line operator without its diagonal: centre lines
-// 16(f[i-1] + f[i+1]) - (f[i-2] + f[i+2]); border lines (i = 1, mirrored at
-// i = nxl-2) 10 f[i-1] - 4 f[i+1] + 14 f[i+2] - 6 f[i+3] + f[i+4]
-// (rhs_center / rhs_border, poisson_par.f:229-540).
-__device__ __forceinline__ float2 xsum(const float2* E, int n, int i, int j, int type, int e) {
-    auto at = [&](int ii) { return E[(size_t)n * ii + j]; };
-    if (type == 0) {
-        float2 a = at(i - 2), b = at(i - 1), c = at(i + 1), d = at(i + 2);
-        return f2(16.f * (b.x + c.x) - (a.x + d.x), 16.f * (b.y + c.y) - (a.y + d.y));
-    }
-    float2 a = at(i - e), b = at(i + e), c = at(i + 2 * e), d = at(i + 3 * e), f = at(i + 4 * e);
-    return f2(10.f * a.x - 4.f * b.x + 14.f * c.x - 6.f * d.x + f.x, 10.f * a.y - 4.f * b.y + 14.f * c.y - 6.f * d.y + f.y);
-}
-
-// Relax one group of lines at level l: lines i = first + step*t, t < nlines,
-// in every active mode; e(i, :) <- line solve of L e = r with the other lines
-// frozen.  One warp per (line, mode); the pentadiagonal solve is split into
-// 32 row chunks (local recurrences, warp scan of precomputed 2x2 chunk
-// propagators, fix-up with precomputed homogeneous responses).
-template <int S>
-__global__ void __launch_bounds__(RELAX_THREADS, RELAX_MIN_BLOCKS) k_relax(MgDev M, int l, int first, int step, int nlines) {
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int gw = blockIdx.x * (RELAX_THREADS / 32) + wib;
-    const int k = gw / nlines;
-    if (k >= M.K || !M.state[2 * k]) return;   // uniform over the warp
-    const int i = first + step * (gw - k * nlines);
-    const int nxl = M.ptsx[l], n = M.ptsy[l];
-    const int type = (i == 1 || i == nxl - 2) ? 1 : 0, dir = (i == 1) ? 1 : -1;
-    extern __shared__ float2 smf[];
-    float2* g = smf + (size_t)wib * 2 * n;
-    float2* rs = g + n;
-    float2* E = M.e + (size_t)k * M.elems + M.off[l];
-    const float2* R = M.r + (size_t)k * M.elems + M.off[l] + (size_t)n * i;
-    // rows j = lane + 32 q, q < S (32 S >= n): all loads of the line issue at once
-    float2 rv[S];
-#pragma unroll
-    for (int q = 0; q < S; q++) {
-        int j = lane + 32 * q;
-        if (j < n) { g[j] = xsum(E, n, i, j, type, dir); rv[q] = R[j]; }
-    }
-    __syncwarp();
-    const float* cf = M.coef + 24 * M.ylvl[l];
-    const float sp2 = cf[1], sp3 = cf[2], cp1 = cf[7], cp2 = cf[8], cp3 = cf[9];
-    const float qx = M.qx[l];
-#pragma unroll
-    for (int q = 0; q < S; q++) {
-        int j = lane + 32 * q;
-        if (j >= n) break;
-        float2 v = f2(0.f, 0.f);
-        if (j >= 1) {
-            float2 t;
-            if (j == 1) t = f2(sp3 * g[2].x + sp2 * g[1].x, sp3 * g[2].y + sp2 * g[1].y);
-            else if (j <= n - 3)
-                t = f2(cp1 * g[j - 1].x + cp2 * g[j].x + cp3 * g[j + 1].x, cp1 * g[j - 1].y + cp2 * g[j].y + cp3 * g[j + 1].y);
-            else t = g[j];
-            float2 s = rv[q];
-            v = f2(s.x - qx * t.x, s.y - qx * t.y);
-        }
-        rs[j] = v;
-    }
-    __syncwarp();
-    const float* T = M.tab + (((size_t)type * M.NL + l) * M.K + k) * M.bs;
-    const int ny = M.ny;
-    const float *L1 = T, *L2 = T + ny, *U1 = T + 2 * ny, *U2 = T + 3 * ny, *ID = T + 4 * ny;
-    const float *h1 = T + 5 * ny, *h2 = T + 6 * ny, *k1 = T + 7 * ny, *k2 = T + 8 * ny;
-    const float* Pf = T + 9 * ny;
-    const float* Pb = Pf + 640;
-    const int r0 = lane * S, r1 = min(n, r0 + S);
-    float2 y[S];
-    float2 ym1 = f2(0.f, 0.f), ym2 = f2(0.f, 0.f);
-#pragma unroll
-    for (int s = 0; s < S; s++) {
-        int j = r0 + s;
-        if (j < r1) {
-            float2 v = rs[j];
-            float a1 = L1[j], a2 = L2[j];
-            float2 yy = f2(v.x - a2 * ym2.x - a1 * ym1.x, v.y - a2 * ym2.y - a1 * ym1.y);
-            y[s] = yy; ym2 = ym1; ym1 = yy;
-        }
-    }
-    float2 b0 = ym1, b1 = ym2;
-#pragma unroll
-    for (int d = 0, off = 1; d < 5; d++, off <<= 1) {
-        float2 o0, o1;
-        o0.x = __shfl_up_sync(0xffffffffu, b0.x, off); o0.y = __shfl_up_sync(0xffffffffu, b0.y, off);
-        o1.x = __shfl_up_sync(0xffffffffu, b1.x, off); o1.y = __shfl_up_sync(0xffffffffu, b1.y, off);
-        if (lane >= off) {
-            const float* P = Pf + (d * 32 + lane) * 4;
-            b0 = f2(b0.x + P[0] * o0.x + P[1] * o1.x, b0.y + P[0] * o0.y + P[1] * o1.y);
-            b1 = f2(b1.x + P[2] * o0.x + P[3] * o1.x, b1.y + P[2] * o0.y + P[3] * o1.y);
-        }
-    }
-    float2 Y1, Y2;
-    Y1.x = __shfl_up_sync(0xffffffffu, b0.x, 1); Y1.y = __shfl_up_sync(0xffffffffu, b0.y, 1);
-    Y2.x = __shfl_up_sync(0xffffffffu, b1.x, 1); Y2.y = __shfl_up_sync(0xffffffffu, b1.y, 1);
-    if (lane == 0) { Y1 = f2(0.f, 0.f); Y2 = f2(0.f, 0.f); }
-#pragma unroll
-    for (int s = 0; s < S; s++) {
-        int j = r0 + s;
-        if (j < r1) y[s] = f2(y[s].x + h1[j] * Y1.x + h2[j] * Y2.x, y[s].y + h1[j] * Y1.y + h2[j] * Y2.y);
-    }
-    float2 xp1 = f2(0.f, 0.f), xp2 = f2(0.f, 0.f);
-#pragma unroll
-    for (int s = S - 1; s >= 0; s--) {
-        int j = r0 + s;
-        if (j < r1) {
-            float u1 = U1[j], u2 = U2[j], id = ID[j];
-            float2 xx = f2((y[s].x - u1 * xp1.x - u2 * xp2.x) * id, (y[s].y - u1 * xp1.y - u2 * xp2.y) * id);
-            y[s] = xx; xp2 = xp1; xp1 = xx;
-        }
-    }
-    b0 = xp1; b1 = xp2;
-#pragma unroll
-    for (int d = 0, off = 1; d < 5; d++, off <<= 1) {
-        float2 o0, o1;
-        o0.x = __shfl_down_sync(0xffffffffu, b0.x, off); o0.y = __shfl_down_sync(0xffffffffu, b0.y, off);
-        o1.x = __shfl_down_sync(0xffffffffu, b1.x, off); o1.y = __shfl_down_sync(0xffffffffu, b1.y, off);
-        if (lane + off < 32) {
-            const float* P = Pb + (d * 32 + lane) * 4;
-            b0 = f2(b0.x + P[0] * o0.x + P[1] * o1.x, b0.y + P[0] * o0.y + P[1] * o1.y);
-            b1 = f2(b1.x + P[2] * o0.x + P[3] * o1.x, b1.y + P[2] * o0.y + P[3] * o1.y);
-        }
-    }
-    float2 X1, X2;
-    X1.x = __shfl_down_sync(0xffffffffu, b0.x, 1); X1.y = __shfl_down_sync(0xffffffffu, b0.y, 1);
-    X2.x = __shfl_down_sync(0xffffffffu, b1.x, 1); X2.y = __shfl_down_sync(0xffffffffu, b1.y, 1);
-    if (lane == 31) { X1 = f2(0.f, 0.f); X2 = f2(0.f, 0.f); }
-    __syncwarp();
-#pragma unroll
-    for (int s = 0; s < S; s++) {
-        int j = r0 + s;
-        if (j < r1) rs[j] = f2(y[s].x + k1[j] * X1.x + k2[j] * X2.x, y[s].y + k1[j] * X1.y + k2[j] * X2.y);
-    }
-    __syncwarp();
-    float2* Ei = E + (size_t)n * i;
-#pragma unroll
-    for (int q = 0; q < S; q++) {
-        int j = lane + 32 * q;
-        if (j >= 1 && j < n) Ei[j] = rs[j];
-    }
-}
-
-// FP32 residual rr = r - L e at level l (interior columns, rows >= 1):
-// the operator of defect (poisson_par.f:543-793) on the line-contiguous layout.
-__global__ void k_resid(MgDev M, int l) {
-    const int nxl = M.ptsx[l], n = M.ptsy[l];
-    size_t per = (size_t)(nxl - 2) * (n - 1);
-    size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (q >= per * M.K) return;
-    int k = (int)(q / per);
-    if (!M.state[2 * k]) return;
-    size_t rq = q % per;
-    int j = 1 + (int)(rq % (n - 1)), i = 1 + (int)(rq / (n - 1));
-    const int yl = M.ylvl[l];
-    const float* cf = M.coef + 24 * yl;
+// FP32 residual r - L e at the interior point (i, j) of the finest level: the
+// operator of defect (poisson_par.f:543-793) point by point (the learned
+// correction's judge and its tests; the V-cycle has its own fused form).
+__device__ __forceinline__ float2 fine_resid(const FineDev& M, int k, int i, int j) {
+    const int nxl = M.nx, n = M.ny;
+    const float* cf = M.coef;
     const float *SP = cf, *CP = cf + 7, *PP = cf + 15, *LP = cf + 19;
-    const float* Q2 = M.qdy2 + (size_t)M.ny * yl;
+    const float* Q2 = M.qdy2;
     const float k2b2 = (float)M.k2b2[k];
-    const float den = M.qx[l];
-    const float2* E = M.e + (size_t)k * M.elems + M.off[l];
-    auto f = [&](int ii, int jj) -> float2 { return E[(size_t)n * ii + jj]; };
+    const float den = M.den;
+    const float2* E = M.e + (size_t)k * M.elems;
+    auto f = [&](int ii, int jj) -> float2 { return E[mg::el(M.L, ii, jj)]; };
     auto bx = [&](int jj) -> float2 {
         if (i == 1 || i == nxl - 2) {
             int e = (i == 1) ? 1 : -1;
@@ -306,135 +146,18 @@ __global__ void k_resid(MgDev M, int l) {
         top = LP[1] * sqrtf((M.alpha2 - k2b2) * M.ify) * sqrtf(q2);
     }
     float2 fij = f(i, j);
-    size_t o = (size_t)k * M.elems + M.off[l] + (size_t)n * i + j;
-    float2 s = M.r[o];
-    M.rr[o] = f2(s.x - (b.x * den + cc.x * q2 + d.x * M.ify - top * fij.x),
-                 s.y - (b.y * den + cc.y * q2 + d.y * M.ify - top * fij.y));
+    float2 s = M.r[(size_t)k * M.elems + mg::el(M.L, i, j)];
+    return f2(s.x - (b.x * den + cc.x * q2 + d.x * M.ify - top * fij.x),
+              s.y - (b.y * den + cc.y * q2 + d.y * M.ify - top * fij.y));
 }
 
-// Full-weighting restriction of rr(l) into r(l+1) with the weights of
-// restrict (poisson_par.f:796-874); the coarse correction e(l+1) starts at 0.
-__global__ void k_restrict32(MgDev M, int l) {
-    const int nxc = M.ptsx[l + 1], nyc = M.ptsy[l + 1], nyf = M.ptsy[l];
-    size_t per = (size_t)nxc * nyc;
-    size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (q >= per * M.K) return;
-    int k = (int)(q / per);
-    if (!M.state[2 * k]) return;
-    int j = (int)((q % per) % nyc), i = (int)((q % per) / nyc);
-    size_t oc = (size_t)k * M.elems + M.off[l + 1] + (size_t)nyc * i + j;
-    M.e[oc] = f2(0.f, 0.f);
-    float2 v = f2(0.f, 0.f);
-    if (i >= 1 && i <= nxc - 2 && j >= 1) {
-        const float2* D = M.rr + (size_t)k * M.elems + M.off[l];
-        auto df = [&](int ii, int jj) { return D[(size_t)nyf * ii + jj]; };
-        int fi = 2 * i, fj = 2 * j;
-        if (j <= nyc - 2) {
-            float2 a = df(fi - 1, fj), b = df(fi + 1, fj), c = df(fi, fj - 1), d = df(fi, fj + 1), e = df(fi, fj);
-            float2 g1 = df(fi + 1, fj + 1), g2 = df(fi + 1, fj - 1), g3 = df(fi - 1, fj + 1), g4 = df(fi - 1, fj - 1);
-            v.x = 0.0625f * (2.f * (a.x + b.x + c.x + d.x) + 4.f * e.x + g1.x + g2.x + g3.x + g4.x);
-            v.y = 0.0625f * (2.f * (a.y + b.y + c.y + d.y) + 4.f * e.y + g1.y + g2.y + g3.y + g4.y);
-        } else {
-            fj = nyf - 1;
-            float2 a = df(fi - 1, fj), e = df(fi, fj), b = df(fi + 1, fj);
-            v = f2(0.25f * (a.x + 2.f * e.x + b.x), 0.25f * (a.y + 2.f * e.y + b.y));
-        }
-    }
-    M.r[oc] = v;
-}
-
-// Bilinear prolongation of e(l) added to e(l-1) (intpol, poisson_par.f:877-920).
-__global__ void k_prolong32(MgDev M, int l) {
-    const int nyc = M.ptsy[l], nxf = M.ptsx[l - 1], nyf = M.ptsy[l - 1];
-    size_t per = (size_t)nxf * nyf;
-    size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (q >= per * M.K) return;
-    int k = (int)(q / per);
-    if (!M.state[2 * k]) return;
-    int j = (int)((q % per) % nyf), i = (int)((q % per) / nyf);
-    if (i < 1 || i > nxf - 2 || j < 1) return;
-    const float2* C = M.e + (size_t)k * M.elems + M.off[l];
-    auto cv = [&](int ci, int cj) { return C[(size_t)nyc * ci + cj]; };
-    auto row = [&](int jj) -> float2 {
-        int cj = jj / 2;
-        if ((i & 1) == 0) return cv(i / 2, cj);
-        float2 a = cv(i / 2, cj), b = cv(i / 2 + 1, cj);
-        return f2(0.5f * (a.x + b.x), 0.5f * (a.y + b.y));
-    };
-    float2 t;
-    if ((j & 1) == 0) t = row(j);
-    else { float2 a = row(j + 1), b = row(j - 1); t = f2(0.5f * (a.x + b.x), 0.5f * (a.y + b.y)); }
-    float2& fe = M.e[(size_t)k * M.elems + M.off[l - 1] + (size_t)nyf * i + j];
-    fe = f2(fe.x + t.x, fe.y + t.y);
-}
-
-// x-only restriction of rr(l) into r(l+1), weights (1/4, 1/2, 1/4) in x;
-// the coarse correction e(l+1) starts at 0.
-__global__ void k_restrict_x(MgDev M, int l) {
-    const int nxc = M.ptsx[l + 1], n = M.ptsy[l + 1];
-    size_t per = (size_t)nxc * n;
-    size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (q >= per * M.K) return;
-    int k = (int)(q / per);
-    if (!M.state[2 * k]) return;
-    int j = (int)((q % per) % n), i = (int)((q % per) / n);
-    size_t oc = (size_t)k * M.elems + M.off[l + 1] + (size_t)n * i + j;
-    M.e[oc] = f2(0.f, 0.f);
-    float2 v = f2(0.f, 0.f);
-    if (i >= 1 && i <= nxc - 2 && j >= 1) {
-        const float2* D = M.rr + (size_t)k * M.elems + M.off[l] + j;
-        float2 a = D[(size_t)n * (2 * i - 1)], b = D[(size_t)n * (2 * i)], c = D[(size_t)n * (2 * i + 1)];
-        v = f2(0.25f * (a.x + 2.f * b.x + c.x), 0.25f * (a.y + 2.f * b.y + c.y));
-    }
-    M.r[oc] = v;
-}
-
-// Linear prolongation in x of e(l) added to e(l-1).
-__global__ void k_prolong_x(MgDev M, int l) {
-    const int nxf = M.ptsx[l - 1], n = M.ptsy[l - 1];
-    size_t per = (size_t)nxf * n;
-    size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (q >= per * M.K) return;
-    int k = (int)(q / per);
-    if (!M.state[2 * k]) return;
-    int j = (int)((q % per) % n), i = (int)((q % per) / n);
-    if (i < 1 || i > nxf - 2 || j < 1) return;
-    const float2* C = M.e + (size_t)k * M.elems + M.off[l] + j;
-    float2 t;
-    if ((i & 1) == 0) t = C[(size_t)n * (i / 2)];
-    else {
-        float2 a = C[(size_t)n * (i / 2)], b = C[(size_t)n * (i / 2 + 1)];
-        t = f2(0.5f * (a.x + b.x), 0.5f * (a.y + b.y));
-    }
-    float2& fe = M.e[(size_t)k * M.elems + M.off[l - 1] + (size_t)n * i + j];
-    fe = f2(fe.x + t.x, fe.y + t.y);
-}
-
-// Exact solve on the coarsest level: e = A_k^{-1} r, one warp per (mode, row).
-// Unknown q is the interior point (1 + q / (n-1), 1 + q % (n-1)).
-__global__ void k_direct(MgDev M) {
-    const int lane = threadIdx.x & 31;
-    const long gw = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int N = M.N;
-    const int k = (int)(gw / N);
-    if (k >= M.K || !M.state[2 * k]) return;
-    const int p = (int)(gw - (long)k * N);
-    const int l = M.NL - 1, n = M.ptsy[l], m = n - 1;
-    const float* A = M.ainv + ((size_t)k * N + p) * N;
-    const float2* R = M.r + (size_t)k * M.elems + M.off[l];
-    float ax = 0.f, ay = 0.f;
-    for (int q = lane; q < N; q += 32) {
-        float a = A[q];
-        float2 v = R[(size_t)n * (1 + q / m) + 1 + q % m];
-        ax = fmaf(a, v.x, ax);
-        ay = fmaf(a, v.y, ay);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        ax += __shfl_xor_sync(0xffffffffu, ax, o);
-        ay += __shfl_xor_sync(0xffffffffu, ay, o);
-    }
-    if (lane == 0) M.e[(size_t)k * M.elems + M.off[l] + (size_t)n * (1 + p / m) + 1 + p % m] = f2(ax, ay);
+// The residual of one mode into out, line-contiguous (nx, ny).
+__global__ void k_fine_resid(FineDev M, int k, float2* out) {
+    const size_t per = (size_t)(M.nx - 2) * (M.ny - 1);
+    const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (q >= per) return;
+    const int j = 1 + (int)(q % (M.ny - 1)), i = 1 + (int)(q / (M.ny - 1));
+    out[(size_t)M.ny * i + j] = fine_resid(M, k, i, j);
 }
 
 // Warm start of one stage's solve from its history h0 (previous step), h1
@@ -489,8 +212,8 @@ __global__ void k_extrap_inc(cplx* fc, size_t elems64, cplx* h0, cplx* h1, const
 // ---- learned first correction (network and training in tb_learn.cu) -------
 // Per mode maxima over both parts of |v1| and |v1 - v2| (history,
 // x-contiguous) and of |D^-1 d0| (d0: the FP32 copy r of the FP64 defect of
-// the guess, line-contiguous), as float bits in scl (K, 3).
-__global__ void k_learn_scale(MgDev M, const cplx* h0, const cplx* h1, const int* valid, unsigned* scl, const float* invD,
+// the guess), as float bits in scl (K, 3).
+__global__ void k_learn_scale(FineDev M, const cplx* h0, const cplx* h1, const int* valid, unsigned* scl, const float* invD,
                               int nx) {
     if (*valid < 2) return;
     const int k = blockIdx.y, ny = M.ny;
@@ -500,8 +223,9 @@ __global__ void k_learn_scale(MgDev M, const cplx* h0, const cplx* h1, const int
         const cplx u = h0[(size_t)k * per + q], w = h1[(size_t)k * per + q];
         a = fmaxf(a, fmaxf(fabsf((float)u.x), fabsf((float)u.y)));
         b = fmaxf(b, fmaxf(fabsf((float)(u.x - w.x)), fabsf((float)(u.y - w.y))));
-        const float2 r = M.r[(size_t)k * M.elems + M.off[0] + q];   // point (q / ny, q % ny)
-        d = fmaxf(d, invD[(size_t)k * ny + q % ny] * fmaxf(fabsf(r.x), fabsf(r.y)));
+        const int i = (int)(q % nx), j = (int)(q / nx);
+        const float2 r = M.r[(size_t)k * M.elems + mg::el(M.L, i, j)];
+        d = fmaxf(d, invD[(size_t)k * ny + j] * fmaxf(fabsf(r.x), fabsf(r.y)));
     }
     for (int o = 16; o > 0; o >>= 1) {
         a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
@@ -517,7 +241,7 @@ __global__ void k_learn_scale(MgDev M, const cplx* h0, const cplx* h1, const int
 
 // The network's input planes X (2K, 4, nx, ny) and the history shift
 // h1 <- h0 that k_extrap leaves to this kernel when the network runs.
-__global__ void k_learn_prep(MgDev M, const cplx* h0, cplx* h1, const int* valid, const float* scl, const float* invD,
+__global__ void k_learn_prep(FineDev M, const cplx* h0, cplx* h1, const int* valid, const float* scl, const float* invD,
                              const float* mfeat, float* X, int nx) {
     const int nv = *valid;
     if (nv == 0) return;
@@ -548,7 +272,7 @@ __global__ void k_learn_prep(MgDev M, const cplx* h0, cplx* h1, const int* valid
         const int i = i0 + r, j = j0 + threadIdx.x;
         if (i >= nx || j >= ny) continue;
         const float2 a = t0[threadIdx.x][r], b = t1[threadIdx.x][r];
-        const float2 d = M.r[(size_t)k * M.elems + M.off[0] + (size_t)ny * i + j];
+        const float2 d = M.r[(size_t)k * M.elems + mg::el(M.L, i, j)];
         const float sj = invD[(size_t)k * ny + j] * id, mf = mfeat[(size_t)k * ny + j];
         const size_t o = (size_t)ny * i + j;
         Xr[o] = a.x * iv; Xr[per + o] = b.x * ii; Xr[2 * per + o] = d.x * sj; Xr[3 * per + o] = mf;
@@ -557,7 +281,7 @@ __global__ void k_learn_prep(MgDev M, const cplx* h0, cplx* h1, const int* valid
 }
 
 // Candidate correction e = max|v1 - v2| * network output on the fine interior.
-__global__ void k_learn_emit(MgDev M, const float* out, const float* scl, const int* valid, int nx) {
+__global__ void k_learn_emit(FineDev M, const float* out, const float* scl, const int* valid, int nx) {
     if (*valid < 2) return;
     const int ny = M.ny;
     const size_t per = (size_t)(nx - 2) * (ny - 1), img = (size_t)nx * ny;
@@ -568,18 +292,18 @@ __global__ void k_learn_emit(MgDev M, const float* out, const float* scl, const 
     const int j = 1 + (int)(rq % (ny - 1)), i = 1 + (int)(rq / (ny - 1));
     const float s = scl[3 * k + 1];
     const size_t o = (size_t)ny * i + j;
-    M.e[(size_t)k * M.elems + M.off[0] + o] = f2(s * out[(size_t)(2 * k) * img + o], s * out[(size_t)(2 * k + 1) * img + o]);
+    M.e[(size_t)k * M.elems + mg::el(M.L, i, j)] = f2(s * out[(size_t)(2 * k) * img + o], s * out[(size_t)(2 * k + 1) * img + o]);
 }
 
 // max |r - L e|^2 per mode (blockIdx.y) over the fine interior, float bits.
-__global__ void k_learn_judge(MgDev M, unsigned* jmax, const int* valid, int nx) {
+__global__ void k_learn_judge(FineDev M, unsigned* jmax, const int* valid, int nx) {
     if (*valid < 2) return;
     const int k = blockIdx.y, ny = M.ny;
     const size_t per = (size_t)(nx - 2) * (ny - 1);
     float m = 0.f;
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < per; q += (size_t)gridDim.x * blockDim.x) {
         const int j = 1 + (int)(q % (ny - 1)), i = 1 + (int)(q / (ny - 1));
-        const float2 v = M.rr[(size_t)k * M.elems + M.off[0] + (size_t)ny * i + j];
+        const float2 v = fine_resid(M, k, i, j);
         m = fmaxf(m, v.x * v.x + v.y * v.y);
     }
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -645,26 +369,14 @@ __global__ void k_learn_keep(unsigned long long* maxsq, unsigned* jmax, int* kee
 __global__ void k_hist_count(int* valid) { *valid = min(*valid + 1, 2); }
 
 // u += e on the interior of the FP64 fine level (fc layout: x-contiguous).
-__global__ void k_apply(MgDev M, cplx* fc, size_t elems64, int nx, int ny) {
-    __shared__ float2 tile[32][33];
+__global__ void k_apply(FineDev M, cplx* fc, size_t elems64) {
     const int k = blockIdx.z;
     if (!M.state[2 * k]) return;
-    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        int i = i0 + r, j = j0 + threadIdx.x;
-        float2 v = f2(0.f, 0.f);
-        if (i < nx && j < ny) v = M.e[(size_t)k * M.elems + M.off[0] + (size_t)ny * i + j];
-        tile[threadIdx.x][r] = v;
-    }
-    __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        int i = i0 + threadIdx.x, j = j0 + r;
-        if (i >= 1 && i <= nx - 2 && j >= 1 && j < ny) {
-            float2 e = tile[r][threadIdx.x];
-            cplx& u = fc[(size_t)k * elems64 + (size_t)i + (size_t)nx * j];
-            u = make_double2(u.x + (double)e.x, u.y + (double)e.y);
-        }
-    }
+    const int i = 1 + blockIdx.x * 128 + threadIdx.x, j = 1 + blockIdx.y;
+    if (i > M.nx - 2) return;
+    const float2 e = M.e[(size_t)k * M.elems + mg::el(M.L, i, j)];
+    cplx& u = fc[(size_t)k * elems64 + (size_t)i + (size_t)M.nx * j];
+    u = make_double2(u.x + (double)e.x, u.y + (double)e.y);
 }
 
 // Per-mode test of the FP64 defect (max |d| over the interior, as
@@ -709,30 +421,21 @@ __global__ void __launch_bounds__(CHECK_THREADS) k_check_loop(unsigned long long
 
 Mixed* get(tb_ctx* c) { return static_cast<Mixed*>(c->mixed); }
 
-MgDev make(tb_ctx* c) {
+FineDev make(tb_ctx* c) {
     Mixed* m = get(c);
-    MgDev M;
+    FineDev M;
     std::memset(&M, 0, sizeof M);
-    M.e = m->e; M.r = m->r; M.rr = m->rr; M.tab = m->tab; M.coef = m->coef; M.qdy2 = m->qdy2; M.ainv = m->ainv;
+    M.e = m->eb; M.r = m->r;
+    M.coef = m->coef + 24 * m->ylvl[0];
+    M.qdy2 = m->qdy2 + (size_t)c->g.ny * m->ylvl[0];
     M.k2b2 = c->k2b2; M.state = c->pstate;
-    M.ny = c->g.ny; M.K = c->g.K; M.NL = m->NL; M.N = m->N;
-    for (int l = 0; l < m->NL; l++) {
-        M.ptsx[l] = m->ptsx[l]; M.ptsy[l] = m->ptsy[l]; M.ylvl[l] = m->ylvl[l]; M.off[l] = m->off[l];
-        M.qx[l] = (float)(1.0 / (12.0 * m->dx2[l] * c->cfg.fac_y));
-    }
+    M.L = m->cyc.lv[0];
     M.elems = m->elems;
-    M.bs = tb_poi_blk_size(c->g.ny);
+    M.nx = c->g.nx; M.ny = c->g.ny; M.K = c->g.K;
+    M.den = (float)(1.0 / (12.0 * m->dx2[0] * c->cfg.fac_y));
     M.ify = (float)(1.0 / c->cfg.fac_y);
     M.alpha2 = (float)(c->cfg.alpha * c->cfg.alpha);
     return M;
-}
-
-// Rows per lane of the line solve: the smallest instantiated S with 32 S >= n.
-int pick_S(int n) {
-    static const int opts[] = {2, 3, 4, 5, 6, 7, 8, 10, 12, 16};
-    for (int s : opts)
-        if (32 * s >= n) return s;
-    return 16;
 }
 
 template <class T>
@@ -827,72 +530,173 @@ bool coarse_inverse(const HostOp& op, int N, float* out) {
     return true;
 }
 
-int launch_relax(tb_ctx* c, const MgDev& M, int S, int l, int first, int step, int nlines) {
-    cudaEvent_t p0 = nullptr;
-    int r;
-    if (l == 0 && (r = tb_prof_begin(c, PROF_RELAX0, &p0))) return r;
-    int nw = nlines * c->g.K;
-    unsigned nb = tb_blocks((size_t)nw, RELAX_THREADS / 32);
-    size_t smem = (size_t)(RELAX_THREADS / 32) * 2 * M.ptsy[l] * sizeof(float2);
-    cudaStream_t st = c->stream;
-    switch (S) {
-        case 2: k_relax<2><<<nb, RELAX_THREADS, smem, st>>>(M, l, first, step, nlines); break;
-        case 3: k_relax<3><<<nb, RELAX_THREADS, smem, st>>>(M, l, first, step, nlines); break;
-        case 4: k_relax<4><<<nb, RELAX_THREADS, smem, st>>>(M, l, first, step, nlines); break;
-        case 5: k_relax<5><<<nb, RELAX_THREADS, smem, st>>>(M, l, first, step, nlines); break;
-        case 6: k_relax<6><<<nb, RELAX_THREADS, smem, st>>>(M, l, first, step, nlines); break;
-        case 7: k_relax<7><<<nb, RELAX_THREADS, smem, st>>>(M, l, first, step, nlines); break;
-        case 8: k_relax<8><<<nb, RELAX_THREADS, smem, st>>>(M, l, first, step, nlines); break;
-        case 10: k_relax<10><<<nb, RELAX_THREADS, smem, st>>>(M, l, first, step, nlines); break;
-        case 12: k_relax<12><<<nb, RELAX_THREADS, smem, st>>>(M, l, first, step, nlines); break;
-        default: k_relax<16><<<nb, RELAX_THREADS, smem, st>>>(M, l, first, step, nlines); break;
-    }
+int apply(tb_ctx* c, const FineDev& M) {
+    k_apply<<<dim3(tb_blocks(c->g.nx - 2, 128), c->g.ny - 1, c->g.K), 128, 0, c->stream>>>(M, c->pfc, c->g.lvl_elems);
     TB_CHECK_LAUNCH(c);
-    return l == 0 ? tb_prof_end(c, PROF_RELAX0, p0) : TB_OK;
+    return TB_OK;
 }
 
-// One relaxation sweep at level l: border lines, then centre colours 0, 1, 2.
-int sweep(tb_ctx* c, const MgDev& M, int l) {
+int defect(tb_ctx* c) {
     Mixed* m = get(c);
-    int nxl = m->ptsx[l], r;
+    return tb_poisson_defect_f32(c, m->r, m->elems, m->cyc.lv[0].T, m->cyc.lv[0].np, m->maxsq);
+}
+
+template <int S>
+int launch_strip(tb_ctx* c, const mg::Cycle& M, int l, int up, int from) {
+    const mg::Level& L = M.lv[l];
+    const size_t smem = mg::strip_bytes(L);
+    const dim3 grid((unsigned)(up ? L.up : L.down), (unsigned)M.K);
+    if (up) mg::k_up<S><<<grid, mg::NT, smem, c->stream>>>(M, l);
+    else mg::k_down<S><<<grid, mg::NT, smem, c->stream>>>(M, l, from);
+    TB_CHECK_LAUNCH(c);
+    return TB_OK;
+}
+int strip(tb_ctx* c, const mg::Cycle& M, int l, int up, int from) {
+    cudaEvent_t p0 = nullptr;
+    int r;
+    if (l == 0 && up && (r = tb_prof_begin(c, PROF_RELAX0, &p0))) return r;
+    switch (M.lv[l].S) {
+        case 2: r = launch_strip<2>(c, M, l, up, from); break;
+        case 4: r = launch_strip<4>(c, M, l, up, from); break;
+        case 5: r = launch_strip<5>(c, M, l, up, from); break;
+        case 7: r = launch_strip<7>(c, M, l, up, from); break;
+        case 9: r = launch_strip<9>(c, M, l, up, from); break;
+        case 13: r = launch_strip<13>(c, M, l, up, from); break;
+        case 17: r = launch_strip<17>(c, M, l, up, from); break;
+        default: r = launch_strip<33>(c, M, l, up, from); break;
+    }
+    if (r) return r;
+    return l == 0 && up ? tb_prof_end(c, PROF_RELAX0, p0) : TB_OK;
+}
+// the largest dynamic shared memory any context may ask of the cycle's kernels
+template <int S>
+int strip_attr() {
+    TB_CUDA(cudaFuncSetAttribute(mg::k_down<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    TB_CUDA(cudaFuncSetAttribute(mg::k_up<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    return TB_OK;
+}
+int cycle_attrs() {
+    int r;
+    if ((r = strip_attr<2>()) || (r = strip_attr<4>()) || (r = strip_attr<5>()) || (r = strip_attr<7>()) || (r = strip_attr<9>()) ||
+        (r = strip_attr<13>()) || (r = strip_attr<17>()) || (r = strip_attr<33>()))
+        return r;
+    return TB_OK;
+}
+
+// The V-cycles of one correction.
+int vcycles(tb_ctx* c) {
+    Mixed* m = get(c);
     cudaEvent_t ps = nullptr;
+    int r;
     if ((r = tb_prof_begin(c, PROF_SOR, &ps))) return r;
-    if ((r = launch_relax(c, M, m->S[l], l, 1, nxl - 3, 2))) return r;
-    for (int col = 0; col < 3; col++) {
-        int first = 2 + col;
-        if (first > nxl - 3) break;
-        int nl = (nxl - 3 - first) / 3 + 1;
-        if ((r = launch_relax(c, M, m->S[l], l, first, 3, nl))) return r;
+    mg::Cycle M = m->cyc;
+    M.state = c->pstate;
+    const int bot = M.NL - 1;
+    for (int v = 0; v < INNER_VCYCLES; v++) {
+        for (int l = 0; l < bot; l++)
+            if ((r = strip(c, M, l, 0, v > 0 && l == 0))) return r;
+        mg::k_direct<<<dim3(tb_blocks(M.N, 4 * mg::NW), M.K), mg::NT, 0, c->stream>>>(M);
+        TB_CHECK_LAUNCH(c);
+        for (int l = bot - 1; l >= 0; l--)
+            if ((r = strip(c, M, l, 1, 0))) return r;
     }
     return tb_prof_end(c, PROF_SOR, ps);
 }
 
-int vcycle(tb_ctx* c, const MgDev& M) {
-    Mixed* m = get(c);
-    const int K = c->g.K, NL = m->NL;
-    int r;
-    for (int l = 0; l < NL - 1; l++) {
-        for (int s = 0; s < NU_PRE; s++)
-            if ((r = sweep(c, M, l))) return r;
-        size_t per = (size_t)(m->ptsx[l] - 2) * (m->ptsy[l] - 1) * K;
-        k_resid<<<tb_blocks(per, 256), 256, 0, c->stream>>>(M, l);
-        TB_CHECK_LAUNCH(c);
-        size_t pc = (size_t)m->ptsx[l + 1] * m->ptsy[l + 1] * K;
-        if (m->semi[l]) k_restrict_x<<<tb_blocks(pc, 256), 256, 0, c->stream>>>(M, l);
-        else k_restrict32<<<tb_blocks(pc, 256), 256, 0, c->stream>>>(M, l);
-        TB_CHECK_LAUNCH(c);
+// A float4 table of doubled coefficients: pair q of the row at out.
+void put_pairs(float4* out, const double* v, int n) {
+    for (int q = 0; q < n; q += 2) out[q / 2] = make_float4((float)v[q], (float)v[q], (float)v[q + 1], (float)v[q + 1]);
+}
+
+// Line-solve rows of one level, line type and mode (mg::Cycle::tab): per row
+// the weights of the right-hand side's x-stencil sums (-qx and the sums' unit
+// folded in), the forward recurrence, the chunk responses and the backward
+// recurrence (1/D folded in), then the 2x2 propagators (mg::MATS per direction).
+// Row 0 (Dirichlet) and the pad rows hold zeros.
+void line_tables(int n, int S, double unit, double qx, const double* cf, const double* L1, const double* L2, const double* U1,
+                 const double* U2, const double* ID, float4* out) {
+    std::vector<double> h1(n), h2(n), k1(n), k2(n);
+    double Mf[mg::NW][4], Mb[mg::NW][4];
+    for (int t = 0; t < mg::NW; t++) {
+        const int r0 = std::min(n, t * S), r1 = std::min(n, r0 + S);
+        for (int u = 0; u < 2; u++) {
+            double ym1 = (u == 0) ? 1.0 : 0.0, ym2 = (u == 0) ? 0.0 : 1.0;
+            for (int j = r0; j < r1; j++) {
+                const double y = j == 0 ? 0.0 : -L2[j] * ym2 - L1[j] * ym1;
+                (u == 0 ? h1 : h2)[j] = y;
+                ym2 = ym1; ym1 = y;
+            }
+            Mf[t][u] = ym1; Mf[t][2 + u] = ym2;
+        }
+        for (int u = 0; u < 2; u++) {
+            double xp1 = (u == 0) ? 1.0 : 0.0, xp2 = (u == 0) ? 0.0 : 1.0;
+            for (int j = r1 - 1; j >= r0; j--) {
+                const double x = j == 0 ? 0.0 : (-U1[j] * xp1 - U2[j] * xp2) * ID[j];
+                (u == 0 ? k1 : k2)[j] = x;
+                xp2 = xp1; xp1 = x;
+            }
+            Mb[t][u] = xp1; Mb[t][2 + u] = xp2;
+        }
     }
-    k_direct<<<tb_blocks((size_t)K * m->N, 8), 256, 0, c->stream>>>(M);
-    TB_CHECK_LAUNCH(c);
-    for (int l = NL - 1; l >= 1; l--) {
-        size_t pf = (size_t)m->ptsx[l - 1] * m->ptsy[l - 1] * K;
-        if (m->semi[l - 1]) k_prolong_x<<<tb_blocks(pf, 256), 256, 0, c->stream>>>(M, l);
-        else k_prolong32<<<tb_blocks(pf, 256), 256, 0, c->stream>>>(M, l);
-        TB_CHECK_LAUNCH(c);
-        for (int s = 0; s < NU_POST; s++)
-            if ((r = sweep(c, M, l - 1))) return r;
+    // per direction, in the order the carry takes: the chunks' propagators, the
+    // products of the chunks before each one in its group of four, the groups' products
+    for (int dir = 0; dir < 2; dir++) {
+        float4* prop = out + (size_t)mg::ROW4 * mg::NW * S + dir * 2 * mg::MATS;
+        double acc[4] = {1, 0, 0, 1};
+        for (int v = 0; v < mg::NW; v++) {
+            const double* m = dir ? Mb[mg::NW - 1 - v] : Mf[v];
+            if (v % 4 == 0) { acc[0] = acc[3] = 1.0; acc[1] = acc[2] = 0.0; }
+            put_pairs(prop + 2 * v, m, 4);
+            put_pairs(prop + 2 * (mg::NW + v), acc, 4);
+            const double a0 = m[0] * acc[0] + m[1] * acc[2], a1 = m[0] * acc[1] + m[1] * acc[3];
+            const double a2 = m[2] * acc[0] + m[3] * acc[2], a3 = m[2] * acc[1] + m[3] * acc[3];
+            acc[0] = a0; acc[1] = a1; acc[2] = a2; acc[3] = a3;
+            if (v % 4 == 3) put_pairs(prop + 2 * (2 * mg::NW + v / 4), acc, 4);
+        }
     }
-    return TB_OK;
+    for (int j = 1; j < n; j++) {
+        double w[3] = {0.0, 0.0, 0.0};
+        if (j == 1) { w[1] = -qx * cf[1]; w[2] = -qx * cf[2]; }
+        else if (j <= n - 3) for (int q = 0; q < 3; q++) w[q] = -qx * cf[7 + q];
+        else w[1] = -qx;
+        const double row[12] = {unit * w[0], unit * w[1], unit * w[2], -L1[j], -L2[j], ID[j] * h1[j], ID[j] * h2[j],
+                                -U1[j] * ID[j], -U2[j] * ID[j], ID[j], k1[j], k2[j]};
+        put_pairs(out + (size_t)mg::ROW4 * j, row, 12);
+    }
+}
+
+// Residual rows of one level and mode: -16 w1[-1..1] of the x-stencil sums and
+// -w2[-2..2] of the values, the centre stencil's diagonal (-30) folded into w2.
+void residual_rows(int n, double den, double ify, double k2b2, double alpha2, const double* cf, const double* Q2,
+                   float4* out) {
+    const double *SP = cf, *CP = cf + 7, *PP = cf + 15, *LP = cf + 19;
+    for (int j = 1; j < n; j++) {
+        double w[8] = {0, 0, 0, 0, 0, 0, 0, 0}, *w1 = w, *w2 = w + 3;
+        const double kk = k2b2 * ify;
+        if (j == 1) {
+            const double q2 = Q2[0];
+            w1[1] = den * SP[1]; w1[2] = den * SP[2];
+            for (int q = 0; q < 4; q++) w2[1 + q] = q2 * SP[3 + q];
+            w2[2] += kk * SP[1]; w2[3] += kk * SP[2];
+        } else if (j <= n - 3) {
+            const double q2 = Q2[j - 2];
+            for (int q = 0; q < 3; q++) w1[q] = den * CP[q];
+            for (int q = 0; q < 5; q++) w2[q] = q2 * CP[3 + q];
+            for (int q = 0; q < 3; q++) w2[1 + q] += kk * CP[q];
+        } else if (j == n - 2) {
+            const double q2 = Q2[j - 1];
+            w1[1] = den;
+            w2[3] = q2 * PP[3]; w2[2] = q2 * PP[2] + kk; w2[1] = q2 * PP[1];
+        } else {
+            const double q2 = Q2[j - 2];
+            w1[1] = den;
+            w2[2] = q2 * LP[2] + kk - LP[1] * std::sqrt((alpha2 - k2b2) * ify) * std::sqrt(q2);
+            w2[1] = q2 * LP[3]; w2[0] = q2 * LP[4];
+        }
+        for (int q = 0; q < 3; q++) w2[1 + q] -= 30.0 * w1[q];
+        for (int q = 0; q < 8; q++) w[q] *= q < 3 ? -16.0 : -1.0;   // the x-stencil sums are in units of 16
+        put_pairs(out + (size_t)mg::RES4 * j, w, 8);
+    }
 }
 
 }  // namespace
@@ -937,18 +741,40 @@ int tb_mixed_setup(tb_ctx* c) {
         return TB_ERR_ARG;
     }
     m->N = (m->ptsx[lc] - 2) * (m->ptsy[lc] - 1);
-    if (m->N > DIRECT_LIMIT) {
-        tb_set_error("mixed form: coarsest level has %d unknowns per mode (limit %d); raise msh", m->N, DIRECT_LIMIT);
+    if (m->N > mg::DIRECT_LIMIT) {
+        tb_set_error("mixed form: coarsest level has %d unknowns per mode (limit %d); raise msh", m->N, mg::DIRECT_LIMIT);
         return TB_ERR_ARG;
     }
+    mg::Cycle& cy = m->cyc;
+    std::memset(&cy, 0, sizeof cy);
+    cy.nu_pre = NU_PRE; cy.nu_post = NU_POST;
     size_t off = 0;
-    for (int l = 0; l < NL; l++) { m->off[l] = off; off += (size_t)m->ptsx[l] * m->ptsy[l]; m->S[l] = pick_S(m->ptsy[l]); }
-    m->elems = off;
+    int t4 = 0;   // tables per mode
+    for (int l = 0; l < NL; l++) {
+        mg::Level& L = cy.lv[l];
+        L.nx = m->ptsx[l]; L.n = m->ptsy[l]; L.semi = m->semi[l];
+        L.S = mg::pick_rows(L.n);
+        const int Tn = L.nx / 3 + 1;   // elements of a colour plane
+        L.T = (Tn + 3) & ~3;
+        L.np = mg::NW * L.S + 2;
+        L.off = (int)off;
+        off += (size_t)3 * L.np * L.T;
+        L.down = mg::strips(Tn, NU_PRE, 1);
+        L.up = mg::strips(Tn, NU_POST, 0);
+        if (l < NL - 1) { L.tab = t4; t4 += mg::level4(L); }
+        if (off > 0x7fffffffu) { tb_set_error("mixed form: grid too large for the FP32 hierarchy"); return TB_ERR_ARG; }
+    }
+    cy.tab4 = t4;
+    cy.elems = m->elems = off;
+    cy.K = K; cy.NL = NL; cy.N = m->N;
+    int r;
+    if ((r = cycle_attrs())) return r;
     size_t w = (size_t)K * m->elems;
-    for (float2** p : {&m->e, &m->r, &m->rr}) {
+    for (float2** p : {&m->ea, &m->eb, &m->r}) {
         TB_CUDA(cudaMalloc(p, w * sizeof(float2)));
         TB_CUDA(cudaMemset(*p, 0, w * sizeof(float2)));
     }
+    cy.ea = m->ea; cy.eb = m->eb; cy.r = m->r;
     TB_CUDA(cudaMalloc(&m->maxsq, K * sizeof(unsigned long long)));
     TB_CUDA(cudaMemset(m->maxsq, 0, K * sizeof(unsigned long long)));
     TB_CUDA(cudaMalloc(&m->hvalid, 4 * sizeof(int)));
@@ -960,24 +786,6 @@ int tb_mixed_setup(tb_ctx* c) {
     if (c->cfg.warm_start)
         for (auto& h : m->hist)
             for (cplx*& p : h) TB_CUDA(cudaMalloc(&p, tb_n3(c) * sizeof(cplx)));
-    // line-solve tables per (type, level, mode): band5 factors of the level's
-    // y-line matrix and chunk tables for this form's rows per lane, in FP32
-    const size_t bs = tb_poi_blk_size(ny);
-    std::vector<float> t32((size_t)2 * NL * K * bs, 0.f);
-    std::vector<double> a, blk(bs);
-    for (int type = 0; type < 2; type++)
-        for (int l = 0; l < NL; l++)
-            for (int k = 0; k < K; k++) {
-                int n = m->ptsy[l];
-                std::fill(blk.begin(), blk.end(), 0.0);
-                tb_poisson_band_matrix_dx(c, type, m->ylvl[l] + 1, k + 1, m->dx2[l], a);
-                tb_band5_factor(n, a, &blk[0], &blk[ny], &blk[2 * ny], &blk[3 * ny], &blk[4 * ny]);
-                tb_chunk_tables(n, ny, m->S[l], &blk[0], &blk[ny], &blk[2 * ny], &blk[3 * ny], &blk[4 * ny], &blk[5 * ny]);
-                float* D = &t32[(((size_t)type * NL + l) * K + k) * bs];
-                for (size_t q = 0; q < bs; q++) D[q] = (float)blk[q];
-            }
-    int r;
-    if ((r = upl(&m->tab, t32))) return r;
     const double* blob = c->coefs.data();
     std::vector<double> cf64((size_t)24 * msh);
     for (int l = 0; l < msh; l++) {   // sp_poi(7,msh) cp_poi(8,msh) pp_poi(4,msh) lp_poi(5,msh) from blob[83]
@@ -986,6 +794,27 @@ int tb_mixed_setup(tb_ctx* c) {
         for (int q = 0; q < 4; q++) cf64[24 * l + 15 + q] = blob[83 + 15 * msh + 4 * l + q];
         for (int q = 0; q < 5; q++) cf64[24 * l + 19 + q] = blob[83 + 19 * msh + 5 * l + q];
     }
+    // line-solve tables per mode, line type and level (band5 factors of the
+    // level's y-line matrix and chunk tables) and residual rows, in FP32
+    std::vector<float4> t32((size_t)K * cy.tab4, make_float4(0.f, 0.f, 0.f, 0.f));
+    std::vector<double> a, L1(ny), L2(ny), U1(ny), U2(ny), ID(ny);
+    for (int k = 0; k < K; k++)
+        for (int l = 0; l < NL - 1; l++) {
+            const mg::Level& L = cy.lv[l];
+            const double* cfl = &cf64[24 * m->ylvl[l]];
+            const double qx = 1.0 / (12.0 * m->dx2[l] * c->cfg.fac_y);
+            float4* T = &t32[(size_t)k * cy.tab4];
+            for (int type = 0; type < 2; type++) {
+                tb_poisson_band_matrix_dx(c, type, m->ylvl[l] + 1, k + 1, m->dx2[l], a);
+                tb_band5_factor(L.n, a, L1.data(), L2.data(), U1.data(), U2.data(), ID.data());
+                line_tables(L.n, L.S, type ? 1.0 : 16.0, qx, cfl, L1.data(), L2.data(), U1.data(), U2.data(), ID.data(),
+                            T + L.tab + type * mg::line4(L));
+            }
+            residual_rows(L.n, qx, 1.0 / c->cfg.fac_y, c->h_k2b2[k], c->cfg.alpha * c->cfg.alpha, cfl,
+                          &c->h_qdy2[(size_t)ny * m->ylvl[l]], T + L.tab + 2 * mg::line4(L));
+        }
+    if ((r = upl(&m->tab, t32))) return r;
+    cy.tab = m->tab;
     std::vector<float> cf(cf64.begin(), cf64.end());
     if ((r = upl(&m->coef, cf))) return r;
     std::vector<float> q2(c->h_qdy2.begin(), c->h_qdy2.end());
@@ -1015,6 +844,7 @@ int tb_mixed_setup(tb_ctx* c) {
     for (int k = 0; k < K; k++)
         if (!ok[k]) { tb_set_error("mixed form: coarsest operator of mode %d is singular", k); return TB_ERR_ARG; }
     if ((r = upl(&m->ainv, ainv))) return r;
+    cy.ainv = m->ainv;
     return TB_OK;
 }
 
@@ -1048,7 +878,7 @@ void tb_mixed_free(tb_ctx* c) {
     for (auto& h : m->hist)
         for (cplx* p : h)
             if (p) cudaFree(p);
-    for (void* p : {(void*)m->e, (void*)m->r, (void*)m->rr, (void*)m->tab, (void*)m->coef, (void*)m->qdy2, (void*)m->ainv,
+    for (void* p : {(void*)m->ea, (void*)m->eb, (void*)m->r, (void*)m->tab, (void*)m->coef, (void*)m->qdy2, (void*)m->ainv,
                     (void*)m->maxsq, (void*)m->hvalid, (void*)m->iter, (void*)m->lkeep})
         if (p) cudaFree(p);
     delete m;
@@ -1058,15 +888,12 @@ void tb_mixed_free(tb_ctx* c) {
 // One FP64 correction recorded as the body of the solve's WHILE node:
 // INNER_VCYCLES V-cycles of the FP32 hierarchy, u += e, the new defect and
 // its test (which sets the loop condition).
-static int record_body(tb_ctx* c, const MgDev& M, double erro, cudaGraphConditionalHandle h) {
+static int record_body(tb_ctx* c, const FineDev& M, double erro, cudaGraphConditionalHandle h) {
     Mixed* m = get(c);
     int r;
-    for (int v = 0; v < INNER_VCYCLES; v++)
-        if ((r = vcycle(c, M))) return r;
-    dim3 tgrid(tb_blocks(c->g.nx, 32), tb_blocks(c->g.ny, 32), c->g.K), tblk(32, 8);
-    k_apply<<<tgrid, tblk, 0, c->stream>>>(M, c->pfc, c->g.lvl_elems, c->g.nx, c->g.ny);
-    TB_CHECK_LAUNCH(c);
-    if ((r = tb_poisson_defect_f32(c, m->r, m->e, m->elems, m->maxsq))) return r;
+    if ((r = vcycles(c))) return r;
+    if ((r = apply(c, M))) return r;
+    if ((r = defect(c))) return r;
     k_check_loop<<<1, CHECK_THREADS, 0, c->stream>>>(m->maxsq, c->pstate, c->perr, c->g.K, erro, m->iter, 0,
                                                      c->cfg.max_vcycles, h);
     TB_CHECK_LAUNCH(c);
@@ -1076,7 +903,7 @@ static int record_body(tb_ctx* c, const MgDev& M, double erro, cudaGraphConditio
 // The correction loop of a solve being recorded into a step graph: first
 // defect and test, then a conditional WHILE node that repeats the body
 // above until every mode has converged or max_vcycles corrections ran.
-static int record_loop(tb_ctx* c, const MgDev& M, double erro) {
+static int record_loop(tb_ctx* c, const FineDev& M, double erro) {
     Mixed* m = get(c);
     cudaStreamCaptureStatus st;
     cudaGraph_t g = nullptr;
@@ -1085,7 +912,7 @@ static int record_loop(tb_ctx* c, const MgDev& M, double erro) {
     cudaGraphConditionalHandle h;
     TB_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, 0));
     int r;
-    if ((r = tb_poisson_defect_f32(c, m->r, m->e, m->elems, m->maxsq))) return r;
+    if ((r = defect(c))) return r;
     k_check_loop<<<1, CHECK_THREADS, 0, c->stream>>>(m->maxsq, c->pstate, c->perr, c->g.K, erro, m->iter, 1,
                                                      c->cfg.max_vcycles, h);
     TB_CHECK_LAUNCH(c);
@@ -1149,11 +976,11 @@ int tb_mixed_line_diag(tb_ctx* c, std::vector<float>& invD, std::vector<float>& 
 // shift the stage's history), then (when applying the network) its candidate
 // correction, kept per mode where max|d0 - L e| < max|d0|.  While sampling,
 // the guess is kept for the training targets.
-static int learned_first(tb_ctx* c, const MgDev& M, int ws, LearnSolve* L) {
+static int learned_first(tb_ctx* c, const FineDev& M, int ws, LearnSolve* L) {
     Mixed* m = get(c);
     const int K = c->g.K, nx = c->g.nx, ny = c->g.ny;
     int r;
-    if ((r = tb_poisson_defect_f32(c, m->r, m->e, m->elems, m->maxsq))) return r;
+    if ((r = defect(c))) return r;
     TB_CUDA(cudaMemsetAsync(L->scl, 0, 3 * K * sizeof(float), c->stream));
     const int* valid = m->hvalid + ws;
     cplx *h0 = m->hist[ws][0], *h1 = m->hist[ws][1];
@@ -1181,19 +1008,14 @@ static int learned_first(tb_ctx* c, const MgDev& M, int ws, LearnSolve* L) {
         const size_t per = (size_t)(nx - 2) * (ny - 1);
         k_learn_emit<<<tb_blocks(per * K, 256), 256, 0, c->stream>>>(M, L->out, L->scl, valid, nx);
         TB_CHECK_LAUNCH(c);
-        k_resid<<<tb_blocks(per * K, 256), 256, 0, c->stream>>>(M, 0);
-        TB_CHECK_LAUNCH(c);
         const unsigned nj = std::min<unsigned>(tb_blocks(per, 256), 64);
         k_learn_judge<<<dim3(nj, K), 256, 0, c->stream>>>(M, L->jmax, valid, nx);
         TB_CHECK_LAUNCH(c);
         k_learn_keep<<<tb_blocks(K, 64), 64, 0, c->stream>>>(m->maxsq, L->jmax, m->lkeep, L->tally, valid, K, gk);
         TB_CHECK_LAUNCH(c);
-        MgDev Mk = M;
+        FineDev Mk = M;
         Mk.state = m->lkeep;
-        dim3 tgrid(tb_blocks(nx, 32), tb_blocks(ny, 32), K), tblk(32, 8);
-        k_apply<<<tgrid, tblk, 0, c->stream>>>(Mk, c->pfc, c->g.lvl_elems, nx, ny);
-        TB_CHECK_LAUNCH(c);
-        return TB_OK;
+        return apply(c, Mk);
     };
     if (!L->gated) return network();
     if (!c->capturing) {
@@ -1249,11 +1071,11 @@ static int learned_first(tb_ctx* c, const MgDev& M, int ws, LearnSolve* L) {
 int tb_mixed_fine_op(tb_ctx* c, FineOp* op) {
     Mixed* m = get(c);
     if (!m) { tb_set_error("mixed form not set up"); return TB_ERR_STATE; }
-    MgDev M = make(c);
-    op->coef = M.coef + 24 * M.ylvl[0];
-    op->qdy2 = M.qdy2 + (size_t)M.ny * M.ylvl[0];
+    FineDev M = make(c);
+    op->coef = M.coef;
+    op->qdy2 = M.qdy2;
     op->k2b2 = M.k2b2;
-    op->den = M.qx[0];
+    op->den = M.den;
     op->ify = M.ify;
     op->alpha2 = M.alpha2;
     op->nx = m->ptsx[0];
@@ -1262,31 +1084,36 @@ int tb_mixed_fine_op(tb_ctx* c, FineOp* op) {
     return TB_OK;
 }
 
-// -L e on the finest level of mode k alone (r = 0), through k_resid.
+// -L e on the finest level of mode k alone (r = 0), through fine_resid.
 int tb_mixed_resid_mode(tb_ctx* c, int k, const float* e, float* out) {
     Mixed* m = get(c);
     if (!m) { tb_set_error("mixed form not set up"); return TB_ERR_STATE; }
     const int K = c->g.K, nx = c->g.nx, ny = c->g.ny;
     if (k < 0 || k >= K) { tb_set_error("mode out of range"); return TB_ERR_ARG; }
-    const size_t img = (size_t)nx * ny;
-    std::vector<float2> h(img);
-    for (size_t q = 0; q < img; q++) h[q] = make_float2(e[q], 0.f);
-    std::vector<int> st((size_t)2 * K, 0);
-    st[2 * k] = 1;
-    MgDev M = make(c);
+    FineDev M = make(c);
+    const size_t img = (size_t)nx * ny, lvl = (size_t)3 * M.L.np * M.L.T;
+    std::vector<float2> h(lvl, make_float2(0.f, 0.f)), o(img, make_float2(0.f, 0.f));
+    for (int i = 0; i < nx; i++)
+        for (int j = 0; j < ny; j++) h[mg::el(M.L, i, j)] = make_float2(e[(size_t)ny * i + j], 0.f);
+    float2* d = nullptr;
     TB_CUDA(cudaStreamSynchronize(c->stream));
-    TB_CUDA(cudaMemcpy(m->e + (size_t)k * m->elems, h.data(), img * sizeof(float2), cudaMemcpyHostToDevice));
-    TB_CUDA(cudaMemset(m->r + (size_t)k * m->elems, 0, img * sizeof(float2)));
-    TB_CUDA(cudaMemset(m->rr + (size_t)k * m->elems, 0, img * sizeof(float2)));
-    TB_CUDA(cudaMemcpy(m->lkeep, st.data(), st.size() * sizeof(int), cudaMemcpyHostToDevice));
-    M.state = m->lkeep;
-    const size_t per = (size_t)(nx - 2) * (ny - 1);
-    k_resid<<<tb_blocks(per * K, 256), 256, 0, c->stream>>>(M, 0);
-    TB_CHECK_LAUNCH(c);
-    TB_CUDA(cudaMemcpyAsync(h.data(), m->rr + (size_t)k * m->elems, img * sizeof(float2), cudaMemcpyDeviceToHost, c->stream));
-    TB_CUDA(cudaStreamSynchronize(c->stream));
-    for (size_t q = 0; q < img; q++) out[q] = h[q].x;
-    TB_CUDA(cudaMemset(m->e + (size_t)k * m->elems, 0, img * sizeof(float2)));
+    TB_CUDA(cudaMalloc(&d, img * sizeof(float2)));
+    auto run = [&]() -> int {
+        TB_CUDA(cudaMemcpy(m->eb + (size_t)k * m->elems, h.data(), lvl * sizeof(float2), cudaMemcpyHostToDevice));
+        TB_CUDA(cudaMemset(m->r + (size_t)k * m->elems, 0, lvl * sizeof(float2)));
+        TB_CUDA(cudaMemset(d, 0, img * sizeof(float2)));
+        const size_t per = (size_t)(nx - 2) * (ny - 1);
+        k_fine_resid<<<tb_blocks(per, 256), 256, 0, c->stream>>>(M, k, d);
+        TB_CHECK_LAUNCH(c);
+        TB_CUDA(cudaMemcpyAsync(o.data(), d, img * sizeof(float2), cudaMemcpyDeviceToHost, c->stream));
+        TB_CUDA(cudaStreamSynchronize(c->stream));
+        TB_CUDA(cudaMemset(m->eb + (size_t)k * m->elems, 0, lvl * sizeof(float2)));
+        return TB_OK;
+    };
+    const int r = run();
+    cudaFree(d);
+    if (r) return r;
+    for (size_t q = 0; q < img; q++) out[q] = o[q].x;
     return TB_OK;
 }
 
@@ -1315,7 +1142,7 @@ int tb_mixed_absorb_stats(tb_ctx* c, const int* hs, const double* he) {
 int tb_poi_uy_mixed(tb_ctx* c, const cplx* dwzdx, double erro) {
     if (!c->mixed) { tb_set_error("mixed form not set up"); return TB_ERR_STATE; }
     const int K = c->g.K, nx = c->g.nx, ny = c->g.ny, max_outer = c->cfg.max_vcycles;
-    MgDev M = make(c);
+    FineDev M = make(c);
     Mixed* mx = get(c);
     int r;
     cudaEvent_t pall = nullptr;
@@ -1348,10 +1175,9 @@ int tb_poi_uy_mixed(tb_ctx* c, const cplx* dwzdx, double erro) {
         if ((r = record_loop(c, M, erro))) return r;
     } else {
         std::vector<int> hs(2 * K);
-        dim3 tgrid(tb_blocks(nx, 32), tb_blocks(ny, 32), K), tblk(32, 8);
         for (int it = 0; it <= max_outer; it++) {
             Mixed* m = get(c);
-            if ((r = tb_poisson_defect_f32(c, m->r, m->e, m->elems, m->maxsq))) return r;
+            if ((r = defect(c))) return r;
             k_check_sq<<<tb_blocks(K, 64), 64, 0, c->stream>>>(m->maxsq, c->pstate, c->perr, K, erro, it, it == max_outer);
             TB_CHECK_LAUNCH(c);
             if (it == max_outer) break;
@@ -1360,10 +1186,8 @@ int tb_poi_uy_mixed(tb_ctx* c, const cplx* dwzdx, double erro) {
             bool any = false;
             for (int k = 0; k < K; k++) any = any || hs[2 * k];
             if (!any) break;
-            for (int v = 0; v < INNER_VCYCLES; v++)
-                if ((r = vcycle(c, M))) return r;
-            k_apply<<<tgrid, tblk, 0, c->stream>>>(M, c->pfc, c->g.lvl_elems, nx, ny);
-            TB_CHECK_LAUNCH(c);
+            if ((r = vcycles(c))) return r;
+            if ((r = apply(c, M))) return r;
         }
     }
     if (L && L->infer && L->gated) {

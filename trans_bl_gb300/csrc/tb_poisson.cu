@@ -1,9 +1,7 @@
 // tb_poisson.cu -- the pieces of poi_uy (poisson_par.f:6-164) that the mixed
 // form shares: the source and start state (function_source) in the complex
 // x-contiguous work arrays, the fine-level FP64 defect of the correction
-// equation, the write-back of fc into uy, and the set-up of the y-line band
-// LU factors with their chunk tables (band5_poi, penta_par.f:308-364) used by
-// both forms.  The plain FP64 form's V-cycle is in tb_plain.cu.
+// equation and the write-back of fc into uy.  The plain FP64 form's V-cycle is in tb_plain.cu.
 #include "tb_internal.h"
 #include <cmath>
 #include <cstring>
@@ -135,13 +133,11 @@ __device__ __forceinline__ cplx poi_Lu_b(const PoiDev& P, int l, int k, int i, i
 }
 
 // Fine-level FP64 defect d = sc - L fc for the mixed form: stored as FP32 in
-// the line-contiguous right-hand side r32 of the correction equation (element
-// (i, j) of mode k at k*elems32 + i*ny + j, through a 32x32 shared tile), the
-// correction e32 zeroed at the same points, and max |d|^2 of each mode
-// folded into maxsq[k] (bit pattern of a non-negative double; a non-finite
+// the right-hand side r32 of the correction equation (line i = 3t + c - 1, row
+// j of mode k at k*elems32 + (c*np + j + 1)*T + t, tb_cycle.cuh), and max |d|^2
+// of each mode folded into maxsq[k] (bit pattern of a non-negative double; a non-finite
 // defect records +inf).
-__global__ void k_defect_f32(PoiDev P, float2* r32, float2* e32, size_t elems32, unsigned long long* maxsq) {
-    __shared__ float2 tile[32][33];
+__global__ void k_defect_f32(PoiDev P, float2* r32, size_t elems32, int T, int np, unsigned long long* maxsq) {
     __shared__ cplx bxs[34][32];   // x-stencil sums of rows j0-1 .. j0+32, computed once
     __shared__ double wmax[8];
     const int k = blockIdx.z;
@@ -158,9 +154,10 @@ __global__ void k_defect_f32(PoiDev P, float2* r32, float2* e32, size_t elems32,
     __syncthreads();
     double m = 0.0;
     bool bad = false;
+    const int iq = i0 + threadIdx.x + 1;
+    const size_t o32 = (size_t)k * elems32 + ((size_t)(iq % 3) * np + 1) * T + iq / 3;   // row 0 of this line
     for (int r = threadIdx.y; r < 32; r += 8) {
         int i = i0 + threadIdx.x, j = j0 + r;
-        float2 v32 = make_float2(0.f, 0.f);
         if (i <= nx - 2 && j <= ny - 1) {
             cplx s = P.sc[(size_t)k * P.elems + (size_t)i + (size_t)nx * j];
             cplx Lu = poi_Lu_b(P, 0, k, i, j, [&](int jj) { return bxs[jj - j0 + 1][threadIdx.x]; });
@@ -168,9 +165,8 @@ __global__ void k_defect_f32(PoiDev P, float2* r32, float2* e32, size_t elems32,
             double a = v.x * v.x + v.y * v.y;
             if (!(a <= 1.7e308)) bad = true;
             else m = fmax(m, a);
-            v32 = make_float2((float)v.x, (float)v.y);
+            r32[o32 + (size_t)j * T] = make_float2((float)v.x, (float)v.y);
         }
-        tile[r][threadIdx.x] = v32;
     }
     if (bad) m = __longlong_as_double(0x7ff0000000000000LL);
 #pragma unroll
@@ -182,14 +178,6 @@ __global__ void k_defect_f32(PoiDev P, float2* r32, float2* e32, size_t elems32,
         double b = wmax[0];
         for (int q = 1; q < 8; q++) b = fmax(b, wmax[q]);
         atomicMax(&maxsq[k], (unsigned long long)__double_as_longlong(b));
-    }
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        int i = i0 + r, j = j0 + threadIdx.x;
-        if (i <= nx - 2 && j <= ny - 1) {
-            size_t o = (size_t)k * elems32 + (size_t)ny * i + j;
-            r32[o] = tile[threadIdx.x][r];
-            e32[o] = make_float2(0.f, 0.f);
-        }
     }
 }
 
@@ -225,65 +213,6 @@ PoiDev make_dev(tb_ctx* c) {
 }
 
 }  // namespace
-
-// Host: chunk tables of the line solve for one (type, level, mode), lane
-// chunks of S rows (lane t owns rows [tS, min(n, tS + S))).
-void tb_chunk_tables(int n, int ny, int S, const double* L1, const double* L2, const double* U1, const double* U2,
-                     const double* ID, double* out) {
-    double *h1 = out, *h2 = out + ny, *k1 = out + 2 * ny, *k2 = out + 3 * ny;
-    double* Pf = out + 4 * ny;
-    double* Pb = Pf + 640;
-    double Mf[32][4], Mb[32][4];
-    for (int t = 0; t < 32; t++) {
-        int r0 = t * S, r1 = std::min(n, r0 + S);
-        // forward: responses to incoming (Y1 = y_{r0-1}, Y2 = y_{r0-2})
-        double e0[2], e1[2];   // outgoing (y_{e}, y_{e-1}) for unit incoming
-        for (int u = 0; u < 2; u++) {
-            double ym1 = (u == 0) ? 1.0 : 0.0, ym2 = (u == 0) ? 0.0 : 1.0;
-            for (int j = r0; j < r1; j++) {
-                double y = -L2[j] * ym2 - L1[j] * ym1;
-                (u == 0 ? h1 : h2)[j] = y;
-                ym2 = ym1; ym1 = y;
-            }
-            e0[u] = ym1; e1[u] = ym2;  // for an empty chunk this is the identity
-        }
-        Mf[t][0] = e0[0]; Mf[t][1] = e0[1]; Mf[t][2] = e1[0]; Mf[t][3] = e1[1];
-        // backward: responses to incoming (X1 = x_{r1}, X2 = x_{r1+1})
-        for (int u = 0; u < 2; u++) {
-            double xp1 = (u == 0) ? 1.0 : 0.0, xp2 = (u == 0) ? 0.0 : 1.0;
-            for (int j = r1 - 1; j >= r0; j--) {
-                double x = (-U1[j] * xp1 - U2[j] * xp2) * ID[j];
-                (u == 0 ? k1 : k2)[j] = x;
-                xp2 = xp1; xp1 = x;
-            }
-            e0[u] = xp1; e1[u] = xp2;
-        }
-        Mb[t][0] = e0[0]; Mb[t][1] = e0[1]; Mb[t][2] = e1[0]; Mb[t][3] = e1[1];
-    }
-    // Kogge-Stone: A_t before each step; b_t += A_t b_{t-off}; A_t = A_t A_{t-off}
-    auto mul = [](const double* A, const double* B, double* C) {
-        double c0 = A[0] * B[0] + A[1] * B[2], c1 = A[0] * B[1] + A[1] * B[3];
-        double c2 = A[2] * B[0] + A[3] * B[2], c3 = A[2] * B[1] + A[3] * B[3];
-        C[0] = c0; C[1] = c1; C[2] = c2; C[3] = c3;
-    };
-    double Af[32][4], Ab[32][4];
-    std::memcpy(Af, Mf, sizeof Af);
-    std::memcpy(Ab, Mb, sizeof Ab);
-    for (int d = 0, off = 1; d < 5; d++, off <<= 1) {
-        for (int t = 0; t < 32; t++) {
-            std::memcpy(Pf + (d * 32 + t) * 4, Af[t], 4 * sizeof(double));
-            std::memcpy(Pb + (d * 32 + t) * 4, Ab[t], 4 * sizeof(double));
-        }
-        double nf[32][4], nb[32][4];
-        for (int t = 0; t < 32; t++) {
-            if (t >= off) mul(Af[t], Af[t - off], nf[t]); else std::memcpy(nf[t], Af[t], sizeof nf[t]);
-            if (t + off < 32) mul(Ab[t], Ab[t + off], nb[t]); else std::memcpy(nb[t], Ab[t], sizeof nb[t]);
-        }
-        std::memcpy(Af, nf, sizeof Af);
-        std::memcpy(Ab, nb, sizeof Ab);
-    }
-}
-
 
 int tb_poisson_setup(tb_ctx* c) {
     int ny = c->g.ny, K = c->g.K;
@@ -321,12 +250,12 @@ int tb_poisson_end(tb_ctx* c) {
     return TB_OK;
 }
 
-int tb_poisson_defect_f32(tb_ctx* c, float2* r32, float2* e32, size_t elems32, unsigned long long* maxsq) {
+int tb_poisson_defect_f32(tb_ctx* c, float2* r32, size_t elems32, int T, int np, unsigned long long* maxsq) {
     PoiDev P = make_dev(c);
     dim3 grid(tb_blocks(c->g.nx - 2, 32), tb_blocks(c->g.ny - 1, 32), c->g.K), blk(32, 8);
     cudaEvent_t ps = nullptr;
     if (tb_prof_begin(c, PROF_DEFECT, &ps)) return TB_ERR_CUDA;
-    k_defect_f32<<<grid, blk, 0, c->stream>>>(P, r32, e32, elems32, maxsq);
+    k_defect_f32<<<grid, blk, 0, c->stream>>>(P, r32, elems32, T, np, maxsq);
     TB_CHECK_LAUNCH(c);
     return tb_prof_end(c, PROF_DEFECT, ps);
 }
