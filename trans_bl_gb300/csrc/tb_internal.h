@@ -224,7 +224,7 @@ int tb_plain_setup(tb_ctx* c);
 int tb_plain_tune(tb_ctx* c, int l, int itera, const int* gis, int ngis, int* best, float* best_ms);
 int tb_poisson_setup(tb_ctx* c);
 int tb_poisson_begin(tb_ctx* c, const cplx* dwzdx);
-int tb_poisson_defect_f32(tb_ctx* c, float2* r32, size_t elems32, int T, int np, unsigned long long* maxsq);
+int tb_poisson_defect_f32(tb_ctx* c, const double* rows, float2* r32, size_t elems32, int T, int np, unsigned long long* maxsq);
 int tb_poisson_end(tb_ctx* c);
 int tb_poi_uy_mixed(tb_ctx* c, const cplx* dwzdx, double erro);
 // Learned first correction of the mixed solve (tb_learn.cu owns the network

@@ -56,6 +56,7 @@ constexpr int DIRECT_MAX = 400;      // unknowns per mode below which coarsening
 struct Mixed {
     float2 *ea = nullptr, *eb = nullptr, *r = nullptr;   // per mode blocks of `elems` (layout: tb_cycle.cuh)
     float4* tab = nullptr;    // per mode: line-solve and residual rows of every level (mg::Cycle::tab)
+    double* drow = nullptr;   // (K, ny, 8) rows of the FP64 defect: -w1[-1..1], -w2[-2..2] (residual_row)
     float* coef = nullptr;    // sp(7) cp(8) pp(4) lp(5) per reference level
     float* qdy2 = nullptr;    // (ny, msh)
     float* ainv = nullptr;    // (K, N, N) inverse of the coarsest operator per mode
@@ -538,7 +539,7 @@ int apply(tb_ctx* c, const FineDev& M) {
 
 int defect(tb_ctx* c) {
     Mixed* m = get(c);
-    return tb_poisson_defect_f32(c, m->r, m->elems, m->cyc.lv[0].T, m->cyc.lv[0].np, m->maxsq);
+    return tb_poisson_defect_f32(c, m->drow, m->r, m->elems, m->cyc.lv[0].T, m->cyc.lv[0].np, m->maxsq);
 }
 
 template <int S>
@@ -665,36 +666,46 @@ void line_tables(int n, int S, double unit, double qx, const double* cf, const d
     }
 }
 
-// Residual rows of one level and mode: -16 w1[-1..1] of the x-stencil sums and
-// -w2[-2..2] of the values, the centre stencil's diagonal (-30) folded into w2.
+// The operator's row j (1 <= j < n) of one level and mode as weights of the
+// x-stencil sums of rows j-1 .. j+1 (w[0..2]) and of the values of rows
+// j-2 .. j+2 (w[3..7]), the centre stencil's diagonal (-30) folded into the
+// latter: L u = sum_q w1[q] X(j+q) + sum_q w2[q] u(j+q).
+void residual_row(int j, int n, double den, double ify, double k2b2, double alpha2, const double* cf, const double* Q2,
+                  double* w) {
+    const double *SP = cf, *CP = cf + 7, *PP = cf + 15, *LP = cf + 19;
+    double *w1 = w, *w2 = w + 3;
+    std::fill(w, w + 8, 0.0);
+    const double kk = k2b2 * ify;
+    if (j == 1) {
+        const double q2 = Q2[0];
+        w1[1] = den * SP[1]; w1[2] = den * SP[2];
+        for (int q = 0; q < 4; q++) w2[1 + q] = q2 * SP[3 + q];
+        w2[2] += kk * SP[1]; w2[3] += kk * SP[2];
+    } else if (j <= n - 3) {
+        const double q2 = Q2[j - 2];
+        for (int q = 0; q < 3; q++) w1[q] = den * CP[q];
+        for (int q = 0; q < 5; q++) w2[q] = q2 * CP[3 + q];
+        for (int q = 0; q < 3; q++) w2[1 + q] += kk * CP[q];
+    } else if (j == n - 2) {
+        const double q2 = Q2[j - 1];
+        w1[1] = den;
+        w2[3] = q2 * PP[3]; w2[2] = q2 * PP[2] + kk; w2[1] = q2 * PP[1];
+    } else {
+        const double q2 = Q2[j - 2];
+        w1[1] = den;
+        w2[2] = q2 * LP[2] + kk - LP[1] * std::sqrt((alpha2 - k2b2) * ify) * std::sqrt(q2);
+        w2[1] = q2 * LP[3]; w2[0] = q2 * LP[4];
+    }
+    for (int q = 0; q < 3; q++) w2[1 + q] -= 30.0 * w1[q];
+}
+
+// FP32 residual rows of one level and mode, negated, the sums in units of 16.
 void residual_rows(int n, double den, double ify, double k2b2, double alpha2, const double* cf, const double* Q2,
                    float4* out) {
-    const double *SP = cf, *CP = cf + 7, *PP = cf + 15, *LP = cf + 19;
     for (int j = 1; j < n; j++) {
-        double w[8] = {0, 0, 0, 0, 0, 0, 0, 0}, *w1 = w, *w2 = w + 3;
-        const double kk = k2b2 * ify;
-        if (j == 1) {
-            const double q2 = Q2[0];
-            w1[1] = den * SP[1]; w1[2] = den * SP[2];
-            for (int q = 0; q < 4; q++) w2[1 + q] = q2 * SP[3 + q];
-            w2[2] += kk * SP[1]; w2[3] += kk * SP[2];
-        } else if (j <= n - 3) {
-            const double q2 = Q2[j - 2];
-            for (int q = 0; q < 3; q++) w1[q] = den * CP[q];
-            for (int q = 0; q < 5; q++) w2[q] = q2 * CP[3 + q];
-            for (int q = 0; q < 3; q++) w2[1 + q] += kk * CP[q];
-        } else if (j == n - 2) {
-            const double q2 = Q2[j - 1];
-            w1[1] = den;
-            w2[3] = q2 * PP[3]; w2[2] = q2 * PP[2] + kk; w2[1] = q2 * PP[1];
-        } else {
-            const double q2 = Q2[j - 2];
-            w1[1] = den;
-            w2[2] = q2 * LP[2] + kk - LP[1] * std::sqrt((alpha2 - k2b2) * ify) * std::sqrt(q2);
-            w2[1] = q2 * LP[3]; w2[0] = q2 * LP[4];
-        }
-        for (int q = 0; q < 3; q++) w2[1 + q] -= 30.0 * w1[q];
-        for (int q = 0; q < 8; q++) w[q] *= q < 3 ? -16.0 : -1.0;   // the x-stencil sums are in units of 16
+        double w[8];
+        residual_row(j, n, den, ify, k2b2, alpha2, cf, Q2, w);
+        for (int q = 0; q < 8; q++) w[q] *= q < 3 ? -16.0 : -1.0;
         put_pairs(out + (size_t)mg::RES4 * j, w, 8);
     }
 }
@@ -815,6 +826,15 @@ int tb_mixed_setup(tb_ctx* c) {
         }
     if ((r = upl(&m->tab, t32))) return r;
     cy.tab = m->tab;
+    std::vector<double> drow((size_t)K * ny * 8, 0.0);
+    for (int k = 0; k < K; k++)
+        for (int j = 1; j < ny; j++) {
+            double* w = &drow[((size_t)k * ny + j) * 8];
+            residual_row(j, ny, 1.0 / (12.0 * c->h_dx2[0] * c->cfg.fac_y), 1.0 / c->cfg.fac_y, c->h_k2b2[k],
+                         c->cfg.alpha * c->cfg.alpha, &cf64[0], &c->h_qdy2[0], w);
+            for (int q = 0; q < 8; q++) w[q] = -w[q];
+        }
+    if ((r = upl(&m->drow, drow))) return r;
     std::vector<float> cf(cf64.begin(), cf64.end());
     if ((r = upl(&m->coef, cf))) return r;
     std::vector<float> q2(c->h_qdy2.begin(), c->h_qdy2.end());
@@ -878,7 +898,7 @@ void tb_mixed_free(tb_ctx* c) {
     for (auto& h : m->hist)
         for (cplx* p : h)
             if (p) cudaFree(p);
-    for (void* p : {(void*)m->ea, (void*)m->eb, (void*)m->r, (void*)m->tab, (void*)m->coef, (void*)m->qdy2, (void*)m->ainv,
+    for (void* p : {(void*)m->ea, (void*)m->eb, (void*)m->r, (void*)m->tab, (void*)m->drow, (void*)m->coef, (void*)m->qdy2, (void*)m->ainv,
                     (void*)m->maxsq, (void*)m->hvalid, (void*)m->iter, (void*)m->lkeep})
         if (p) cudaFree(p);
     delete m;

@@ -68,117 +68,80 @@ __global__ void k_source(PoiDev P, const cplx* wx, const cplx* dwzdx, const cplx
 }
 
 // ---------------------------------------------------------------------------
-// The level-l operator of defect (poisson_par.f:543-793) applied to fc at the
-// interior point (i, j) of mode k: L fc = den*Dxx + q2*Dyy + k2b2*ify*M - top.
-// The x-stencil sum of row jj (rhs_center / rhs_border incl. the diagonal):
-__device__ __forceinline__ cplx poi_bx(const PoiDev& P, int l, int k, int i, int jj) {
-    const int nxl = P.ptsx[l];
-    const cplx* F = P.fc + (size_t)k * P.elems + P.off[l] + (size_t)nxl * jj;
-    if (i == 1 || i == nxl - 2) {
-        int e = (i == 1) ? 1 : -1;
-        cplx a = F[i - e], c0 = F[i], b = F[i + e], c = F[i + 2 * e], d = F[i + 3 * e], g = F[i + 4 * e];
-        return make_double2(10.0 * a.x - 15.0 * c0.x - 4.0 * b.x + 14.0 * c.x - 6.0 * d.x + g.x,
-                            10.0 * a.y - 15.0 * c0.y - 4.0 * b.y + 14.0 * c.y - 6.0 * d.y + g.y);
-    }
-    cplx a = F[i - 2], b = F[i - 1], c0 = F[i], c = F[i + 1], d = F[i + 2];
-    return make_double2(-a.x + 16.0 * b.x - 30.0 * c0.x + 16.0 * c.x - d.x, -a.y + 16.0 * b.y - 30.0 * c0.y + 16.0 * c.y - d.y);
-}
-
-// L fc at (i, j) with the x-stencil sums supplied by bx(jj).
-template <class BX>
-__device__ __forceinline__ cplx poi_Lu_b(const PoiDev& P, int l, int k, int i, int j, BX bx) {
-    const int nxl = P.ptsx[l], n = P.ptsy[l];
-    const double* cf = P.coef + 24 * l;
-    const double *SPc = cf, *CPc = cf + 7, *PPc = cf + 15, *LPc = cf + 19;
-    double k2b2 = P.k2b2[k];
-    double den = P.den[l], ify = P.ify;
-    const cplx* F = P.fc + (size_t)k * P.elems + P.off[l];
-    auto f = [&](int ii, int jj) -> cplx { return F[(size_t)ii + (size_t)nxl * jj]; };
-    cplx b, cc, d;
-    double q2;
-    double top = 0.0;
-    if (j == 1) {
-        cplx b1 = bx(1), b2 = bx(2);
-        b = make_double2(SPc[2] * b2.x + SPc[1] * b1.x, SPc[2] * b2.y + SPc[1] * b1.y);
-        cplx f0 = f(i, 0), f1 = f(i, 1), f2 = f(i, 2), f3 = f(i, 3);
-        cc = make_double2(SPc[3] * f0.x + SPc[4] * f1.x + SPc[5] * f2.x + SPc[6] * f3.x,
-                          SPc[3] * f0.y + SPc[4] * f1.y + SPc[5] * f2.y + SPc[6] * f3.y);
-        d = make_double2(k2b2 * (SPc[1] * f1.x + SPc[2] * f2.x), k2b2 * (SPc[1] * f1.y + SPc[2] * f2.y));
-        q2 = P.qdy2[0 + (size_t)P.ny * l];
-    } else if (j <= n - 3) {
-        cplx ba = bx(j - 1), bb = bx(j), bc = bx(j + 1);
-        b = make_double2(CPc[0] * ba.x + CPc[1] * bb.x + CPc[2] * bc.x, CPc[0] * ba.y + CPc[1] * bb.y + CPc[2] * bc.y);
-        cplx fm2 = f(i, j - 2), fm1 = f(i, j - 1), f0 = f(i, j), fp1 = f(i, j + 1), fp2 = f(i, j + 2);
-        cc = make_double2(CPc[3] * fm2.x + CPc[4] * fm1.x + CPc[5] * f0.x + CPc[6] * fp1.x + CPc[7] * fp2.x,
-                          CPc[3] * fm2.y + CPc[4] * fm1.y + CPc[5] * f0.y + CPc[6] * fp1.y + CPc[7] * fp2.y);
-        d = make_double2(k2b2 * (CPc[0] * fm1.x + CPc[1] * f0.x + CPc[2] * fp1.x), k2b2 * (CPc[0] * fm1.y + CPc[1] * f0.y + CPc[2] * fp1.y));
-        q2 = P.qdy2[(j - 2) + (size_t)P.ny * l];
-    } else if (j == n - 2) {
-        b = bx(j);
-        cplx fm1 = f(i, j - 1), f0 = f(i, j), fp1 = f(i, j + 1);
-        cc = make_double2(PPc[3] * fp1.x + PPc[2] * f0.x + PPc[1] * fm1.x, PPc[3] * fp1.y + PPc[2] * f0.y + PPc[1] * fm1.y);
-        d = make_double2(k2b2 * f0.x, k2b2 * f0.y);
-        q2 = P.qdy2[(j - 1) + (size_t)P.ny * l];
-    } else {
-        b = bx(j);
-        cplx fm2 = f(i, j - 2), fm1 = f(i, j - 1), f0 = f(i, j);
-        cc = make_double2(LPc[2] * f0.x + LPc[3] * fm1.x + LPc[4] * fm2.x, LPc[2] * f0.y + LPc[3] * fm1.y + LPc[4] * fm2.y);
-        d = make_double2(k2b2 * f0.x, k2b2 * f0.y);
-        q2 = P.qdy2[(j - 2) + (size_t)P.ny * l];
-        double alpha2 = sqrt((P.alpha * P.alpha - k2b2) / P.fac_y);
-        top = LPc[1] * alpha2 * sqrt(q2);
-    }
-    cplx fij = f(i, j);
-    return make_double2(b.x * den + cc.x * q2 + d.x * ify - top * fij.x, b.y * den + cc.y * q2 + d.y * ify - top * fij.y);
-}
-
-// Fine-level FP64 defect d = sc - L fc for the mixed form: stored as FP32 in
-// the right-hand side r32 of the correction equation (line i = 3t + c - 1, row
-// j of mode k at k*elems32 + (c*np + j + 1)*T + t, tb_cycle.cuh), and max |d|^2
-// of each mode folded into maxsq[k] (bit pattern of a non-negative double; a non-finite
+// Fine-level FP64 defect d = sc - L fc for the mixed form (the operator of
+// defect, poisson_par.f:543-793): stored as FP32 in the right-hand side r32 of
+// the correction equation (line i = 3t + c - 1, row j of mode k at
+// k*elems32 + (c*np + j + 1)*T + t, tb_cycle.cuh), and max |d|^2 of each mode
+// folded into maxsq[k] (bit pattern of a non-negative double; a non-finite
 // defect records +inf).
-__global__ void k_defect_f32(PoiDev P, float2* r32, size_t elems32, int T, int np, unsigned long long* maxsq) {
-    __shared__ cplx bxs[34][32];   // x-stencil sums of rows j0-1 .. j0+32, computed once
-    __shared__ double wmax[8];
+//
+// An FP64 warp instruction holds its pipe for 64 cycles, so their number is
+// what the kernel costs.  L fc is the sum of three x-stencil sums and five
+// values with weights that depend on the row and the mode only (rows, set up
+// once: -w1[-1..1], -w2[-2..2] with every constant factor and the stencil's
+// diagonal folded in), and a thread marches down a column with both windows
+// in registers, so a stencil sum is formed once: 24 FP64 instructions a complex
+// point instead of 46 with the operator's terms formed one by one (all modes
+// active, 1025 x 193 x 64: 975 -> 530 us).  The maximum is compared as integer bit patterns.
+constexpr int DEF_ROWS = 24;   // rows per thread: two more stencil sums per chunk
+__global__ void __launch_bounds__(128) k_defect_f32(PoiDev P, const double* __restrict__ rows, float2* r32, size_t elems32, int T,
+                                                    int np, unsigned long long* maxsq) {
+    __shared__ unsigned long long wmax[4];
     const int k = blockIdx.z;
     if (!P.state[2 * k]) return;   // uniform over the block
     const int nx = P.nx, ny = P.ny;
-    const int i0 = 1 + blockIdx.x * 32, j0 = 1 + blockIdx.y * 32;
-    {
-        const int i = i0 + threadIdx.x;
-        for (int r = threadIdx.y; r < 34; r += 8) {
-            int jj = j0 - 1 + r;
-            bxs[r][threadIdx.x] = (i <= nx - 2 && jj >= 1 && jj <= ny - 1) ? poi_bx(P, 0, k, i, jj) : make_double2(0.0, 0.0);
-        }
-    }
-    __syncthreads();
-    double m = 0.0;
-    bool bad = false;
-    const int iq = i0 + threadIdx.x + 1;
-    const size_t o32 = (size_t)k * elems32 + ((size_t)(iq % 3) * np + 1) * T + iq / 3;   // row 0 of this line
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        int i = i0 + threadIdx.x, j = j0 + r;
-        if (i <= nx - 2 && j <= ny - 1) {
-            cplx s = P.sc[(size_t)k * P.elems + (size_t)i + (size_t)nx * j];
-            cplx Lu = poi_Lu_b(P, 0, k, i, j, [&](int jj) { return bxs[jj - j0 + 1][threadIdx.x]; });
-            cplx v = make_double2(s.x - Lu.x, s.y - Lu.y);
-            double a = v.x * v.x + v.y * v.y;
-            if (!(a <= 1.7e308)) bad = true;
-            else m = fmax(m, a);
-            r32[o32 + (size_t)j * T] = make_float2((float)v.x, (float)v.y);
-        }
-    }
-    if (bad) m = __longlong_as_double(0x7ff0000000000000LL);
+    const int i = 1 + blockIdx.x * 128 + threadIdx.x;
+    const int j0 = 1 + blockIdx.y * DEF_ROWS, j1 = min(ny, j0 + DEF_ROWS);
+    unsigned long long m = 0;
+    if (i <= nx - 2) {
+        const cplx* F = P.fc + (size_t)k * P.elems + i;
+        const cplx* SC = P.sc + (size_t)k * P.elems + i;
+        const double* W = rows + (size_t)k * ny * 8;
+        const int iq = i + 1;
+        float2* out = r32 + (size_t)k * elems32 + ((size_t)(iq % 3) * np + 1) * T + iq / 3;   // row 0 of this line
+        const bool border = i == 1 || i == nx - 2;
+        const int e = (i == 1) ? 1 : -1;
+        const cplx z = make_double2(0.0, 0.0);
+        auto val = [&](int j) -> cplx { return (j >= 0 && j < ny) ? F[(size_t)nx * j] : z; };
+        // x-stencil sum of row j without its centre term -30 f; a border line
+        // (one-sided, centre term -15 f) adds the 15 f that the folded weight has too much
+        auto sum = [&](int j, cplx f) -> cplx {
+            if (j < 1 || j >= ny) return z;   // weight 0
+            const cplx* R = F + (size_t)nx * j;
+            if (border) {
+                const cplx a = R[-e], b = R[e], c = R[2 * e], d = R[3 * e], g = R[4 * e];
+                return make_double2(fma(15.0, f.x, fma(10.0, a.x, fma(-4.0, b.x, fma(14.0, c.x, fma(-6.0, d.x, g.x))))),
+                                    fma(15.0, f.y, fma(10.0, a.y, fma(-4.0, b.y, fma(14.0, c.y, fma(-6.0, d.y, g.y))))));
+            }
+            const cplx a = R[-2], b = R[-1], c = R[1], d = R[2];
+            return make_double2(fma(16.0, b.x + c.x, -(a.x + d.x)), fma(16.0, b.y + c.y, -(a.y + d.y)));
+        };
+        cplx f0 = val(j0 - 2), f1 = val(j0 - 1), f2 = val(j0), f3 = val(j0 + 1);
+        cplx x0 = sum(j0 - 1, f1), x1 = sum(j0, f2);
+        const unsigned long long largest = (unsigned long long)__double_as_longlong(1.7e308);
+#pragma unroll 2
+        for (int j = j0; j < j1; j++) {
+            const cplx f4 = val(j + 2), x2 = sum(j + 1, f3);
+            const double* w = W + 8 * j;
+            cplx v = SC[(size_t)nx * j];
+            const cplx t[8] = {x0, x1, x2, f0, f1, f2, f3, f4};
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    const int w = (threadIdx.y * 32 + threadIdx.x) >> 5;
-    if ((threadIdx.x & 31) == 0) wmax[w] = m;
-    __syncthreads();
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
-        double b = wmax[0];
-        for (int q = 1; q < 8; q++) b = fmax(b, wmax[q]);
-        atomicMax(&maxsq[k], (unsigned long long)__double_as_longlong(b));
+            for (int q = 0; q < 8; q++) {
+                const double c = w[q];
+                v = make_double2(fma(c, t[q].x, v.x), fma(c, t[q].y, v.y));
+            }
+            const unsigned long long a = (unsigned long long)__double_as_longlong(fma(v.x, v.x, v.y * v.y));
+            m = max(m, a > largest ? 0x7ff0000000000000ull : a);
+            out[(size_t)j * T] = make_float2((float)v.x, (float)v.y);
+            f0 = f1; f1 = f2; f2 = f3; f3 = f4;
+            x0 = x1; x1 = x2;
+        }
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) atomicMax(&maxsq[k], max(max(wmax[0], wmax[1]), max(wmax[2], wmax[3])));
 }
 
 // uy(i,j,k) = fc(i,j,1) for j >= 2, 2 <= i <= ptsx-1 (poisson_par.f:53-57).
@@ -250,12 +213,12 @@ int tb_poisson_end(tb_ctx* c) {
     return TB_OK;
 }
 
-int tb_poisson_defect_f32(tb_ctx* c, float2* r32, size_t elems32, int T, int np, unsigned long long* maxsq) {
+int tb_poisson_defect_f32(tb_ctx* c, const double* rows, float2* r32, size_t elems32, int T, int np, unsigned long long* maxsq) {
     PoiDev P = make_dev(c);
-    dim3 grid(tb_blocks(c->g.nx - 2, 32), tb_blocks(c->g.ny - 1, 32), c->g.K), blk(32, 8);
+    dim3 grid(tb_blocks(c->g.nx - 2, 128), tb_blocks(c->g.ny - 1, DEF_ROWS), c->g.K);
     cudaEvent_t ps = nullptr;
     if (tb_prof_begin(c, PROF_DEFECT, &ps)) return TB_ERR_CUDA;
-    k_defect_f32<<<grid, blk, 0, c->stream>>>(P, r32, elems32, T, np, maxsq);
+    k_defect_f32<<<grid, 128, 0, c->stream>>>(P, rows, r32, elems32, T, np, maxsq);
     TB_CHECK_LAUNCH(c);
     return tb_prof_end(c, PROF_DEFECT, ps);
 }
