@@ -272,8 +272,8 @@ int tb_learn_op_apply(tb_ctx* ctx, int k, const float* e, float* out);
 
 /* ---- launch shapes ----------------------------------------------------
    tb_autotune times the candidate launch shapes of the stage's batched
-   kernels on this context's grid and keeps the fastest: warps per block of
-   the x-line solves (1, 2), threads per block of the y-line solves (32, 64,
+   kernels on this context's grid and keeps the fastest: lines per block of
+   the x-line solves (1: half of what fits, 2: what fits), threads per block of the y-line solves (32, 64,
    128) and, for the mixed form with P >= 16, resident blocks per SM of the
    tensor-core passes (1, 2, 4, 8, capped by shared and tensor memory), and,
    for the plain form, warps per y-line solve of the Poisson sweeps (1, 2, 4).
@@ -372,8 +372,8 @@ int tb_profile_read(tb_ctx* ctx, int family, double* ms, long long* launches);
    DEVICE buffers wx, wy, wz (complex*16 (nx, ny, kfour)), for hosts that must
    not allocate GPU memory after start-up (a memory manager that owns all free
    device memory, or a real-time section).  Needs no context and
-   allocates nothing: the filtered lines are staged in a 32 MiB array built
-   into the library, so one call takes nx*ny*kfour <= 2^21 - 4096 points and
+   allocates nothing: the lines are filtered in place, the operator's tables
+   kept in a 32 MiB array built into the library; one call takes nx*ny*kfour <= 2^21 - 4096 points and
    nx <= 4096 (filter larger grids one slice of Fourier modes per call) and
    returns TB_ERR_ARG beyond that.  The first call on a device sets up the
    array's address and must precede any stream capture (after cudaDeviceReset

@@ -3,6 +3,7 @@
 // recomputes inside every call (derivs_k, create_ctes, lhs5+ludecomp,
 // coef_center/coef_border+band5_poi, var_ts, buffer ramps, gibbs_function).
 #include "tb_internal.h"
+#include "tb_xline.cuh"
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -119,56 +120,57 @@ int upload(T** dst, const std::vector<T>& src) {
     return TB_OK;
 }
 
-// Chunk tables of a Thomas sweep split over 32 lanes of S rows (TriLHS).
-void chunk_tri(const std::vector<double>& a, const std::vector<double>& g, const std::vector<double>& ib, int S,
-               std::vector<double>& hf, std::vector<double>& hb, std::vector<double>& pf, std::vector<double>& pb) {
-    int n = (int)a.size();
-    hf.assign(n, 0.0); hb.assign(n, 0.0); pf.assign(160, 0.0); pb.assign(160, 0.0);
-    double Af[32], Ab[32];
-    for (int t = 0; t < 32; t++) {
-        int r0 = t * S, r1 = std::min(n, r0 + S);
-        double h = 1.0;
-        for (int i = r0; i < r1; i++) { h *= -a[i] * ib[i]; hf[i] = h; }
-        Af[t] = (r1 > r0) ? hf[r1 - 1] : 1.0;
-        h = 1.0;
-        for (int i = r1 - 1; i >= r0; i--) { h = (r1 < n) ? h * -g[i + 1] : 0.0; hb[i] = h; }
-        Ab[t] = (r1 > r0) ? hb[r0] : 1.0;
-    }
-    for (int d = 0, off = 1; d < 5; d++, off <<= 1) {
-        double nf[32], nb[32];
-        for (int t = 0; t < 32; t++) {
-            pf[d * 32 + t] = Af[t];
-            pb[d * 32 + t] = Ab[t];
-            nf[t] = (t >= off) ? Af[t] * Af[t - off] : Af[t];
-            nb[t] = (t + off < 32) ? Ab[t] * Ab[t + off] : Ab[t];
-        }
-        std::copy(nf, nf + 32, Af);
-        std::copy(nb, nb + 32, Ab);
-    }
-}
-
-int upload_tri(TriLHS& t, const std::vector<double>& a, const std::vector<double>& b, const std::vector<double>& c,
-               bool chunked = false) {
+int upload_tri(TriLHS& t, const std::vector<double>& a, const std::vector<double>& b, const std::vector<double>& c) {
     std::vector<double> g, ib;
     thomas_factors(a, b, c, g, ib);
     int r;
     if ((r = upload(&t.a, a))) return r;
     if ((r = upload(&t.g, g))) return r;
-    if ((r = upload(&t.ib, ib))) return r;
-    if (!chunked) return TB_OK;
-    int n = (int)a.size();
-    t.S = (n + 31) / 32;
-    std::vector<double> hf, hb, pf, pb;
-    chunk_tri(a, g, ib, t.S, hf, hb, pf, pb);
-    if ((r = upload(&t.hf, hf))) return r;
-    if ((r = upload(&t.hb, hb))) return r;
-    if ((r = upload(&t.pf, pf))) return r;
-    if ((r = upload(&t.pb, pb))) return r;
-    auto f32 = [](const std::vector<double>& v) { return std::vector<float>(v.begin(), v.end()); };
-    if ((r = upload(&t.af, f32(a))) || (r = upload(&t.gf, f32(g))) || (r = upload(&t.ibf, f32(ib))) ||
-        (r = upload(&t.hff, f32(hf))) || (r = upload(&t.hbf, f32(hb))) || (r = upload(&t.pff, f32(pf))))
-        return r;
-    return upload(&t.pbf, f32(pb));
+    return upload(&t.ib, ib);
+}
+
+// Row tables of an x-line operator (tb_xline.cuh) with right-hand sides in
+// units of kappa.
+int upload_xline(TriLHS& t, int op, const xl::Weights& wt, const std::vector<double>& a, const std::vector<double>& b,
+                 const std::vector<double>& c, double kappa) {
+    std::vector<double> g, ib;
+    thomas_factors(a, b, c, g, ib);
+    const int n = (int)a.size(), S = (n + 31) / 32;
+    t.S = S;
+    std::vector<double> T(xl::table_size(S), 0.0);
+    double *pf = &T[160 * S], *pb = pf + 160, Af[32], Ab[32];
+    for (int lane = 0; lane < 32; lane++) {
+        const int r0 = std::min(n, lane * S), r1 = std::min(n, r0 + S);
+        auto at = [&](int tab, int i) -> double& { return T[(size_t)32 * (tab * S + i - r0) + lane]; };
+        double h = 1.0;
+        for (int i = r0; i < r1; i++) {
+            const double l = i ? a[i] * ib[i - 1] : 0.0;
+            h *= -l;
+            at(0, i) = l;
+            at(1, i) = kappa * ib[i];
+            at(2, i) = kappa * ib[i] * h;
+            at(3, i) = i + 1 < n ? g[i + 1] : 0.0;
+        }
+        Af[lane] = h;
+        h = 1.0;
+        for (int i = r1 - 1; i >= r0; i--) { h *= -at(3, i); at(4, i) = h; }
+        Ab[lane] = h;
+    }
+    for (int d = 0, off = 1; d < 5; d++, off <<= 1) {
+        double nf[32], nb[32];
+        for (int q = 0; q < 32; q++) {
+            pf[d * 32 + q] = Af[q];
+            pb[d * 32 + q] = Ab[q];
+            nf[q] = (q >= off) ? Af[q] * Af[q - off] : Af[q];
+            nb[q] = (q + off < 32) ? Ab[q] * Ab[q + off] : Ab[q];
+        }
+        std::copy(nf, nf + 32, Af);
+        std::copy(nb, nb + 32, Ab);
+    }
+    for (int q = 0; q < 8; q++)
+        for (int e = 0; e < 32; e++) T[160 * S + 320 + 32 * q + e] = xl::end_weight(op, e, q, wt);
+    int r = upload(&t.xt, T);
+    return r ? r : upload(&t.xtf, std::vector<float>(T.begin(), T.end()));
 }
 
 // lhs5 (loop_par.f:258-299) + ludecomp (penta_par.f:6-50), 1-based (n,5).
@@ -212,6 +214,12 @@ void ludecomp(int n, const std::vector<double>& a, std::vector<double>& lu) {
 }
 
 }  // namespace
+
+// The filter's weights (filter_par.f:181-332) in units of its centre weight.
+xl::Weights tb_filter_weights(double al) {
+    const double af = (11.0 + 10.0 * al) / 16.0, u = af != 0.0 ? af : 1.0;
+    return {af / u, (15.0 + 34.0 * al) / 64.0 / u, (-3.0 + 6.0 * al) / 32.0 / u, (1.0 - 2.0 * al) / 64.0 / u, 0.0625 / u};
+}
 
 // band5_poi (penta_par.f:308-364): NR banded LU, m1 = m2 = 2, no pivoting.
 // Returns per row (0-based j): L1 = al(j-1,1), L2 = al(j-2,2), U1 = a(j,2),
@@ -336,14 +344,15 @@ int tb_host_build_tables(tb_ctx* c) {
         a[0] = 0; b[0] = 1; cc[0] = 0; a[1] = 1; b[1] = 6; cc[1] = 2;
         for (int i = 2; i < nx - 2; i++) { a[i] = 1; b[i] = 3; cc[i] = 1; }
         a[nx - 2] = 2; b[nx - 2] = 6; cc[nx - 2] = 1; a[nx - 1] = 4; b[nx - 1] = 1; cc[nx - 1] = 0;
-        if ((r = upload_tri(c->tx1, a, b, cc, true))) return r;
+        if ((r = upload_xline(c->tx1, xl::D1, {}, a, b, cc, 1.0 / (12.0 * cf.dx)))) return r;
         a[0] = 0; b[0] = 13; cc[0] = 137; a[1] = 1; b[1] = 12; cc[1] = 3;
         for (int i = 2; i < nx - 2; i++) { a[i] = 2; b[i] = 11; cc[i] = 2; }
         a[nx - 2] = 3; b[nx - 2] = 12; cc[nx - 2] = 1; a[nx - 1] = 137; b[nx - 1] = 13; cc[nx - 1] = 0;
-        if ((r = upload_tri(c->tx2, a, b, cc, true))) return r;
+        if ((r = upload_xline(c->tx2, xl::D2, {}, a, b, cc, 3.0 / (4.0 * cf.dx * cf.dx)))) return r;
         std::fill(a.begin(), a.end(), 0.0); std::fill(b.begin(), b.end(), 1.0); std::fill(cc.begin(), cc.end(), 0.0);
         for (int i = 3; i < nx - 3; i++) { a[i] = cf.alphaf; cc[i] = cf.alphaf; }
-        if ((r = upload_tri(c->tfil, a, b, cc, true))) return r;
+        const double af = (11.0 + 10.0 * cf.alphaf) / 16.0;
+        if ((r = upload_xline(c->tfil, xl::FILTER, tb_filter_weights(cf.alphaf), a, b, cc, af != 0.0 ? af : 1.0))) return r;
     }
     // y compact LHS (coefy/coefy_fv/coeffy derivs_par.f:1040-1142) and RHS row weights
     {

@@ -39,17 +39,11 @@ struct TriLHS {
     double* a;   // (n)
     double* g;   // (n) gam
     double* ib;  // (n) 1/bet
-    // Chunked form for one warp per line (x-lines): lane t owns rows
-    // [tS, min(n, tS + S)).  hf_i = d u_i / d u_{tS-1} of the forward sweep,
-    // hb_i = d x_i / d x_{tS+S} of the backward sweep, and the Kogge-Stone
-    // step factors pf[d][t], pb[d][t] of the chunk-end (start) responses.
-    double* hf = nullptr;   // (n)
-    double* hb = nullptr;   // (n)
-    double* pf = nullptr;   // (5, 32)
-    double* pb = nullptr;   // (5, 32)
+    // x-lines, S rows per lane: the row tables of
+    // tb_xline.cuh, and their FP32 copy (lines of the mixed form's modes k >= 1)
+    double* xt = nullptr;
+    float* xtf = nullptr;
     int S = 0;
-    // FP32 copies of the chunked form (lines of the mixed form's modes k >= 1)
-    float *af = nullptr, *gf = nullptr, *ibf = nullptr, *hff = nullptr, *hbf = nullptr, *pff = nullptr, *pbf = nullptr;
 };
 // Row weights of the stretched-y compact RHS: row j (0-based) is
 // sum_m w[7*j+m] * f[j + off[j] + m], m < cnt[j].
@@ -184,9 +178,12 @@ void tb_poisson_band_matrix_dx(const tb_ctx* c, int type, int lvl, int k, double
 void tb_band5_factor(int n, std::vector<double>& a, double* L1, double* L2, double* U1, double* U2, double* ID);
 
 // ---- kernel launchers ------------------------------------------------------
-// Batched x-line operators (derivs_par.f:80-113, filter_par.f:144-177).
+namespace xl { struct Weights; }
+xl::Weights tb_filter_weights(double alphaf);   // filter stencil (tb_host.cpp)
+// Batched x-line operators (derivs_par.f:80-113, filter_par.f:144-177).  The
+// filter's jobs of one call are all in place (src = dst) or none.
 enum XOp { XOP_D1 = 0, XOP_D2 = 1, XOP_FILTER = 2 };
-struct XJob { const cplx* src; cplx* dst; int op; };  // src and dst must not alias
+struct XJob { const cplx* src; cplx* dst; int op; };
 int tb_launch_xlines(tb_ctx* c, const XJob* jobs, int njobs);
 enum YOp { YOP_D1 = 0, YOP_D1FV = 1, YOP_D2 = 2 };
 struct YJob { const cplx* src; cplx* dst; int op; };

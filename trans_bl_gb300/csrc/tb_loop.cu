@@ -117,16 +117,6 @@ __global__ void k_outuy_bc(cplx* uy, const double* uyb, int nx, int ny, int K, i
     uy[q] = ((form == 0 || form == 4) && k == 0) ? make_double2(uyb[(nx - 1) + (size_t)nx * j], 0.0) : make_double2(0.0, 0.0);
 }
 
-// filter_trid copy-back (filter_par.f:166-174): i >= 2, j >= 2.
-__global__ void k_copy_inner(cplx* dst, const cplx* src, int nx, int ny, int K) {
-    size_t n = (size_t)nx * ny * K;
-    size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (q >= n) return;
-    int i = (int)(q % nx), j = (int)((q / nx) % ny);
-    if (i < 1 || j < 1) return;
-    dst[q] = src[q];
-}
-
 // ---------------------------------------------------------------------------
 // x-direction recurrences, one warp per line (tb_warp.cuh).  Shared memory
 // per warp: two line buffers of 32 x Sp complex (inputs E, rows V).
@@ -549,16 +539,10 @@ int tb_rk_update(tb_ctx* c, int stage) {
     return c->cfg.my_form == 2 ? tb_rk_update_th(c, stage) : TB_OK;
 }
 
+// filter_trid (filter_par.f:144-177), in place on rows i >= 2, j >= 2 (1-based)
 int tb_filter(tb_ctx* c) {
-    cplx** t = c->tmp;
-    XJob xj[3] = {{c->wx, t[0], XOP_FILTER}, {c->wy, t[1], XOP_FILTER}, {c->wz, t[2], XOP_FILTER}};
-    int r;
-    if ((r = tb_launch_xlines(c, xj, 3))) return r;
-    unsigned nb = tb_blocks(tb_n3(c), 256);
-    k_copy_inner<<<nb, 256, 0, c->stream>>>(c->wx, t[0], c->g.nx, c->g.ny, c->g.K); TB_CHECK_LAUNCH(c);
-    k_copy_inner<<<nb, 256, 0, c->stream>>>(c->wy, t[1], c->g.nx, c->g.ny, c->g.K); TB_CHECK_LAUNCH(c);
-    k_copy_inner<<<nb, 256, 0, c->stream>>>(c->wz, t[2], c->g.nx, c->g.ny, c->g.K); TB_CHECK_LAUNCH(c);
-    return TB_OK;
+    XJob xj[3] = {{c->wx, c->wx, XOP_FILTER}, {c->wy, c->wy, XOP_FILTER}, {c->wz, c->wz, XOP_FILTER}};
+    return tb_launch_xlines(c, xj, 3);
 }
 
 int tb_bzone_k(tb_ctx* c) {
