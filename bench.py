@@ -492,7 +492,7 @@ def main():
         achieved = flops / (r_ms * 1e-3 / max(r_n, 1)) / 1e12 if r_n else 0.0
         roof = {"bound": "fp64", "achieved": achieved, "peak": fp64, "unit": "TFLOP/s", "frac": achieved / fp64,
                 "traffic": None, "peak_source": "measured in this run (tb_fp64_peak: FMA chains, 2 flops each)",
-                "kernel": "k_wsor (wavefront of lexicographic y-line sweeps, one CTA per mode and part)",
+                "kernel": "k_wsor (wavefront of lexicographic y-line sweeps, one cluster per mode and part)",
                 "algorithmic_flops_per_call": flops, "kernel_ms_total": r_ms, "kernel_calls": r_n,
                 "share_of_step": r_ms / prof_ms if prof_ms > 0 else None}
     else:

@@ -16,44 +16,62 @@
 //    ptsx-1 at step ptsx-8+5s (0-based line indices 1 and ptsx-2).  Every line
 //    solve then reads exactly the values the sequential order gives it, and
 //    no two solves of one step touch a line that the other writes (the
-//    border stencils reach 4 lines inwards, which sets the lag of 5).
-//  - The lines of fc and sc the sweeps in flight touch sit in 32-line rings
-//    in shared memory (each line read from and written to global memory once
-//    per group of up to five sweeps, the next line prefetched while a step
-//    solves); a level small enough is held whole.
-//  - Each line solve (band LU factored once at set-up) runs on a group of 1,
-//    2 or 4 warps: row chunks with local recurrences and zero carry, a warp
-//    scan of the chunk-end 2x2 propagators, the warps chained through shared
-//    memory, and a fix-up with precomputed homogeneous responses.  On GB300
-//    an FP64 warp instruction holds its sub-partition's FP64 pipe for ~64
-//    cycles whatever the number of active lanes, so a line's latency is set
-//    by the FP64 instructions per warp: one sweep in flight spreads each line
-//    over four warps (all four sub-partitions), several sweeps over two.
+//    border stencils reach 4 lines inwards, which sets the lag of 5).  The last
+//    sweep of a V-cycle on the fine level runs in one wavefront with the first
+//    three of the next.
+//  - What a step costs is the FP64 instructions of one line solve: a warp's
+//    holds its sub-partition's FP64 pipe for ~64 cycles whatever the number of
+//    active lanes.  So the sweeps of a wavefront sit on different SMs, in the
+//    CTAs of a cluster, and a line on all four sub-partitions of its SM, one
+//    row a lane where 128 lanes suffice (k_wsor).
 // Defect, restriction, correction and interpolation are grid-parallel.
 #include "tb_internal.h"
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 
 namespace {
 
 constexpr int LAG = 5;      // steps between successive sweeps of the wavefront
-constexpr int RING = 32;    // lines in the shared-memory rings (streamed levels)
-constexpr int MAX_STREAM_SWEEPS = 5;   // sweeps in flight that fit the ring: LAG*(5-1) + 10 <= 32
-constexpr int WARP_TAB = 1544;         // per warp of a line group: Pf 640, Pb 640, R 128, Q 128, A 4, B 4
-constexpr int NGROUP = 3;              // line groups of 1, 2 and 4 warps
-constexpr int PREFETCH = 4;            // line elements a thread prefetches into registers per ring
+constexpr int RING = 16;    // lines of a slot's ring: a sweep and the one behind it touch 14
+constexpr int NGROUP = 3;   // line groups of 1, 2 and 4 warps
+constexpr int MAX_CLUSTER = 8;
 
 __host__ __device__ inline int group_warps(int gi) { return 1 << gi; }
-__host__ __device__ inline int rows_per_lane(int n, int G) { int s = (n + 32 * G - 1) / (32 * G); return s < 1 ? 1 : s; }
-// one (group, type, level, mode) block of line-solve tables: L1 L2 U1 U2 ID
-// h1 h2 k1 k2 (n each, compact), then WARP_TAB doubles per warp of the group
-__host__ __device__ inline int tab_size(int n, int G) { return 9 * n + WARP_TAB * G; }
-__host__ __device__ inline size_t tab_block(int ny) { return (size_t)tab_size(ny, 4); }
+// Rows per lane of a line of n points (rows 1 .. n-1) on G warps, rounded up to
+// a size the kernel is built for.
+__host__ __device__ inline int rows_per_lane(int n, int G) {
+    const int s = (n - 1 + 32 * G - 1) / (32 * G);
+    return s <= 4 ? (s < 1 ? 1 : s) : s <= 6 ? 6 : s <= 8 ? 8 : s <= 12 ? 12 : 16;
+}
+// Line-solve tables of one (group, type, level, mode): entry e of chunk c (lane
+// c % 32 of warp c / 32, rows 1 + c S .. c S + S) at e * 32 G + c.
+//   per row s, from 8 s: weights WL WC WR of the x-stencil sums of rows j-1, j,
+//     j+1 in the right-hand side (negative), L1 L2, U1 U2 (times ID), ID
+//   WZ  -L times the fixed value of row 0, rows 1 and 2 (entries of rows s < 2)
+//   S > 2: per row the responses H1 H2 (forward) and K1 K2 (backward) to the
+//     states entering the chunk
+//   PF, PB  5 x 4: Kogge-Stone matrices of the chunk propagators in a warp
+//   CF, CB  3 x (4; S = 1: 2): response of the chunk's rows (S <= 2) or of the state
+//     entering it (S > 2) to the state leaving warp w of those before (after) it
+__host__ __device__ constexpr int tab_wz(int S) { return 8 * S; }
+__host__ __device__ constexpr int tab_h(int S) { return 8 * S + (S < 2 ? 1 : 2); }
+__host__ __device__ constexpr int tab_pf(int S) { return tab_h(S) + (S > 2 ? 4 * S : 0); }
+__host__ __device__ constexpr int tab_pb(int S) { return tab_pf(S) + 20; }
+__host__ __device__ constexpr int tab_cw(int S) { return S == 1 ? 2 : 4; }
+__host__ __device__ constexpr int tab_cf(int S) { return tab_pb(S) + 20; }
+__host__ __device__ constexpr int tab_cb(int S) { return tab_cf(S) + 3 * tab_cw(S); }
+__host__ __device__ constexpr int tab_entries(int S) { return tab_cb(S) + 3 * tab_cw(S); }
+__host__ __device__ inline int tab_size(int n, int G) { return tab_entries(rows_per_lane(n, G)) * 32 * G; }
+__host__ __device__ inline size_t tab_block(int ny) {
+    const int a = tab_size(ny, 1), b = tab_size(ny, 2), c = tab_size(ny, 4), m = a > b ? a : b;
+    return (size_t)(m > c ? m : c);
+}
 
 struct PlainDev {
     double *fc, *sc, *fct, *def;   // per block b = 2k + part: pelems doubles (fc, sc, fct), dstride (def)
-    const double* tab;             // line-solve tables per (group, type, level, mode), blocks of tab_block(ny)
+    const double* tab;             // line-solve tables per (group, type, level, mode), blocks of tabs
     const double* coef;            // sp(7) cp(8) pp(4) lp(5) per level
     const double* qdy2;            // (ny, msh)
     const double* k2b2;
@@ -62,267 +80,376 @@ struct PlainDev {
     unsigned long long* maxsq;     // per mode: max |defect|^2 of the fine level (double bits)
     int nx, ny, K, msh;
     int ptsx[TB_MAX_MSH], ptsy[TB_MAX_MSH];
-    size_t off[TB_MAX_MSH], pelems, dstride;
+    size_t off[TB_MAX_MSH], pelems, dstride, tabs;
     double den[TB_MAX_MSH];        // 1 / (12 dx2 fac_y)
     double fac_y, alpha, ify;
 };
 
 __device__ __forceinline__ const double* tab_ptr(const PlainDev& P, int gi, int type, int l, int k) {
-    return P.tab + ((((size_t)gi * 2 + type) * P.msh + l) * P.K + k) * tab_block(P.ny);
+    return P.tab + ((((size_t)gi * 2 + type) * P.msh + l) * P.K + k) * P.tabs;
 }
 
 __device__ __forceinline__ void group_barrier(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+__device__ __forceinline__ void push(uint32_t addr, double v) {   // into a CTA of the cluster
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t in_cta(const double* p, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // One y-line solve of sor on a group of G warps: rhs_center / rhs_border1 /
 // rhs_border2 (poisson_par.f:343-540), banbk5_poi (penta_par.f:367-404) and
-// fc = fc + rf (x - fc) for rows j >= 1 (0-based).  The rows are cut into
-// 32 G chunks of S rows (warp g, lane t owns chunk 32 g + t); each chunk runs
-// its local recurrences with zero carry, the chunk-end 2x2 propagators are
-// scanned within each warp (Kogge-Stone), the warp totals are chained through
-// shared memory, and every row is fixed up with its precomputed homogeneous
-// responses.  The x-stencil lines come as pointers into shared memory: for a
-// centre line (i-2, i-1, i+1, i+2), for a border line the four inner lines in
-// order of distance and the outer line.  TR: row tables (stride n); TW: the
-// group's warp tables.
-template <int S, int G, bool BORDER>
-__device__ __forceinline__ void line_solve(const double* __restrict__ TR, const double* __restrict__ TW, int n,
-                                           const double* a0, const double* a1, const double* a2, const double* a3,
-                                           const double* a4, double* F, const double* SC, const double* cf, double qx,
-                                           double rf, int g, int lane, double* xch, int bar) {
-    // rhs = sc - qx (weights . g), with qx folded into the weights
-    const double sp2 = qx * cf[1], sp3 = qx * cf[2], cp1 = qx * cf[7], cp2 = qx * cf[8], cp3 = qx * cf[9];
-    const int r0 = (32 * g + lane) * S, r1 = min(n, r0 + S);
-    // x-stencil sums of rows r0-1 .. r0+S (index q = row - r0 + 1)
-    double gs[S + 2];
+// fc + rf (x - fc) for the rows j >= 1 (0-based), S rows a lane.  Each chunk
+// runs its local recurrences with zero carry, the chunk-end 2x2 propagators
+// are scanned within each warp (Kogge-Stone, `lv` levels), and the states
+// leaving the other warps enter through precomputed responses.  With one or
+// two rows a lane the scanned state is the rows themselves.  Row 0 keeps its
+// value f0, which enters rows 1 and 2.  Rows past the line have zero tables.
+//
+// FP64 instructions a warp, four warps of one row a lane: 3 stencil, 3 weights,
+// 1 + 16 scan and up to 6 for the other warps in each direction, 1 scaling, 2
+// update: 55 of ~64 cycles.  The x-stencil lines come as pointers to the
+// chunk's rows (stride NC = 32 G): for a centre line (i-2, i-1, i+1, i+2), for
+// a border line the four inner lines in order of distance and the outer line.
+template <int S>
+__device__ __forceinline__ void line_solve(bool border, const double* T, int G, int g, int lane, int lv, const double* a0,
+                                           const double* a1, const double* a2, const double* a3, const double* a4,
+                                           const double* F, const double (&sc)[S], double f0, double rf, double (&out)[S],
+                                           double* xch, int bar) {
+    const int NC = 32 * G, c = 32 * g + lane;
+    const double* t = T + c;
+    auto tab = [&](int e) { return t[e * NC]; };
+    // x-stencil sums of the chunk's rows, and of the row on either side
+    double gs[S];
+    if (!border) {
 #pragma unroll
-    for (int q = 0; q < S + 2; q++) {
-        const int j = r0 - 1 + q;
-        double v = 0.0;
-        if (j >= 1 && j < n) {
-            if (!BORDER) v = -a0[j] + 16.0 * a1[j] + 16.0 * a2[j] - a3[j];   // -(1 f(i-2)) + 16 f(i-1) + 16 f(i+1) - 1 f(i+2)
-            else v = 10.0 * a4[j] - 4.0 * a0[j] + 14.0 * a1[j] - 6.0 * a2[j] + a3[j];
-        }
-        gs[q] = v;
+        for (int s = 0; s < S; s++) gs[s] = fma(16.0, a1[s * NC] + a2[s * NC], -(a0[s * NC] + a3[s * NC]));
+    } else {
+#pragma unroll
+        for (int s = 0; s < S; s++)
+            gs[s] = 10.0 * a4[s * NC] - 4.0 * a0[s * NC] + 14.0 * a1[s * NC] - 6.0 * a2[s * NC] + a3[s * NC];
     }
-    const double *L1 = TR, *L2 = TR + n, *U1 = TR + 2 * n, *U2 = TR + 3 * n, *ID = TR + 4 * n;
-    const double *h1 = TR + 5 * n, *h2 = TR + 6 * n, *k1 = TR + 7 * n, *k2 = TR + 8 * n;
-    const double* Tg = TW + WARP_TAB * g;
-    const double *Pf = Tg, *Pb = Tg + 640, *Rm = Tg + 1280 + 4 * lane, *Qm = Tg + 1408 + 4 * lane;
+    double gm = __shfl_up_sync(0xffffffffu, gs[S - 1], 1), gp = __shfl_down_sync(0xffffffffu, gs[0], 1);
+    if (G > 1) {
+        if (lane == 0) xch[2 * g] = gs[0];
+        if (lane == 31) xch[2 * g + 1] = gs[S - 1];
+        group_barrier(bar, 32 * G);
+        if (lane == 0 && g > 0) gm = xch[2 * (g - 1) + 1];
+        if (lane == 31 && g + 1 < G) gp = xch[2 * (g + 1)];
+    }
     double y[S];
-    double ym1 = 0.0, ym2 = 0.0;
 #pragma unroll
     for (int s = 0; s < S; s++) {
-        const int j = r0 + s;
-        if (j < r1) {
-            double r;
-            if (j == 0) r = F[0];
-            else if (j == 1) r = SC[j] - sp3 * gs[s + 2] - sp2 * gs[s + 1];
-            else if (j <= n - 3) r = SC[j] - cp1 * gs[s] - cp2 * gs[s + 1] - cp3 * gs[s + 2];
-            else if (BORDER) r = SC[j] - qx * gs[s + 1];
-            else r = SC[j] - qx * (-(a3[j] + a0[j]) + 16.0 * (a2[j] + a1[j]));   // rhs_center's two top rows
-            const double yy = r - L2[j] * ym2 - L1[j] * ym1;
-            y[s] = yy; ym2 = ym1; ym1 = yy;
-        }
+        double r = fma(tab(8 * s + 1), gs[s], sc[s]);
+        r = fma(tab(8 * s), s ? gs[s > 0 ? s - 1 : 0] : gm, r);
+        r = fma(tab(8 * s + 2), s + 1 < S ? gs[s + 1 < S ? s + 1 : 0] : gp, r);
+        if (s < 2 && g == 0) r = fma(tab(tab_wz(S) + s), f0, r);
+        if (s > 0) r = fma(-tab(8 * s + 3), y[s > 0 ? s - 1 : 0], r);
+        if (s > 1) r = fma(-tab(8 * s + 4), y[s > 1 ? s - 2 : 0], r);
+        y[s] = r;
     }
     // forward: scan of the chunk-end states (y_e, y_{e-1}) within the warp
-    double b0 = ym1, b1 = ym2;
+    double b0 = y[S - 1], b1 = S > 1 ? y[S > 1 ? S - 2 : 0] : 0.0;
 #pragma unroll
     for (int d = 0, off = 1; d < 5; d++, off <<= 1) {
+        if (d >= lv) break;
         const double o0 = __shfl_up_sync(0xffffffffu, b0, off), o1 = __shfl_up_sync(0xffffffffu, b1, off);
         if (lane >= off) {
-            const double* M = Pf + (d * 32 + lane) * 4;
-            const double n0 = b0 + M[0] * o0 + M[1] * o1;
-            const double n1 = b1 + M[2] * o0 + M[3] * o1;
-            b0 = n0; b1 = n1;
+            const int e = tab_pf(S) + 4 * d;
+            if (S == 1 && d == 0) {   // one row: the propagator is (m0 m1; 1 0)
+                b0 = fma(tab(e), o0, b0);
+                b1 = o0;
+            } else {
+                b0 = fma(tab(e), o0, fma(tab(e + 1), o1, b0));
+                b1 = fma(tab(e + 2), o0, fma(tab(e + 3), o1, b1));
+            }
         }
     }
-    double Y1 = __shfl_up_sync(0xffffffffu, b0, 1), Y2 = __shfl_up_sync(0xffffffffu, b1, 1);
-    if (lane == 0) { Y1 = 0.0; Y2 = 0.0; }
+    double* xf = xch + 2 * G;
     if (G > 1) {
-        // the warps' outgoing states, chained in order: z = state entering warp g
-        if (lane == 31) { xch[4 * g] = b0; xch[4 * g + 1] = b1; }
+        if (lane == 31) { xf[2 * g] = b0; xf[2 * g + 1] = b1; }
         group_barrier(bar, 32 * G);
-        double z0 = 0.0, z1 = 0.0;
-        for (int w = 0; w < g; w++) {
-            const double* A = TW + WARP_TAB * w + 1536;
-            const double n0 = xch[4 * w] + A[0] * z0 + A[1] * z1;
-            const double n1 = xch[4 * w + 1] + A[2] * z0 + A[3] * z1;
-            z0 = n0; z1 = n1;
-        }
-        Y1 = Y1 + Rm[0] * z0 + Rm[1] * z1;
-        Y2 = Y2 + Rm[2] * z0 + Rm[3] * z1;
+    }
+    constexpr int CW = tab_cw(S);
+    if (S > 2) {
+        b0 = __shfl_up_sync(0xffffffffu, b0, 1);
+        b1 = __shfl_up_sync(0xffffffffu, b1, 1);
+        if (lane == 0) { b0 = 0.0; b1 = 0.0; }
     }
 #pragma unroll
-    for (int s = 0; s < S; s++) {
-        const int j = r0 + s;
-        if (j < r1) y[s] = y[s] + h1[j] * Y1 + h2[j] * Y2;
+    for (int w = 0; w < 3; w++)
+        if (w < g) {
+            const double z0 = xf[2 * w], z1 = xf[2 * w + 1];
+            const int e = tab_cf(S) + CW * w;
+            b0 = fma(tab(e), z0, fma(tab(e + 1), z1, b0));
+            if (S > 1) b1 = fma(tab(e + (S > 1 ? 2 : 0)), z0, fma(tab(e + (S > 1 ? 3 : 0)), z1, b1));
+        }
+    if (S <= 2) {
+        y[S - 1] = b0;
+        if (S == 2) y[0] = b1;
+    } else {
+#pragma unroll
+        for (int s = 0; s < S; s++) y[s] = fma(tab(tab_h(S) + 4 * s), b0, fma(tab(tab_h(S) + 4 * s + 1), b1, y[s]));
     }
-    double xp1 = 0.0, xp2 = 0.0;
+    // backward, likewise from the high lanes
 #pragma unroll
     for (int s = S - 1; s >= 0; s--) {
-        const int j = r0 + s;
-        if (j < r1) {
-            const double xx = (y[s] - U1[j] * xp1 - U2[j] * xp2) * ID[j];
-            y[s] = xx; xp2 = xp1; xp1 = xx;
-        }
+        double x = tab(8 * s + 7) * y[s];
+        if (s + 1 < S) x = fma(-tab(8 * s + 5), y[s + 1 < S ? s + 1 : 0], x);
+        if (s + 2 < S) x = fma(-tab(8 * s + 6), y[s + 2 < S ? s + 2 : 0], x);
+        y[s] = x;
     }
-    // backward: scan of the chunk-start states (x_s, x_{s+1}) from the high lanes
-    b0 = xp1; b1 = xp2;
+    b0 = y[0]; b1 = S > 1 ? y[S > 1 ? 1 : 0] : 0.0;
 #pragma unroll
     for (int d = 0, off = 1; d < 5; d++, off <<= 1) {
+        if (d >= lv) break;
         const double o0 = __shfl_down_sync(0xffffffffu, b0, off), o1 = __shfl_down_sync(0xffffffffu, b1, off);
         if (lane + off < 32) {
-            const double* M = Pb + (d * 32 + lane) * 4;
-            const double n0 = b0 + M[0] * o0 + M[1] * o1;
-            const double n1 = b1 + M[2] * o0 + M[3] * o1;
-            b0 = n0; b1 = n1;
+            const int e = tab_pb(S) + 4 * d;
+            if (S == 1 && d == 0) {
+                b0 = fma(tab(e), o0, b0);
+                b1 = o0;
+            } else {
+                b0 = fma(tab(e), o0, fma(tab(e + 1), o1, b0));
+                b1 = fma(tab(e + 2), o0, fma(tab(e + 3), o1, b1));
+            }
         }
     }
-    double X1 = __shfl_down_sync(0xffffffffu, b0, 1), X2 = __shfl_down_sync(0xffffffffu, b1, 1);
-    if (lane == 31) { X1 = 0.0; X2 = 0.0; }
+    double* xb = xch + 4 * G;
     if (G > 1) {
-        if (lane == 0) { xch[4 * g + 2] = b0; xch[4 * g + 3] = b1; }
+        if (lane == 0) { xb[2 * g] = b0; xb[2 * g + 1] = b1; }
         group_barrier(bar, 32 * G);
-        double z0 = 0.0, z1 = 0.0;
-        for (int w = G - 1; w > g; w--) {
-            const double* B = TW + WARP_TAB * w + 1540;
-            const double n0 = xch[4 * w + 2] + B[0] * z0 + B[1] * z1;
-            const double n1 = xch[4 * w + 3] + B[2] * z0 + B[3] * z1;
-            z0 = n0; z1 = n1;
+    }
+    if (S > 2) {
+        b0 = __shfl_down_sync(0xffffffffu, b0, 1);
+        b1 = __shfl_down_sync(0xffffffffu, b1, 1);
+        if (lane == 31) { b0 = 0.0; b1 = 0.0; }
+    }
+#pragma unroll
+    for (int w = 0; w < 3; w++)
+        if (g + 1 + w < G) {   // the warps after this one
+            const double z0 = xb[2 * (g + 1 + w)], z1 = xb[2 * (g + 1 + w) + 1];
+            const int e = tab_cb(S) + CW * w;
+            b0 = fma(tab(e), z0, fma(tab(e + 1), z1, b0));
+            if (S > 1) b1 = fma(tab(e + (S > 1 ? 2 : 0)), z0, fma(tab(e + (S > 1 ? 3 : 0)), z1, b1));
         }
-        X1 = X1 + Qm[0] * z0 + Qm[1] * z1;
-        X2 = X2 + Qm[2] * z0 + Qm[3] * z1;
+    if (S <= 2) {
+        y[0] = b0;
+        if (S == 2) y[S - 1] = b1;
+    } else {
+#pragma unroll
+        for (int s = 0; s < S; s++) y[s] = fma(tab(tab_h(S) + 4 * s + 2), b0, fma(tab(tab_h(S) + 4 * s + 3), b1, y[s]));
     }
 #pragma unroll
     for (int s = 0; s < S; s++) {
-        const int j = r0 + s;
-        if (j < r1 && j >= 1) {
-            const double xx = y[s] + k1[j] * X1 + k2[j] * X2;
-            const double fo = F[j];
-            F[j] = fo + rf * (xx - fo);
+        out[s] = y[s];
+        if (rf != 1.0) {
+            const double fo = F[s * NC];
+            out[s] = fma(rf, y[s] - fo, fo);
         }
     }
 }
 
-// `ns` lexicographic sweeps at level l, all (mode, part) blocks with an active
-// mode, each line solved by a group of G warps (table group gi).  whole = 1:
-// the level's fc and sc are held whole in shared memory (any ns); else their
-// lines stream through rings of RING lines (ns <= MAX_STREAM_SWEEPS), the
-// next line prefetched into registers while the current step's lines solve.
-template <int S, int G>
-__global__ void k_wsor(PlainDev P, int l, int ns, double rf, int whole, int gi) {
-    const int b = blockIdx.x, k = b >> 1;
-    if (!P.state[2 * k]) return;   // uniform over the block
-    const int nxl = P.ptsx[l], n = P.ptsy[l], m = nxl - 2;
+// Shapes of one k_wsor launch.
+struct Wave {
+    int l, ns, gi;      // level, sweeps, line group
+    int C, W;           // CTAs of a cluster, line groups (slots) of a CTA
+    int lv;             // scan levels
+    int seq;            // too few lines for the wavefront: the reference's order on one group
+    int parity;         // rings per slot: 2 where a slot runs several sweeps
+    int staged;         // tables in shared memory: 2 both types, 1 the centre lines'
+    double rf0, rf;     // relaxation factor of the first sweep and of the others
+};
+__host__ __device__ inline size_t wave_lines(const Wave& v, int NC, int S) {
+    return ((size_t)v.W * v.parity * RING + 2) * NC * S;
+}
+
+// `ns` lexicographic sweeps at level l of one (mode, part) with an active mode
+// on one cluster.  A slot is a group of G warps with a ring of lines; slot q of
+// the cluster's C W runs the sweeps q, q + C W, ...  The first sweep reads its
+// lines from global memory, every sweep hands each relaxed line to the ring
+// of the slot behind it (in another CTA through distributed shared memory),
+// and the last one writes it back; one cluster barrier a step orders this.
+// A further group per CTA solves the far border line of its slots' sweeps
+// beside their centre lines.  A slot that runs several sweeps alternates
+// between two rings.
+//
+// One CTA per (mode, part), two warps a line and all sweeps of a wavefront on
+// the SM's four FP64 pipes took 361 ms a step at 385 x 129 x 1 and 450 ms at
+// 513 x 129 x 8; this takes 134 and 180 ms, 3.4 us a step of the wavefront of four
+// sweeps on 129 rows.
+// STAGED: both types' tables fit shared memory beside the rings, and every load
+// of a solve is one from shared memory.
+template <int S, bool STAGED>
+__global__ void __launch_bounds__(256) k_wsor(PlainDev P, Wave V) {
+    const int C = V.C, rank = blockIdx.x % C, b = blockIdx.x / C, k = b >> 1, l = V.l;
+    if (!P.state[2 * k]) return;   // uniform over the cluster
+    const int nxl = P.ptsx[l], n = P.ptsy[l], m = nxl - 2, ns = V.ns;
+    const int G = 1 << V.gi, NC = 32 * G, LS = NC * S, W = V.W, NS = C * W;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int grp = warp >> V.gi, g = warp & (G - 1), c = 32 * g + lane;
     extern __shared__ double smem[];
-    const int tsz = tab_size(n, G);
-    const int lines = whole ? nxl : RING;
-    double* tabc = smem;                               // centre-line tables
-    double* fcb = smem + tsz;                          // fc lines
-    double* scb = fcb + (size_t)lines * n;             // sc lines
-    double* xch = scb + (size_t)lines * n;             // group exchange, 4 G per group
-    const double* tabb = tab_ptr(P, gi, 1, l, k);      // border-line tables (global, cached)
-    {
-        const double* tg = tab_ptr(P, gi, 0, l, k);
-        for (int q = threadIdx.x; q < tsz; q += blockDim.x) tabc[q] = tg[q];
-    }
+    double* rings = smem;                                        // (W, parity, RING, S, NC)
+    double* edge = rings + (size_t)W * V.parity * RING * LS;     // lines 0 and nxl - 1
+    double* xch = edge + 2 * LS + 6 * G * grp;                   // group exchange
+    double* ts = edge + 2 * LS + 6 * G * (W + 1);                // staged tables
+    const double *tc = tab_ptr(P, V.gi, 0, l, k), *tb = tab_ptr(P, V.gi, 1, l, k);
     double* Fg = P.fc + (size_t)b * P.pelems + P.off[l];
     const double* SCg = P.sc + (size_t)b * P.pelems + P.off[l];
-    const double* cf = P.coef + 24 * l;
-    const double qx = P.den[l];
-    const int nth = blockDim.x, tid = threadIdx.x;
-    const int warp = tid >> 5, lane = tid & 31;
-    const int grp = warp / G, g = warp % G, W = (blockDim.x >> 5) / G;
-    double* gx = xch + 4 * G * grp;
-    const int bar = 1 + grp;
-    auto FL = [&](int q) -> double* { return fcb + (size_t)(whole ? q : (q & (RING - 1))) * n; };
-    auto SL = [&](int q) -> double* { return scb + (size_t)(whole ? q : (q & (RING - 1))) * n; };
-    auto centre = [&](int i) {
-        line_solve<S, G, false>(tabc, tabc + 9 * n, n, FL(i - 2), FL(i - 1), FL(i + 1), FL(i + 2), nullptr, FL(i), SL(i),
-                                cf, qx, rf, g, lane, gx, bar);
-    };
-    auto border1 = [&]() {
-        line_solve<S, G, true>(tabb, tabb + 9 * n, n, FL(2), FL(3), FL(4), FL(5), FL(0), FL(1), SL(1), cf, qx, rf, g,
-                               lane, gx, bar);
-    };
-    auto border2 = [&]() {
-        line_solve<S, G, true>(tabb, tabb + 9 * n, n, FL(m - 1), FL(m - 2), FL(m - 3), FL(m - 4), FL(m + 1), FL(m),
-                               SL(m), cf, qx, rf, g, lane, gx, bar);
-    };
-    const int first = whole ? nxl : min(nxl, 8);   // lines 0..7 are the first step's window
-    for (int q = tid; q < first * n; q += nth) {
-        const int line = q / n, j = q % n;
-        FL(line)[j] = Fg[(size_t)line * n + j];
-        SL(line)[j] = SCg[(size_t)line * n + j];
+    {
+        const int tsz = tab_entries(S) * NC;
+        if (STAGED || V.staged) {
+            for (int q = tid; q < tsz; q += blockDim.x) ts[q] = tc[q];
+            tc = ts;
+        }
+        if (STAGED) {
+            for (int q = tid; q < tsz; q += blockDim.x) ts[tsz + q] = tb[q];
+            tb = ts + tsz;
+        }
+        // rows past the line stay zero in every ring
+        for (int q = tid; q < W * V.parity * RING * LS; q += blockDim.x) rings[q] = 0.0;
     }
     __syncthreads();
-    if (m < 7) {
-        // too few lines for the wavefront: one warp in the reference's order
-        if (warp == 0) {
-            for (int s = 0; s < ns; s++) {
-                border1(); __syncwarp();
-                border2(); __syncwarp();
-                for (int i = 2; i <= m - 1; i++) { centre(i); __syncwarp(); }
-            }
-        }
-        __syncthreads();
-    } else {
-        const int T = m - 1 + LAG * (ns - 1);
-        int stored = 0;
-        double pf[PREFETCH], ps[PREFETCH];   // line t+8 of fc and sc in flight
-        auto fetch = [&](int line) {
+    const int row0 = 1 + c * S;   // the chunk's first row
+    auto ring = [&](int w, int s) { return rings + (size_t)(w * V.parity + (V.parity > 1 ? (s / NS) & 1 : 0)) * RING * LS; };
+    // line q of a sweep as its slot sees it, at the chunk's rows
+    auto at = [&](const double* R, int q) -> const double* {
+        return (q == 0 ? edge : q == nxl - 1 ? edge + LS : R + (size_t)(q & (RING - 1)) * LS) + c;
+    };
+    auto fill = [&](double* dst, int q) {
 #pragma unroll
-            for (int e = 0; e < PREFETCH; e++) {
-                const int j = tid + e * nth;
-                if (line < nxl && j < n) { pf[e] = Fg[(size_t)line * n + j]; ps[e] = SCg[(size_t)line * n + j]; }
-            }
-        };
-        if (!whole) fetch(8);
-        for (int t = 0; t < T; t++) {
-            for (int s = grp; s < ns; s += W) {
-                const int u = t - LAG * s;    // step within sweep s
-                if (u == 0) border1();
-                if (u >= 1 && u <= m - 2) centre(u + 1);
-                if (u == m - 6) border2();
-            }
-            __syncthreads();
-            if (!whole) {
-                // lines no task at step >= t+1 touches go back to global memory;
-                // line t+8 (step t+1's window edge) enters the rings
-                const int lo = max(0, t - LAG * (ns - 1));
-                for (int q = tid; q < (lo - stored) * n; q += nth) {
-                    const int line = stored + q / n, j = q % n;
-                    Fg[(size_t)line * n + j] = FL(line)[j];
-                }
-                stored = lo;
-                const int line = t + 8;
-                if (line < nxl) {
-#pragma unroll
-                    for (int e = 0; e < PREFETCH; e++) {
-                        const int j = tid + e * nth;
-                        if (j < n) { FL(line)[j] = pf[e]; SL(line)[j] = ps[e]; }
-                    }
-                    for (int j = tid + PREFETCH * nth; j < n; j += nth) {
-                        FL(line)[j] = Fg[(size_t)line * n + j];
-                        SL(line)[j] = SCg[(size_t)line * n + j];
-                    }
-                }
-                fetch(t + 9);
-                __syncthreads();
-            }
-        }
-        if (!whole) {
-            for (int q = tid; q < (nxl - stored) * n; q += nth) {
-                const int line = stored + q / n, j = q % n;
-                Fg[(size_t)line * n + j] = FL(line)[j];
-            }
-        }
+        for (int s = 0; s < S; s++) dst[s * NC + c] = (row0 + s < n) ? Fg[(size_t)q * n + row0 + s] : 0.0;
+    };
+    if (grp == 0) {
+        fill(edge, 0);
+        fill(edge + LS, nxl - 1);
+        if (rank == 0)
+            for (int q = 1; q <= min(m, 7); q++) fill(rings + (size_t)(q & (RING - 1)) * LS, q);
     }
-    if (whole) {
-        for (int q = tid; q < nxl * n; q += nth) Fg[q] = fcb[q];
+    if (C > 1) {
+        cluster_arrive();
+        cluster_wait();
+    } else __syncthreads();
+    auto load_sc = [&](int line, double (&v)[S], double& f0) {
+#pragma unroll
+        for (int s = 0; s < S; s++) v[s] = (row0 + s < n) ? SCg[(size_t)line * n + row0 + s] : 0.0;
+        if (g == 0) f0 = Fg[(size_t)line * n];
+    };
+    // the last sweep's line (0: none) on its way to global memory
+    int done = 0;
+    double res[S];
+    auto write_back = [&]() {
+        if (done) {
+#pragma unroll
+            for (int q = 0; q < S; q++)
+                if (row0 + q < n) Fg[(size_t)done * n + row0 + q] = res[q];
+            done = 0;
+        }
+    };
+    // relax line `line` of sweep s in slot w (of this CTA)
+    auto relax = [&](int w, int s, int line, const double (&sc)[S], double f0) {
+        double* R = ring(w, s);
+        const bool lo = line == 1, hi = line == m, bd = lo || hi;
+        const int e = lo ? 1 : -1;
+        const double* F = at(R, line);
+        double out[S];
+        line_solve<S>(bd, bd ? tb : tc, G, g, lane, V.lv, at(R, bd ? line + e : line - 2), at(R, bd ? line + 2 * e : line - 1),
+                      at(R, bd ? line + 3 * e : line + 1), at(R, bd ? line + 4 * e : line + 2), bd ? at(R, line - e) : nullptr, F,
+                      sc, f0, s == 0 ? V.rf0 : V.rf, out, xch, 1 + grp);
+        double* own = R + (size_t)(line & (RING - 1)) * LS + c;
+#pragma unroll
+        for (int q = 0; q < S; q++) own[q * NC] = out[q];
+        if (s == ns - 1) {
+            done = line;
+#pragma unroll
+            for (int q = 0; q < S; q++) res[q] = out[q];
+        } else if (!V.seq) {
+            const int slot = (s + 1) % NS, w2 = slot % W, r2 = slot / W;
+            double* next = ring(w2, s + 1) + (size_t)(line & (RING - 1)) * LS + c;
+            if (r2 == rank) {
+#pragma unroll
+                for (int q = 0; q < S; q++) next[q * NC] = out[q];
+            } else {
+                const uint32_t a = in_cta(next, r2);
+#pragma unroll
+                for (int q = 0; q < S; q++) push(a + 8u * q * NC, out[q]);
+            }
+        }
+    };
+    if (V.seq) {
+        // one group in the reference's order; lines 0 .. 8 at most, all in the ring
+        if (grp == 0)
+            for (int q = 0; q < ns * m; q++) {
+                const int s = q / m, r = q - s * m, line = r == 0 ? 1 : r == 1 ? m : r;
+                double sc[S], f0 = 0.0;
+                load_sc(line, sc, f0);
+                relax(0, s, line, sc, f0);
+                write_back();
+                if (G > 1) group_barrier(1, 32 * G); else __syncwarp();
+            }
+        return;
+    }
+    // A line group runs its slot's sweep s at step u = t - 5 s: line 1, then the
+    // centre lines.  The last group watches all slots of the CTA for the step
+    // of the far border line.
+    const bool bgrp = grp == W;
+    const int turn = V.parity > 1 ? LAG * NS : 0x3fffffff;   // steps from a slot's sweep to its next
+    int sw = rank * W + (bgrp ? 0 : grp);   // current sweep of the group's (first) slot
+    double scn[S], f0n = 0.0, fln[S];
+#pragma unroll
+    for (int q = 0; q < S; q++) { scn[q] = 0.0; fln[q] = 0.0; }
+    // the task of the group at step t: line (0: none) of sweep `s` in slot `w`
+    auto task = [&](int t, int& w, int& s) -> int {
+        if (!bgrp) {
+            w = grp; s = sw;
+            if (t - LAG * s >= turn) s += NS;
+            const int u = t - LAG * s;
+            return (u < 0 || u > m - 2 || s >= ns) ? 0 : u + 1;
+        }
+        for (int q = 0; q < W; q++) {
+            s = sw + q;
+            if (t - LAG * s >= turn) s += NS;
+            if (t - LAG * s == m - 6 && s < ns) { w = q; return m; }
+        }
+        return 0;
+    };
+    int w = 0, s = 0, line = task(0, w, s);
+    if (line) load_sc(line, scn, f0n);
+    const int T = m - 1 + LAG * (ns - 1);
+    for (int t = 0; t < T; t++) {
+        double sc[S], f0 = f0n;
+#pragma unroll
+        for (int q = 0; q < S; q++) sc[q] = scn[q];
+        int w2 = 0, s2 = 0;
+        const int line2 = task(t + 1, w2, s2);
+        if (line2) load_sc(line2, scn, f0n);
+        const bool feed = rank == 0 && grp == 0 && t + 8 <= m;   // line t + 8 of the first sweep
+        if (feed) {
+#pragma unroll
+            for (int q = 0; q < S; q++) fln[q] = (row0 + q < n) ? Fg[(size_t)(t + 8) * n + row0 + q] : 0.0;
+        }
+        if (line) relax(w, s, line, sc, f0);
+        if (feed) {
+            double* dst = rings + (size_t)((t + 8) & (RING - 1)) * LS + c;
+#pragma unroll
+            for (int q = 0; q < S; q++) dst[q * NC] = fln[q];
+        }
+        // written between the barrier's halves, or its release would wait for global memory
+        __syncwarp();
+        if (C > 1) cluster_arrive();
+        write_back();
+        line = line2; w = w2; s = s2;
+        if (t + 1 - LAG * sw - (bgrp ? LAG * (W - 1) : 0) >= turn) sw += NS;
+        __syncwarp();
+        if (C > 1) cluster_wait(); else __syncthreads();
     }
 }
 
@@ -585,183 +712,186 @@ PlainDev make_plain(tb_ctx* c) {
         P.den[l] = 1.0 / (12.0 * c->h_dx2[l] * c->cfg.fac_y);
     }
     P.ify = 1.0 / c->cfg.fac_y;
-    P.pelems = c->g.lvl_elems; P.dstride = (size_t)c->g.nx * c->g.ny;
+    P.pelems = c->g.lvl_elems; P.dstride = (size_t)c->g.nx * c->g.ny; P.tabs = tab_block(c->g.ny);
     P.fac_y = c->cfg.fac_y; P.alpha = c->cfg.alpha;
     return P;
 }
 
-// Line-solve tables of one (group, type, level, mode) for G warps of 32 row
-// chunks of S rows: the band LU rows (L1 L2 U1 U2 ID), the chunk-local
-// homogeneous responses h1 h2 (forward, to the incoming y_{r0-1}, y_{r0-2})
-// and k1 k2 (backward, to x_{r1}, x_{r1+1}), and per warp the Kogge-Stone
-// step matrices Pf, Pb of its 32 chunk propagators, the prefix R (warp start
-// to each chunk start, forward), the suffix Q (warp end to each chunk end,
-// backward) and the warp totals A (forward) and B (backward).
+// Line-solve tables (layout above tab_wz) of one (group, type, level, mode)
+// for G warps of 32 chunks of S rows, from the band LU rows L1 L2 U1 U2 ID.  The rows
+// past the line are rows of zeros, so every chunk has S.
 void group_tables(int n, int S, int G, const double* L1, const double* L2, const double* U1, const double* U2,
-                  const double* ID, double* out) {
-    std::memcpy(out, L1, n * sizeof(double));
-    std::memcpy(out + n, L2, n * sizeof(double));
-    std::memcpy(out + 2 * n, U1, n * sizeof(double));
-    std::memcpy(out + 3 * n, U2, n * sizeof(double));
-    std::memcpy(out + 4 * n, ID, n * sizeof(double));
-    double *h1 = out + 5 * n, *h2 = out + 6 * n, *k1 = out + 7 * n, *k2 = out + 8 * n;
-    const int C = 32 * G;
-    std::vector<double> Mf((size_t)C * 4), Mb((size_t)C * 4);
-    for (int t = 0; t < C; t++) {
-        const int r0 = t * S, r1 = std::min(n, r0 + S);
-        double e0[2], e1[2];
-        for (int u = 0; u < 2; u++) {
-            double ym1 = (u == 0) ? 1.0 : 0.0, ym2 = (u == 0) ? 0.0 : 1.0;
-            for (int j = r0; j < r1; j++) {
-                double y = -L2[j] * ym2 - L1[j] * ym1;
-                (u == 0 ? h1 : h2)[j] = y;
-                ym2 = ym1; ym1 = y;
-            }
-            e0[u] = ym1; e1[u] = ym2;   // an empty chunk passes its state on unchanged
-        }
-        Mf[4 * t] = e0[0]; Mf[4 * t + 1] = e0[1]; Mf[4 * t + 2] = e1[0]; Mf[4 * t + 3] = e1[1];
-        for (int u = 0; u < 2; u++) {
-            double xp1 = (u == 0) ? 1.0 : 0.0, xp2 = (u == 0) ? 0.0 : 1.0;
-            for (int j = r1 - 1; j >= r0; j--) {
-                double x = (-U1[j] * xp1 - U2[j] * xp2) * ID[j];
-                (u == 0 ? k1 : k2)[j] = x;
-                xp2 = xp1; xp1 = x;
-            }
-            e0[u] = xp1; e1[u] = xp2;
-        }
-        Mb[4 * t] = e0[0]; Mb[4 * t + 1] = e0[1]; Mb[4 * t + 2] = e1[0]; Mb[4 * t + 3] = e1[1];
-    }
-    auto mul = [](const double* A, const double* B, double* Cm) {   // Cm = A B
-        double c0 = A[0] * B[0] + A[1] * B[2], c1 = A[0] * B[1] + A[1] * B[3];
-        double c2 = A[2] * B[0] + A[3] * B[2], c3 = A[2] * B[1] + A[3] * B[3];
-        Cm[0] = c0; Cm[1] = c1; Cm[2] = c2; Cm[3] = c3;
+                  const double* ID, const double* cf, double qx, double* out) {
+    const int NC = 32 * G;
+    using M2 = std::array<double, 4>;
+    auto mul = [](const M2& A, const M2& B) {   // A B
+        return M2{A[0] * B[0] + A[1] * B[2], A[0] * B[1] + A[1] * B[3], A[2] * B[0] + A[3] * B[2], A[2] * B[1] + A[3] * B[3]};
     };
-    const double I[4] = {1.0, 0.0, 0.0, 1.0};
-    for (int g = 0; g < G; g++) {
-        double* W = out + 9 * n + (size_t)WARP_TAB * g;
-        double *Pf = W, *Pb = W + 640, *R = W + 1280, *Q = W + 1408, *A = W + 1536, *B = W + 1540;
-        const double* mf = &Mf[(size_t)128 * g];
-        const double* mb = &Mb[(size_t)128 * g];
-        double Af[32][4], Ab[32][4];
-        std::memcpy(Af, mf, sizeof Af);
-        std::memcpy(Ab, mb, sizeof Ab);
-        for (int d = 0, off = 1; d < 5; d++, off <<= 1) {
-            for (int t = 0; t < 32; t++) {
-                std::memcpy(Pf + (d * 32 + t) * 4, Af[t], 4 * sizeof(double));
-                std::memcpy(Pb + (d * 32 + t) * 4, Ab[t], 4 * sizeof(double));
+    std::vector<M2> Mf(NC), Mb(NC);
+    for (int c = 0; c < NC; c++) {
+        auto at = [&](int e) -> double& { return out[(size_t)e * NC + c]; };
+        std::vector<double> l1(S), l2(S), u1(S), u2(S);
+        for (int s = 0; s < S; s++) {
+            const int j = 1 + c * S + s;
+            const bool in = j < n;
+            if (in) {
+                // sc - qx (weights . x-stencil sums), rhs_center / rhs_border (poisson_par.f:343-540)
+                at(8 * s) = (j > 1 && j <= n - 3) ? -qx * cf[7] : 0.0;
+                at(8 * s + 1) = j == 1 ? -qx * cf[1] : j <= n - 3 ? -qx * cf[8] : -qx;
+                at(8 * s + 2) = j == 1 ? -qx * cf[2] : j <= n - 3 ? -qx * cf[9] : 0.0;
             }
-            double nf[32][4], nb[32][4];
-            for (int t = 0; t < 32; t++) {
-                if (t >= off) mul(Af[t], Af[t - off], nf[t]); else std::memcpy(nf[t], Af[t], sizeof nf[t]);
-                if (t + off < 32) mul(Ab[t], Ab[t + off], nb[t]); else std::memcpy(nb[t], Ab[t], sizeof nb[t]);
-            }
-            std::memcpy(Af, nf, sizeof Af);
-            std::memcpy(Ab, nb, sizeof Ab);
+            l1[s] = (in && j > 1) ? L1[j] : 0.0; l2[s] = (in && j > 2) ? L2[j] : 0.0;
+            u1[s] = in ? U1[j] * ID[j] : 0.0; u2[s] = in ? U2[j] * ID[j] : 0.0;
+            at(8 * s + 3) = l1[s]; at(8 * s + 4) = l2[s];
+            at(8 * s + 5) = u1[s]; at(8 * s + 6) = u2[s];
+            at(8 * s + 7) = in ? ID[j] : 0.0;
+            if (s < 2) at(tab_wz(S) + s) = in && j == 1 ? -L1[1] : in && j == 2 ? -L2[2] : 0.0;
         }
-        // R_t = Mf_{t-1} ... Mf_0, A = Mf_31 ... Mf_0
-        double acc[4];
-        std::memcpy(acc, I, sizeof acc);
+        // responses to the entering states (y_{-1}, y_{-2}) and (x_S, x_{S+1})
+        for (int u = 0; u < 2; u++) {
+            double p1 = u == 0, p2 = u == 1;
+            for (int s = 0; s < S; s++) {
+                const double y = -l1[s] * p1 - l2[s] * p2;
+                if (S > 2) at(tab_h(S) + 4 * s + u) = y;
+                p2 = p1; p1 = y;
+            }
+            Mf[c][u] = p1; Mf[c][2 + u] = p2;
+            p1 = u == 0; p2 = u == 1;
+            for (int s = S - 1; s >= 0; s--) {
+                const double x = -u1[s] * p1 - u2[s] * p2;
+                if (S > 2) at(tab_h(S) + 4 * s + 2 + u) = x;
+                p2 = p1; p1 = x;
+            }
+            Mb[c][u] = p1; Mb[c][2 + u] = p2;
+        }
+    }
+    const M2 I{1.0, 0.0, 0.0, 1.0};
+    std::vector<M2> A(G, I), B(G, I);   // propagators of whole warps
+    for (int g = 0; g < G; g++)
         for (int t = 0; t < 32; t++) {
-            std::memcpy(R + 4 * t, acc, sizeof acc);
-            double nx4[4];
-            mul(mf + 4 * t, acc, nx4);
-            std::memcpy(acc, nx4, sizeof acc);
+            A[g] = mul(Mf[32 * g + t], A[g]);
+            B[g] = mul(Mb[32 * g + 31 - t], B[g]);
         }
-        std::memcpy(A, acc, sizeof acc);
-        // Q_t = Mb_{t+1} ... Mb_31, B = Mb_0 ... Mb_31
-        std::memcpy(acc, I, sizeof acc);
-        for (int t = 31; t >= 0; t--) {
-            std::memcpy(Q + 4 * t, acc, sizeof acc);
-            double nx4[4];
-            mul(mb + 4 * t, acc, nx4);
-            std::memcpy(acc, nx4, sizeof acc);
+    for (int g = 0; g < G; g++) {
+        std::vector<M2> a(Mf.begin() + 32 * g, Mf.begin() + 32 * g + 32), b(Mb.begin() + 32 * g, Mb.begin() + 32 * g + 32);
+        for (int d = 0, off = 1; d < 5; d++, off <<= 1) {
+            std::vector<M2> na = a, nb = b;
+            for (int t = 0; t < 32; t++) {
+                for (int q = 0; q < 4; q++) {
+                    out[(size_t)(tab_pf(S) + 4 * d + q) * NC + 32 * g + t] = a[t][q];
+                    out[(size_t)(tab_pb(S) + 4 * d + q) * NC + 32 * g + t] = b[t][q];
+                }
+                if (t >= off) na[t] = mul(a[t], a[t - off]);
+                if (t + off < 32) nb[t] = mul(b[t], b[t + off]);
+            }
+            a = na; b = nb;
         }
-        std::memcpy(B, acc, sizeof acc);
+        const int CW = tab_cw(S);
+        M2 f = I, r = I;   // from the warp's start (end) to the chunk's
+        for (int t = 0; t < 32; t++) {
+            const int cf_ = 32 * g + t, cb_ = 32 * g + 31 - t;
+            if (S <= 2) { f = mul(Mf[cf_], f); r = mul(Mb[cb_], r); }
+            M2 x = f;
+            for (int w = g - 1; w >= 0; w--) {   // from warp w's end to this warp's start
+                for (int q = 0; q < CW; q++) out[(size_t)(tab_cf(S) + CW * w + q) * NC + cf_] = x[q];
+                x = mul(x, A[w]);
+            }
+            x = r;
+            for (int w = g + 1; w < G; w++) {
+                for (int q = 0; q < CW; q++) out[(size_t)(tab_cb(S) + CW * (w - g - 1) + q) * NC + cb_] = x[q];
+                x = mul(x, B[w]);
+            }
+            if (S > 2) { f = mul(Mf[cf_], f); r = mul(Mb[cb_], r); }
+        }
     }
 }
 
-// Warps per line (as log2, the table group) for a launch of ns sweeps on
-// rows of n: one sweep at a time spreads each line over four warps (one per
-// SM sub-partition), several sweeps over two, unless the tuner chose; every
-// warp of a group keeps at least 32 rows.
-int plain_group(const tb_ctx* c, int n, int ns, int whole) {
-    if (whole) return 0;
-    int gi = (ns == 1) ? (c->tune_pg1 ? c->tune_pg1 - 1 : 2) : (c->tune_pg3 ? c->tune_pg3 - 1 : 1);
-    while (gi > 0 && n <= 32 * group_warps(gi - 1)) gi--;
+// Warps per line (as log2, the table group) of a launch with `slots` sweeps in
+// flight on lines of n points: one row a lane as far as four warps go, for the
+// shortest line solve, and fewer warps where the sub-partitions of all SMs have more
+// than a warp each, for fewer instructions in all (a line takes 4 x 55 on four
+// warps, 2 x 82 on two); or what the tuner chose.
+int plain_group(const tb_ctx* c, int n, int itera, int slots) {
+    const int tuned = itera == 1 ? c->tune_pg1 : c->tune_pg3;
+    int gi = tuned ? tuned - 1 : NGROUP - 1;
+    while (gi > 0 && n - 1 <= 32 * group_warps(gi - 1)) gi--;
+    const int sms = c->sm_count > 0 ? c->sm_count : 148;
+    if (!tuned)
+        while (gi > 0 && (long)2 * c->g.K * slots * group_warps(gi) > 4L * sms) gi--;
     return gi;
 }
 
-template <int S, int G>
-int launch_wsor_s(tb_ctx* c, const PlainDev& P, int l, int ns, double rf, int whole, int gi, int groups) {
-    const int n = c->g.ptsy[l], lines = whole ? c->g.ptsx[l] : RING;
-    const size_t smem = ((size_t)tab_size(n, G) + (size_t)2 * lines * n + (size_t)4 * G * groups) * sizeof(double);
-    TB_CUDA(cudaFuncSetAttribute(k_wsor<S, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // at most the groups the kernel's register count allows in one block; a
-    // group then runs the tasks of several sweeps in some steps, which are independent
-    cudaFuncAttributes fa;
-    TB_CUDA(cudaFuncGetAttributes(&fa, k_wsor<S, G>));
-    groups = std::max(1, std::min(groups, fa.maxThreadsPerBlock / (32 * G)));
-    k_wsor<S, G><<<2 * c->g.K, 32 * G * groups, smem, c->stream>>>(P, l, ns, rf, whole, gi);
+template <int S, bool STAGED>
+int launch_wsor_t(tb_ctx* c, const PlainDev& P, const Wave& V, size_t smem) {
+    TB_CUDA(cudaFuncSetAttribute(k_wsor<S, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)V.C; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(2 * c->g.K * V.C));
+    cfg.blockDim = dim3((unsigned)(32 * group_warps(V.gi) * (V.W + 1)));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = V.C > 1 ? 1 : 0;
+    TB_CUDA(cudaLaunchKernelEx(&cfg, k_wsor<S, STAGED>, P, V));
     TB_CHECK_LAUNCH(c);
     return TB_OK;
 }
 
-template <int G>
-int launch_wsor_g(tb_ctx* c, const PlainDev& P, int l, int ns, double rf, int whole, int gi, int groups, int S) {
-    switch (S) {
-        case 1: return launch_wsor_s<1, G>(c, P, l, ns, rf, whole, gi, groups);
-        case 2: return launch_wsor_s<2, G>(c, P, l, ns, rf, whole, gi, groups);
-        case 3: return launch_wsor_s<3, G>(c, P, l, ns, rf, whole, gi, groups);
-        case 4: return launch_wsor_s<4, G>(c, P, l, ns, rf, whole, gi, groups);
-        case 5: return launch_wsor_s<5, G>(c, P, l, ns, rf, whole, gi, groups);
-        case 6: return launch_wsor_s<6, G>(c, P, l, ns, rf, whole, gi, groups);
-        case 7: return launch_wsor_s<7, G>(c, P, l, ns, rf, whole, gi, groups);
-        case 8: return launch_wsor_s<8, G>(c, P, l, ns, rf, whole, gi, groups);
-        default: break;
-    }
-    if (G == 1) {
-        switch (S) {
-            case 9: return launch_wsor_s<9, 1>(c, P, l, ns, rf, whole, gi, groups);
-            case 10: return launch_wsor_s<10, 1>(c, P, l, ns, rf, whole, gi, groups);
-            case 11: return launch_wsor_s<11, 1>(c, P, l, ns, rf, whole, gi, groups);
-            case 12: return launch_wsor_s<12, 1>(c, P, l, ns, rf, whole, gi, groups);
-            default: return launch_wsor_s<16, 1>(c, P, l, ns, rf, whole, gi, groups);
-        }
-    }
-    tb_set_error("plain Poisson: %d rows per lane on %d warps per line", S, G);
-    return TB_ERR_ARG;
+template <int S>
+int launch_wsor(tb_ctx* c, const PlainDev& P, const Wave& V, size_t smem) {
+    return V.staged > 1 ? launch_wsor_t<S, true>(c, P, V, smem) : launch_wsor_t<S, false>(c, P, V, smem);
 }
 
-// `itera` sweeps of sor at level l (poisson_par.f:167-226) for every active mode.
-int plain_sor(tb_ctx* c, const PlainDev& P, int l, int itera, double rf) {
-    const int nxl = c->g.ptsx[l], n = c->g.ptsy[l], m = nxl - 2;
-    const size_t whole_bytes = ((size_t)tab_size(n, 1) + (size_t)2 * nxl * n + 4 * 32) * sizeof(double);
-    const bool can_whole = whole_bytes <= (size_t)200 * 1024;
+// `itera` sweeps of sor at level l (poisson_par.f:167-226) for every active
+// mode, the first with relaxation factor rf0.
+int plain_sor(tb_ctx* c, const PlainDev& P, int l, int itera, double rf0, double rf) {
+    const int n = c->g.ptsy[l], m = c->g.ptsx[l] - 2;
     cudaEvent_t ps = nullptr;
     if (tb_prof_begin(c, PROF_SOR, &ps)) return TB_ERR_CUDA;
-    int done = 0;
-    while (done < itera) {
-        int ns, whole, groups;
-        if (m < 7 || (itera - done > MAX_STREAM_SWEEPS && can_whole)) {
-            // all remaining sweeps with the level held in shared memory; group w
-            // runs the sweeps w, w + W, ... (the wavefront stays full once
-            // W > (m - 2) / LAG)
-            whole = 1;
-            ns = itera - done;
-            groups = (m < 7) ? 1 : std::min({32, ns, (m - 2) / LAG + 1});
-        } else {
-            whole = 0;
-            ns = std::min(MAX_STREAM_SWEEPS, itera - done);
-            groups = ns;
+    for (int done = 0; done < itera;) {
+        Wave V;
+        std::memset(&V, 0, sizeof V);
+        V.l = l; V.ns = itera - done; V.rf0 = done ? rf : rf0; V.rf = rf;
+        V.C = V.W = V.parity = 1;
+        V.seq = m < 7;   // border stencils and wavefront want distinct lines
+        // sweeps in flight: the first ends after m - 1 steps
+        const int want = V.seq ? 1 : std::min(V.ns, (m - 1 + LAG - 1) / LAG);
+        V.gi = plain_group(c, n, itera, want);
+        const int G = group_warps(V.gi), S = rows_per_lane(n, G), NC = 32 * G;
+        // one-warp groups: three to a CTA beside the border group, the SM's four sub-partitions
+        if (want > 1) {
+            const int most = G == 1 ? 3 : 1;
+            if (want > most) {
+                V.C = 2;
+                while (V.C < MAX_CLUSTER && V.C * most < want) V.C *= 2;
+            }
+            V.W = std::min(most, (want + V.C - 1) / V.C);
         }
-        const int gi = (m < 7) ? 0 : plain_group(c, n, ns, whole);
-        const int G = group_warps(gi), S = rows_per_lane(n, G);
+        auto bytes = [&]() { return (wave_lines(V, NC, S) + (size_t)6 * G * (V.W + 1)) * sizeof(double); };
+        const size_t room = (size_t)226 * 1024, table = (size_t)tab_size(n, G) * sizeof(double);
+        if (!V.seq && V.ns > V.C * V.W) {   // slots run several sweeps, or the launch fewer
+            if (m - 1 <= LAG * V.C * V.W) V.parity = 2;
+            if (V.parity == 1 || bytes() > room) { V.parity = 1; V.ns = V.C * V.W; }
+        }
+        while (bytes() > room && V.W > 1) { V.W--; V.ns = std::min(V.ns, V.C * V.W); }
+        V.staged = bytes() + 2 * table <= room ? 2 : bytes() + table <= room ? 1 : 0;
+        for (int chunks = (n - 1 + S - 1) / S; V.lv < 5 && (1 << V.lv) < chunks;) V.lv++;
+        const size_t smem = bytes() + V.staged * table;
         int r;
-        if (G == 1) r = launch_wsor_g<1>(c, P, l, ns, rf, whole, gi, groups, S);
-        else if (G == 2) r = launch_wsor_g<2>(c, P, l, ns, rf, whole, gi, groups, S);
-        else r = launch_wsor_g<4>(c, P, l, ns, rf, whole, gi, groups, S);
+        switch (S) {
+            case 1: r = launch_wsor<1>(c, P, V, smem); break;
+            case 2: r = launch_wsor<2>(c, P, V, smem); break;
+            case 3: r = launch_wsor<3>(c, P, V, smem); break;
+            case 4: r = launch_wsor<4>(c, P, V, smem); break;
+            case 6: r = launch_wsor<6>(c, P, V, smem); break;
+            case 8: r = launch_wsor<8>(c, P, V, smem); break;
+            case 12: r = launch_wsor<12>(c, P, V, smem); break;
+            default: r = launch_wsor<16>(c, P, V, smem); break;
+        }
         if (r) return r;
-        done += ns;
+        done += V.ns;
     }
     return tb_prof_end(c, PROF_SOR, ps);
 }
@@ -784,10 +914,10 @@ int tb_plain_tune(tb_ctx* c, int l, int itera, const int* gis, int ngis, int* be
     for (int q = 0; q < ngis && !r; q++) {
         *keep = gis[q] + 1;
         k_pactivate<<<tb_blocks(c->g.K, 64), 64, 0, c->stream>>>(c->pstate, c->g.K);
-        r = plain_sor(c, P, l, itera, 1.0);   // warm-up
+        r = plain_sor(c, P, l, itera, 1.0, 1.0);   // warm-up
         if (r) break;
         cudaEventRecord(a, c->stream);
-        for (int rep = 0; rep < 3 && !r; rep++) r = plain_sor(c, P, l, itera, 1.0);
+        for (int rep = 0; rep < 3 && !r; rep++) r = plain_sor(c, P, l, itera, 1.0, 1.0);
         cudaEventRecord(b, c->stream);
         float ms = 0.f;
         if (!r && cudaEventSynchronize(b) == cudaSuccess) cudaEventElapsedTime(&ms, a, b);
@@ -821,6 +951,9 @@ int tb_plain_setup(tb_ctx* c) {
     // band LU of the y-line matrices (band5_poi, penta_par.f:308-364), factored
     // once per (type, level, mode), with the chunk tables of each line group
     const size_t bs = tab_block(ny);
+    const PlainDev P = make_plain(c);
+    std::vector<double> cf((size_t)24 * msh);
+    TB_CUDA(cudaMemcpy(cf.data(), c->pcoef, cf.size() * sizeof(double), cudaMemcpyDeviceToHost));
     std::vector<double> all((size_t)NGROUP * 2 * msh * K * bs, 0.0), a;
     std::vector<double> L1(ny), L2(ny), U1(ny), U2(ny), ID(ny);
     for (int type = 0; type < 2; type++)
@@ -832,7 +965,8 @@ int tb_plain_setup(tb_ctx* c) {
                 for (int gi = 0; gi < NGROUP; gi++) {
                     const int G = group_warps(gi);
                     double* T = &all[((((size_t)gi * 2 + type) * msh + l) * K + k) * bs];
-                    group_tables(n, rows_per_lane(n, G), G, L1.data(), L2.data(), U1.data(), U2.data(), ID.data(), T);
+                    group_tables(n, rows_per_lane(n, G), G, L1.data(), L2.data(), U1.data(), U2.data(), ID.data(), &cf[24 * l],
+                                 P.den[l], T);
                 }
             }
     if (c->pl_tab) cudaFree(c->pl_tab);
@@ -871,7 +1005,9 @@ int tb_poi_uy_k(tb_ctx* c, const cplx* dwzdx, double erro) {
     int r;
     for (int v = 1; v <= vmax; v++) {
         for (int l = 0; l < msh - 1; l++) {
-            if ((r = plain_sor(c, P, l, 3, 1.2))) return r;
+            // the fine level's sweep that ends the cycle before goes ahead of this one's
+            const int behind = (l == 0 && v > 1) ? 1 : 0;
+            if ((r = plain_sor(c, P, l, 3 + behind, behind ? 1.0 : 1.2, 1.2))) return r;
             if ((r = defect(l, -1.0))) return r;
             if (l == 0) { k_pcheck<<<tb_blocks(K, 64), 64, 0, c->stream>>>(P, erro, v); TB_CHECK_LAUNCH(c); }
             const int per = c->g.ptsx[l + 1] * c->g.ptsy[l + 1];
@@ -879,7 +1015,7 @@ int tb_poi_uy_k(tb_ctx* c, const cplx* dwzdx, double erro) {
             TB_CHECK_LAUNCH(c);
             if ((r = defect(l + 1, 1.0))) return r;
         }
-        if ((r = plain_sor(c, P, msh - 1, 60, 1.2))) return r;
+        if ((r = plain_sor(c, P, msh - 1, 60, 1.2, 1.2))) return r;
         for (int l = msh - 1; l >= 1; l--) {
             const int per = (c->g.ptsx[l] - 2) * c->g.ptsy[l];
             k_pcorrection<<<dim3(tb_blocks(per, 128), 2 * K), 128, 0, c->stream>>>(P, l);
@@ -887,7 +1023,8 @@ int tb_poi_uy_k(tb_ctx* c, const cplx* dwzdx, double erro) {
             const int perf = (c->g.ptsx[l - 1] - 2) * c->g.ptsy[l - 1];
             k_pintpol<<<dim3(tb_blocks(perf, 128), 2 * K), 128, 0, c->stream>>>(P, l);
             TB_CHECK_LAUNCH(c);
-            if ((r = plain_sor(c, P, l - 1, 1, 1.0))) return r;
+            if (l > 1 || v == vmax)
+                if ((r = plain_sor(c, P, l - 1, 1, 1.0, 1.0))) return r;
         }
         TB_CUDA(cudaMemcpyAsync(hs.data(), c->pstate, 2 * K * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
         TB_CUDA(cudaStreamSynchronize(c->stream));
