@@ -15,9 +15,6 @@
 
 namespace {
 
-__device__ __forceinline__ cplx cmul(double s, cplx a) { return make_double2(s * a.x, s * a.y); }
-__device__ __forceinline__ cplx cfma(double s, cplx a, cplx b) { return make_double2(fma(s, a.x, b.x), fma(s, a.y, b.y)); }
-
 struct XArgs {
     XJob job[8];
     int njobs, nx, ny, K;
@@ -66,37 +63,39 @@ __global__ void __launch_bounds__(64 * XW_MAX) k_xwarp(XArgs A) {
 
 struct YArgs {
     YJob job[8];
-    int njobs, nx, ny, K;
+    int nx2, ny, K;
     TriLHS t[3];
     YRhs r[3];
 };
 
-template <int OP>
+// One real line a thread: the real and the imaginary parts of a field are
+// lines of their own, neighbours in memory.  The rows' 1/pivot is folded into the
+// right-hand side's weights and the sub-diagonal, so an interior row takes 5
+// instructions for its right-hand side and one for each sweep.  All jobs run in
+// one launch, blockIdx.y the job.  Bound by the FP64 pipe on large grids and by the
+// chain of rows on small ones: a step's 8 launches take 0.62 ms at 257 x 97 x 8 and
+// 4.3 ms at 1025 x 193 x 32; a launch per operator with a complex line a thread and
+// one instruction more a row took 1.30 and 6.3 ms.
 __global__ void __launch_bounds__(128) k_ylines(YArgs A) {
-    int nlines = A.nx * A.K;
-    int gid = blockIdx.x * blockDim.x + threadIdx.x;
-    int jb = gid / nlines;
-    int line = gid - jb * nlines;
-    if (jb >= A.njobs) return;
-    const YJob& J = A.job[jb];
-    if (J.op != OP) return;
-    int i = line % A.nx, k = line / A.nx;
-    int ny = A.ny;
-    size_t s = A.nx;
-    size_t base = (size_t)i + (size_t)A.nx * ny * k;
-    const cplx* __restrict__ f = J.src + base;
-    cplx* __restrict__ o = J.dst + base;
-    const TriLHS& T = A.t[OP];
-    const YRhs& R = A.r[OP];
-    cplx u = make_double2(0.0, 0.0);
+    const int line = blockIdx.x * blockDim.x + threadIdx.x, ny = A.ny;
+    if (line >= A.nx2 * A.K) return;
+    const YJob& J = A.job[blockIdx.y];
+    const int i = line % A.nx2, k = line / A.nx2;
+    const size_t s = A.nx2, base = (size_t)i + s * ny * k;
+    const double* __restrict__ f = reinterpret_cast<const double*>(J.src) + base;
+    double* __restrict__ o = reinterpret_cast<double*>(J.dst) + base;
+    const double* __restrict__ ta = A.t[J.op].a;
+    const double* __restrict__ tg = A.t[J.op].g;
+    const YRhs& R = A.r[J.op];
+    const double* __restrict__ wr = R.w;
+    double u = 0.0;
     // one row of the forward sweep with its rhs from the tables (boundary rows)
     auto generic = [&](int j) {
-        cplx r = make_double2(0.0, 0.0);
+        double r = 0.0;
         const int c0 = R.cnt[j], of = R.off[j];
-        const double* w = R.w + 7 * j;
-        for (int m = 0; m < c0; m++) r = cfma(w[m], f[(size_t)(j + of + m) * s], r);
-        const double a = T.a[j], ib = T.ib[j];
-        u = make_double2((r.x - a * u.x) * ib, (r.y - a * u.y) * ib);
+        const double* w = wr + 7 * j;
+        for (int m = 0; m < c0; m++) r = fma(w[m], f[(size_t)(j + of + m) * s], r);
+        u = fma(-ta[j], u, r);
         o[(size_t)j * s] = u;
     };
     // The sweeps are sequential in j, so each row's loads are issued YPD rows
@@ -106,26 +105,25 @@ __global__ void __launch_bounds__(128) k_ylines(YArgs A) {
     generic(0);
     generic(1);
     {
-        cplx w0 = f[0], w1 = f[s], w2 = f[2 * s], w3 = f[3 * s];
-        cplx pre[YPD];
+        double w0 = f[0], w1 = f[s], w2 = f[2 * s], w3 = f[3 * s];
+        double pre[YPD];
 #pragma unroll
-        for (int q = 0; q < YPD; q++) pre[q] = (4 + q < ny) ? f[(size_t)(4 + q) * s] : make_double2(0.0, 0.0);
+        for (int q = 0; q < YPD; q++) pre[q] = (4 + q < ny) ? f[(size_t)(4 + q) * s] : 0.0;
         for (int jb = 2; jb < ny - 2; jb += YPD) {
 #pragma unroll
             for (int q = 0; q < YPD; q++) {
                 const int j = jb + q;
                 if (j < ny - 2) {
-                    const cplx w4 = pre[q];   // row j + 2
+                    const double w4 = pre[q];   // row j + 2
                     const int nr = j + 2 + YPD;
                     if (nr < ny) pre[q] = f[(size_t)nr * s];
-                    const double* w = R.w + 7 * j;
-                    cplx r = cmul(w[0], w0);
-                    r = cfma(w[1], w1, r);
-                    r = cfma(w[2], w2, r);
-                    r = cfma(w[3], w3, r);
-                    r = cfma(w[4], w4, r);
-                    const double a = T.a[j], ib = T.ib[j];
-                    u = make_double2((r.x - a * u.x) * ib, (r.y - a * u.y) * ib);
+                    const double* w = wr + 7 * j;
+                    double r = w[0] * w0;
+                    r = fma(w[1], w1, r);
+                    r = fma(w[2], w2, r);
+                    r = fma(w[3], w3, r);
+                    r = fma(w[4], w4, r);
+                    u = fma(-ta[j], u, r);
                     o[(size_t)j * s] = u;
                     w0 = w1; w1 = w2; w2 = w3; w3 = w4;
                 }
@@ -136,29 +134,24 @@ __global__ void __launch_bounds__(128) k_ylines(YArgs A) {
     generic(ny - 1);
     // backward sweep, rows ny-2 .. 0, the forward values read YPD rows ahead
     {
-        cplx pre[YPD];
+        double pre[YPD];
 #pragma unroll
-        for (int q = 0; q < YPD; q++) pre[q] = (ny - 2 - q >= 0) ? o[(size_t)(ny - 2 - q) * s] : make_double2(0.0, 0.0);
+        for (int q = 0; q < YPD; q++) pre[q] = (ny - 2 - q >= 0) ? o[(size_t)(ny - 2 - q) * s] : 0.0;
         for (int jb = ny - 2; jb >= 0; jb -= YPD) {
 #pragma unroll
             for (int q = 0; q < YPD; q++) {
                 const int j = jb - q;
                 if (j >= 0) {
-                    const cplx v = pre[q];
+                    const double v = pre[q];
                     const int nr = j - YPD;
                     if (nr >= 0) pre[q] = o[(size_t)nr * s];
-                    const double g = T.g[j + 1];
-                    u = make_double2(v.x - g * u.x, v.y - g * u.y);
+                    u = fma(-tg[j + 1], u, v);
                     o[(size_t)j * s] = u;
                 }
             }
         }
     }
 }
-
-}  // namespace
-
-namespace {
 
 // Launch of one operator's jobs.  A line's time is its FP64 instructions, so an SM
 // takes lines in fours, dealt evenly over its sub-partitions: blocks of 8
@@ -243,18 +236,13 @@ int tb_launch_ylines(tb_ctx* c, const YJob* jobs, int njobs) {
         if (jobs[q].src == jobs[q].dst) { tb_set_error("y-line job %d: in-place operation", q); return TB_ERR_ARG; }
         A.job[q] = jobs[q];
     }
-    A.njobs = njobs; A.nx = c->g.nx; A.ny = c->g.ny; A.K = c->g.K;
+    A.nx2 = 2 * c->g.nx; A.ny = c->g.ny; A.K = c->g.K;
     A.t[0] = c->ty1; A.t[1] = c->tyfv; A.t[2] = c->ty2;
     A.r[0] = c->ry1; A.r[1] = c->ryfv; A.r[2] = c->ry2;
-    size_t total = (size_t)njobs * c->g.nx * c->g.K;
-    bool has[3] = {false, false, false};
-    for (int q = 0; q < njobs; q++) has[jobs[q].op] = true;
     const int yt = (c->tune_yt == 32 || c->tune_yt == 64) ? c->tune_yt : 128;   // threads per block (tb_autotune)
-    unsigned nb = tb_blocks(total, yt);
     cudaEvent_t ps = nullptr;
     if (tb_prof_begin(c, PROF_YLINES, &ps)) return TB_ERR_CUDA;
-    if (has[0]) { k_ylines<YOP_D1><<<nb, yt, 0, c->stream>>>(A); TB_CHECK_LAUNCH(c); }
-    if (has[1]) { k_ylines<YOP_D1FV><<<nb, yt, 0, c->stream>>>(A); TB_CHECK_LAUNCH(c); }
-    if (has[2]) { k_ylines<YOP_D2><<<nb, yt, 0, c->stream>>>(A); TB_CHECK_LAUNCH(c); }
+    k_ylines<<<dim3(tb_blocks((size_t)A.nx2 * A.K, yt), njobs), yt, 0, c->stream>>>(A);
+    TB_CHECK_LAUNCH(c);
     return tb_prof_end(c, PROF_YLINES, ps);
 }

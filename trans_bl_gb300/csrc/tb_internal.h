@@ -33,20 +33,20 @@ void tb_set_error(const char* fmt, ...);
     } while (0)
 
 // Device-side line operator tables ----------------------------------------
-// Thomas factors of a constant tridiagonal LHS: forward u_i = (r_i - a_i u_{i-1}) * ib_i,
-// backward u_i -= g_{i+1} u_{i+1}  (tridparx/tridy, derivs_par.f:775-975).
+// Thomas factors of a constant tridiagonal LHS (tridparx/tridy,
+// derivs_par.f:775-975).  y-lines: forward u_j = r_j - a_j u_{j-1} with a_j and the
+// weights of r_j over the pivot, backward u_j -= g_{j+1} u_{j+1}.  x-lines, S rows
+// per lane: the row tables of tb_xline.cuh, and their FP32 copy (lines of
+// the mixed form's modes k >= 1).
 struct TriLHS {
-    double* a;   // (n)
-    double* g;   // (n) gam
-    double* ib;  // (n) 1/bet
-    // x-lines, S rows per lane: the row tables of
-    // tb_xline.cuh, and their FP32 copy (lines of the mixed form's modes k >= 1)
+    double* a = nullptr;   // (n)
+    double* g = nullptr;   // (n) gam
     double* xt = nullptr;
     float* xtf = nullptr;
     int S = 0;
 };
 // Row weights of the stretched-y compact RHS: row j (0-based) is
-// sum_m w[7*j+m] * f[j + off[j] + m], m < cnt[j].
+// sum_m w[7*j+m] * f[j + off[j] + m], m < cnt[j], over the LHS's pivot.
 struct YRhs {
     double* w;   // (ny*7)
     int* off;    // (ny)
