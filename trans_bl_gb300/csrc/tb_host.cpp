@@ -4,6 +4,7 @@
 // coef_center/coef_border+band5_poi, var_ts, buffer ramps, gibbs_function).
 #include "tb_internal.h"
 #include "tb_xline.cuh"
+#include <array>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -416,21 +417,64 @@ int tb_host_build_tables(tb_ctx* c) {
         if ((r = upload(&c->ry2.off, off))) return r;
         if ((r = upload(&c->ry2.cnt, cnt))) return r;
     }
-    // x-penta LU per mode (lhs5 + ludecomp; reciprocal of the diagonal in column 3)
+    // x-penta LU per mode (lhs5 + ludecomp) as row tables; row 0 is the boundary row
     {
-        std::vector<double> all((size_t)K * 5 * nx, 0.0), a, lu;
+        const int S = (nx + 31) / 32, N = 32 * S, tsz = penta_table_size(S);
+        const double kappa = 8.0 * cf.dx * cf.dx;
+        c->px.S = S;
+        c->px.unit = 1.0 / kappa;
+        std::vector<double> all((size_t)K * tsz, 0.0), a, lu;
+        using M2 = std::array<double, 4>;
+        auto mul = [](const M2& A, const M2& B) {
+            return M2{A[0] * B[0] + A[1] * B[2], A[0] * B[1] + A[1] * B[3], A[2] * B[0] + A[3] * B[2], A[2] * B[1] + A[3] * B[3]};
+        };
         for (int k = 2; k <= K; k++) {
-            double k2b2 = cf.dx * cf.dx * c->h_k2b2[k - 1];
-            lhs5(nx, k2b2, a);
+            lhs5(nx, cf.dx * cf.dx * c->h_k2b2[k - 1], a);
             ludecomp(nx, a, lu);
-            for (int col = 0; col < 5; col++)
-                for (int i = 0; i < nx; i++) {
-                    double v = lu[(size_t)i + (size_t)nx * col];
-                    if (col == 2) v = 1.0 / v;
-                    all[((size_t)(k - 1) * 5 + col) * nx + i] = v;
+            double* T = &all[(size_t)(k - 1) * tsz];
+            auto LU = [&](int i, int col) { return lu[(size_t)i + (size_t)nx * col]; };
+            M2 Mf[32], Mb[32];
+            for (int t = 0; t < 32; t++) {
+                const int r0 = std::min(nx, t * S), r1 = std::min(nx, r0 + S);
+                auto at = [&](int e, int i) -> double& { return T[(size_t)e * N + 32 * (i - r0) + t]; };
+                for (int i = r0; i < r1; i++) {
+                    const double iu = i ? 1.0 / LU(i, 2) : 1.0;
+                    at(0, i) = i > 1 ? LU(i, 0) : 0.0;
+                    at(1, i) = i ? LU(i, 1) : 0.0;
+                    at(2, i) = kappa * iu;
+                    at(3, i) = i ? LU(i, 3) * iu : 0.0;
+                    at(4, i) = i ? LU(i, 4) * iu : 0.0;
                 }
+                for (int u = 0; u < 2; u++) {
+                    double p1 = u == 0, p2 = u == 1;
+                    for (int i = r0; i < r1; i++) {
+                        const double y = -at(1, i) * p1 - at(0, i) * p2;
+                        at(5 + u, i) = at(2, i) * y;
+                        p2 = p1; p1 = y;
+                    }
+                    Mf[t][u] = p1; Mf[t][2 + u] = p2;
+                    p1 = u == 0; p2 = u == 1;
+                    for (int i = r1 - 1; i >= r0; i--) {
+                        const double x = -at(3, i) * p1 - at(4, i) * p2;
+                        at(7 + u, i) = x;
+                        p2 = p1; p1 = x;
+                    }
+                    Mb[t][u] = p1; Mb[t][2 + u] = p2;
+                }
+            }
+            double *Pf = T + 9 * N, *Pb = Pf + 640;
+            for (int d = 0, off = 1; d < 5; d++, off <<= 1) {
+                M2 nf[32], nb[32];
+                for (int t = 0; t < 32; t++) {
+                    for (int q = 0; q < 4; q++) { Pf[128 * d + 32 * q + t] = Mf[t][q]; Pb[128 * d + 32 * q + t] = Mb[t][q]; }
+                    nf[t] = t >= off ? mul(Mf[t], Mf[t - off]) : Mf[t];
+                    nb[t] = t + off < 32 ? mul(Mb[t], Mb[t + off]) : Mb[t];
+                }
+                std::copy(nf, nf + 32, Mf);
+                std::copy(nb, nb + 32, Mb);
+            }
         }
-        if ((r = upload(&c->px.lu, all))) return r;
+        if ((r = upload(&c->px.tab, all))) return r;
     }
     {
         // Poisson coefficients per level for the device kernels: sp(7) cp(8) pp(4) lp(5)

@@ -52,11 +52,15 @@ struct YRhs {
     int* off;    // (ny)
     int* cnt;    // (ny)
 };
-// Pentadiagonal x-LU of lhs5 per Fourier mode (penta_par.f:6-50): lu(i,c) with
-// reciprocal diagonal; one block of 5*nx per mode.
+// Pentadiagonal x-LU of lhs5 per Fourier mode k >= 1 (penta_par.f:6-50) as row
+// tables of lines in 32 chunks of S rows (layout at penta_sweeps, tb_loop.cu); the
+// right-hand sides come in units of 1 / unit = 8 dx^2.
 struct PentaX {
-    double* lu;   // (K, 5, nx): [k][c][i], c = 0..4 -> lu(:,1..5), c = 2 holds 1/lu(:,3)
+    double* tab;   // (K, penta_table_size(S))
+    int S;
+    double unit;
 };
+__host__ __device__ inline int penta_table_size(int S) { return 9 * 32 * S + 2 * 640; }
 
 struct TbGrid {
     int nx, ny, K, P, msh;

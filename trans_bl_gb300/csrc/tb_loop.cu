@@ -209,84 +209,150 @@ __global__ void __launch_bounds__(64) k_wz_wall(cplx* wz, const cplx* wx, const 
 }
 
 // Pentadiagonal x solve with the LU of lhs5 (lusolver / lusolver_1,
-// penta_par.f:53-208) of mode k, rhs rows
-//   r_0 = boundary value, r_1 = c12 (e_0 + 10 e_1 + e_2),
-//   r_i = c8 (e_{i-1} + 5.5 e_i + e_{i+1}),  r_{n-2} = c12 (e_{n-1} + 10 e_{n-2} + e_{n-3}),
-//   r_{n-1} = rn,
-// with e in E (overwritten); the solution (rows 1..n-1) goes to out.
-__device__ void penta_line(cplx* E, const WarpLine& L, int lane, const double* lu, cplx r0v, cplx rn, double c12,
-                           double c8, cplx* out) {
-    const int n = L.n, r0 = lane * L.S, r1 = min(n, r0 + L.S);
-    auto e = [&](int i) { return E[L.slot(i)]; };
-    cplx* Vl = E + lane * L.Sp;   // the rhs and the solution overwrite this lane's rows of e in place
-    // what the stencils read outside the lane's rows (e(r0-1), e(r1)) and the
-    // rhs of rows 1 and n-2, taken before any lane overwrites its rows
-    const cplx z = make_double2(0.0, 0.0);
-    cplx ep = (r0 >= 1 && r0 < r1) ? e(r0 - 1) : z;
-    const cplx en = (r1 < n && r0 < r1) ? e(r1) : z;
-    cplx v1 = z, vn2 = z;
-    if (1 >= r0 && 1 < r1) { cplx a = e(0), b = e(1), c = e(2); v1 = make_double2(c12 * (a.x + 10.0 * b.x + c.x), c12 * (a.y + 10.0 * b.y + c.y)); }
-    if (n - 2 >= r0 && n - 2 < r1) { cplx a = e(n - 1), b = e(n - 2), c = e(n - 3); vn2 = make_double2(c12 * (a.x + 10.0 * b.x + c.x), c12 * (a.y + 10.0 * b.y + c.y)); }
-    __syncwarp();
-    for (int i = r0; i < r1; i++) {
-        const cplx b = Vl[i - r0];   // e(i), not yet overwritten
-        cplx v;
-        if (i == 0) v = r0v;
-        else if (i == 1) v = v1;
-        else if (i <= n - 3) {
-            const cplx a = ep, c = (i + 1 < r1) ? Vl[i + 1 - r0] : en;
-            v = make_double2(c8 * (a.x + 5.5 * b.x + c.x), c8 * (a.y + 5.5 * b.y + c.y));
-        } else if (i == n - 2) v = vn2;
-        else v = rn;
-        ep = b;
-        Vl[i - r0] = v;
+// penta_par.f:53-208) of one mode, by one warp for the real or the imaginary part
+// of a line.  The plane L (lane t's rows [tS, tS + S) at t (S | 1)) holds e and takes
+// the solution; in units of 8 dx^2 the rhs rows are
+//   r_0 = boundary value, r_1 = (e_0 + 10 e_1 + e_2) / 96, r_i = e_{i-1} + 5.5 e_i + e_{i+1},
+//   r_{n-2} = (e_{n-1} + 10 e_{n-2} + e_{n-3}) / 96, r_{n-1} = rn,
+// r0v and rn given unscaled.  T: the mode's row tables (penta_table_size), entries of
+// row tS + q at q * 32 + t: L1 L2 of the forward sweep, SI = 8 dx^2 / u3, C D of
+// the backward sweep, the responses H1 H2 (with SI) and K1 K2 of the rows to the states
+// entering the chunk, then the Kogge-Stone matrices of both sweeps.
+__device__ __forceinline__ void penta_sweeps(const double* __restrict__ T, int S, int n, double* L, double* E, int lane, double r0v,
+                                             double rn, double unit) {
+    const int Sp = S | 1, r0 = min(n, lane * S), r1 = min(n, r0 + S);
+    double* Ul = L + lane * Sp;
+    const double* Tr = T + lane;
+    const int N = 32 * S;   // doubles of one row table
+    auto e = [&](int i) { return L[(i / S) * Sp + i % S]; };
+    if (lane < 4) {   // r_0, r_1, r_{n-2}, r_{n-1}
+        const int i = lane == 1 ? 1 : n - 2;
+        const bool mid = lane == 1 || lane == 2;
+        E[lane] = (mid ? fma(10.0, e(i), e(i - 1) + e(i + 1)) : lane ? rn : r0v) * (mid ? 1.0 / 96.0 : unit);
     }
-    const double *L1 = lu, *L2 = lu + n, *IU3 = lu + 2 * n, *U4 = lu + 3 * n, *U5 = lu + 4 * n;
-    // forward y_i = r_i - l2_i y_{i-1} - l1_i y_{i-2}; row 0 is the boundary row
-    warp_rec2_fwd(Vl, r0, r1, lane, [=](int i) { return i == 0 ? 0.0 : L2[i]; }, [=](int i) { return i <= 1 ? 0.0 : L1[i]; });
-    // backward x_i = (y_i - u4_i x_{i+1} - u5_i x_{i+2}) / u3_i; row 0 keeps its value
-    warp_rec2_bwd(Vl, r0, r1, lane, [=](int i) { return i == 0 ? 0.0 : U4[i]; }, [=](int i) { return i == 0 ? 0.0 : U5[i]; },
-                  [=](int i) { return i == 0 ? 1.0 : IU3[i]; });
+    double ep = (r0 >= 1 && r0 < r1) ? e(r0 - 1) : 0.0;
+    const double en = r1 < n ? e(r1) : 0.0;
     __syncwarp();
-    for (int i = lane; i < n; i += 32)
-        if (i >= 1) out[i] = E[L.slot(i)];
+    double y1 = 0.0, y2 = 0.0;
+    for (int q = 0; q < r1 - r0; q++) {
+        const int i = r0 + q;
+        const double b = Ul[q], c = (i + 1 < r1) ? Ul[q + 1] : en;
+        double t = fma(5.5, b, ep + c);
+        if (i < 2 || i >= n - 2) t = E[i < 2 ? i : i - n + 4];
+        ep = b;
+        const double y = fma(-Tr[N + 32 * q], y1, fma(-Tr[32 * q], y2, t));
+        Ul[q] = y;
+        y2 = y1; y1 = y;
+    }
+    const double* Pf = Tr + 9 * N;
+#pragma unroll
+    for (int d = 0, off = 1; d < 5; d++, off <<= 1) {
+        const double o1 = __shfl_up_sync(0xffffffffu, y1, off), o2 = __shfl_up_sync(0xffffffffu, y2, off);
+        if (lane >= off) {
+            y1 = fma(Pf[128 * d], o1, fma(Pf[128 * d + 32], o2, y1));
+            y2 = fma(Pf[128 * d + 64], o1, fma(Pf[128 * d + 96], o2, y2));
+        }
+    }
+    double Y1 = __shfl_up_sync(0xffffffffu, y1, 1), Y2 = __shfl_up_sync(0xffffffffu, y2, 1);
+    if (lane == 0) { Y1 = 0.0; Y2 = 0.0; }
+    double x1 = 0.0, x2 = 0.0;
+#pragma unroll 2
+    for (int q = r1 - r0 - 1; q >= 0; q--) {
+        const double* t = Tr + 32 * q;
+        const double r = fma(t[5 * N], Y1, fma(t[6 * N], Y2, t[2 * N] * Ul[q]));
+        const double x = fma(-t[3 * N], x1, fma(-t[4 * N], x2, r));
+        Ul[q] = x;
+        x2 = x1; x1 = x;
+    }
+    const double* Pb = Pf + 640;
+#pragma unroll
+    for (int d = 0, off = 1; d < 5; d++, off <<= 1) {
+        const double o1 = __shfl_down_sync(0xffffffffu, x1, off), o2 = __shfl_down_sync(0xffffffffu, x2, off);
+        if (lane + off < 32) {
+            x1 = fma(Pb[128 * d], o1, fma(Pb[128 * d + 32], o2, x1));
+            x2 = fma(Pb[128 * d + 64], o1, fma(Pb[128 * d + 96], o2, x2));
+        }
+    }
+    double X1 = __shfl_down_sync(0xffffffffu, x1, 1), X2 = __shfl_down_sync(0xffffffffu, x2, 1);
+    if (lane == 31) { X1 = 0.0; X2 = 0.0; }
+#pragma unroll 2
+    for (int q = 0; q < r1 - r0; q++) Ul[q] = fma(Tr[7 * N + 32 * q], X1, fma(Tr[8 * N + 32 * q], X2, Ul[q]));
 }
 
-// x-penta Poisson of poi_ux / poi_uz (loop_par.f:519-563, 641-685), one warp
-// per line (j >= 1, k >= 1): e = D + s v_kb W, rhs scaled by g (ux: s = +1,
-// g = -1; uz: s = -1, g = +1); the last row is (g' D + v_kb W) / (k beta)^2.
+// Points t64, t64 + 64, ... of a line shared by a pair of warps: fn(i, slot).
+template <class Fn>
+__device__ __forceinline__ void pair_points(int t64, int S, int n, Fn fn) {
+    const int dc = 64 / S, dr = 64 % S, Sp = S | 1;
+    int c = t64 / S, r = t64 % S;
+#pragma unroll 4
+    for (int i = t64; i < n; i += 64) {
+        fn(i, c * Sp + r);
+        c += dc; r += dr;
+        if (r >= S) { r -= S; c++; }
+    }
+}
+__device__ __forceinline__ void pair_barrier(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+__host__ __device__ inline int penta_line_size(int S) { return 64 * (S | 1) + 8; }   // two planes and the end rows
+
+// x-penta Poisson of poi_ux / poi_uz (loop_par.f:519-563, 641-685), a pair of
+// warps per line (j >= 1, k >= 1), one for its real and one for its imaginary part:
+// with g = -1 (ux) or 1 (uz), e = g D - v_kb W, and the last row is
+// (v_kb W - g D) / (k beta)^2.
+//
+// Bound by the FP64 pipe: 12 instructions a real value (22 with the chunk's
+// responses followed in the sweeps) and the scans.  A block takes a run of lines in the
+// order of the modes and keeps the row tables of the mode it is at in shared
+// memory: 598 us before, 367 us at 1025 x 193 x 32.
 struct PentaArgs {
     const cplx* D;   // d2uydxdy or dwydx
     const cplx* W;   // wy or duydy
     cplx* out;       // ux or uz
-    const double* lu;
-    int nx, ny, K, uz;
-    double dxx, beta;
+    const double* tab;
+    int nx, ny, K, S, staged;
+    double g, beta, unit;
 };
-__global__ void __launch_bounds__(64) k_penta_x(PentaArgs A) {
-    extern __shared__ cplx wsm[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int t = blockIdx.x * (blockDim.x >> 5) + wib;
-    if (t >= (A.ny - 1) * (A.K - 1)) return;
-    const int j = 1 + t % (A.ny - 1), k = 1 + t / (A.ny - 1);
-    const int n = A.nx;
-    const WarpLine L{n, WarpLine::chunk(n), WarpLine::padded(n)};
-    cplx* E = wsm + (size_t)wib * 32 * L.Sp;
-    size_t base = (size_t)n * (j + (size_t)A.ny * k);
-    const cplx* D = A.D + base;
-    const cplx* W = A.W + base;
-    cplx* O = A.out + base;
-    const double kb = (double)k * A.beta;
-    const double s = A.uz ? -1.0 : 1.0, g = A.uz ? 1.0 : -1.0;
-    for (int i = lane; i < n; i += 32) {
-        cplx v = ikb(kb, W[i]), d = D[i];
-        E[L.slot(i)] = make_double2(d.x + s * v.x, d.y + s * v.y);
+constexpr int PENTA_MAX = 8;   // lines per block at most
+__global__ void __launch_bounds__(64 * PENTA_MAX) k_penta_x(PentaArgs A) {
+    extern __shared__ double ps[];
+    const int pair = threadIdx.x >> 6, part = (threadIdx.x >> 5) & 1, lane = threadIdx.x & 31, t64 = threadIdx.x & 63;
+    const int W = blockDim.x >> 6, n = A.nx, S = A.S, rows = A.ny - 1, plane = 32 * (S | 1), tsz = penta_table_size(S);
+    double* F = ps + (A.staged ? tsz : 0) + (size_t)pair * penta_line_size(S);
+    double* L = F + part * plane;
+    const long total = (long)rows * (A.K - 1);
+    const int end = (int)(total * (blockIdx.x + 1) / gridDim.x);
+    for (int first = (int)(total * blockIdx.x / gridDim.x); first < end;) {
+        const int k = 1 + first / rows, last = min(end, k * rows);   // the run's lines of mode k
+        const double* T = A.tab + (size_t)k * tsz;
+        if (A.staged) {
+            __syncthreads();
+            for (int q = threadIdx.x; q < tsz; q += blockDim.x) ps[q] = T[q];
+            __syncthreads();
+            T = ps;
+        }
+        const double kb = (double)k * A.beta, den = 1.0 / ((double)k * (double)k * A.beta * A.beta);
+        for (int t = first + pair; t < last; t += W) {
+            const int j = 1 + t - (k - 1) * rows;
+            const size_t base = (size_t)n * (j + (size_t)A.ny * k);
+            const cplx *D = A.D + base, *Wv = A.W + base;
+            cplx* O = A.out + base;
+            pair_points(t64, S, n, [&](int i, int slot) {
+                const cplx d = D[i], w = Wv[i];
+                F[slot] = fma(-kb, w.y, A.g * d.x);
+                F[plane + slot] = fma(kb, w.x, A.g * d.y);
+            });
+            pair_barrier(1 + pair);
+            const double r0v = reinterpret_cast<const double*>(O)[part];
+            const double rn = -den * L[((n - 1) / S) * (S | 1) + (n - 1) % S];
+            __syncwarp();
+            penta_sweeps(T, S, n, L, F + 2 * plane + 4 * part, lane, r0v, rn, A.unit);
+            pair_barrier(1 + pair);
+            pair_points(t64, S, n, [&](int i, int slot) {
+                if (i >= 1) O[i] = make_double2(F[slot], F[plane + slot]);
+            });
+            pair_barrier(1 + pair);
+        }
+        first = last;
     }
-    __syncwarp();
-    const double den = 1.0 / ((double)k * (double)k * A.beta * A.beta);
-    cplx v = ikb(kb, W[n - 1]), dn = D[n - 1];
-    cplx rn = A.uz ? make_double2((-dn.x + v.x) * den, (-dn.y + v.y) * den) : make_double2((v.x + dn.x) * den, (v.y + dn.y) * den);
-    penta_line(E, L, lane, A.lu + (size_t)k * 5 * n, O[0], rn, g * (A.dxx / 12.0), g * (8.0 * A.dxx), O);
 }
 
 // lapv (loop_par.f:194-205) for every (i, k).
@@ -320,16 +386,13 @@ __global__ void k_dwydy_wall(cplx* out, const cplx* wy, const double* w, int nx,
 
 // wx_wall (loop_par.f:174-255): per mode k >= 1, d2wy/dxdy by explicit
 // stencils, then the x-penta solve with the LU of lhs5 (lusolver_1,
-// penta_par.f:53-127); one warp per mode.
-__global__ void __launch_bounds__(64) k_wx_wall(cplx* wx, const cplx* dwdy, const cplx* lapv, const double* lu_all, int nx,
-                                                int ny, int K, double dx, double dxx, double beta) {
-    extern __shared__ cplx wsm[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int k = 1 + blockIdx.x * (blockDim.x >> 5) + wib;
-    if (k >= K) return;
-    const int n = nx;
-    const WarpLine L{n, WarpLine::chunk(n), WarpLine::padded(n)};
-    cplx* E = wsm + (size_t)wib * 32 * L.Sp;
+// penta_par.f:53-127); a pair of warps per mode.
+__global__ void __launch_bounds__(64) k_wx_wall(cplx* wx, const cplx* dwdy, const cplx* lapv, const double* tab, int nx,
+                                                int ny, int S, double dx, double unit, double beta) {
+    extern __shared__ double ws[];
+    const int part = threadIdx.x >> 5, lane = threadIdx.x & 31, plane = 32 * (S | 1);
+    const int k = 1 + blockIdx.x, n = nx;
+    double* L = ws + part * plane;
     const cplx* dw = dwdy + (size_t)nx * k;
     const cplx* LV = lapv + (size_t)nx * k;
     cplx* WX = wx + (size_t)nx * ny * k;  // row j = 1
@@ -361,21 +424,50 @@ __global__ void __launch_bounds__(64) k_wx_wall(cplx* wx, const cplx* dwdy, cons
         for (int m = 0; m < 7; m++) { acc.x += cw[m] * dw[m].x; acc.y += cw[m] * dw[m].y; }
         return make_double2(acc.x * idx6, acc.y * idx6);
     };
-    for (int i = lane; i < n; i += 32) {
-        cplx a = d2(i), v = ikb(kb, LV[i]);
-        E[L.slot(i)] = make_double2(-a.x + v.x, -a.y + v.y);
-    }
-    __syncwarp();
+    pair_points(threadIdx.x, S, n, [&](int i, int slot) {
+        const cplx a = d2(i), v = ikb(kb, LV[i]);
+        ws[slot] = v.x - a.x;
+        ws[plane + slot] = v.y - a.y;
+    });
+    __syncthreads();
     const double den = 1.0 / ((double)k * (double)k * beta * beta);
-    cplx dd = d2(n - 1), vv = ikb(kb, LV[n - 1]);
-    cplx rn = make_double2((dd.x - vv.x) * den, (dd.y - vv.y) * den);
-    penta_line(E, L, lane, lu_all + (size_t)k * 5 * n, WX[0], rn, dxx / 12.0, 8.0 * dxx, WX);
+    const double r0v = reinterpret_cast<const double*>(WX)[part], rn = -den * L[((n - 1) / S) * (S | 1) + (n - 1) % S];
+    __syncwarp();
+    penta_sweeps(tab + (size_t)k * penta_table_size(S), S, n, L, ws + 2 * plane + 4 * part, lane, r0v, rn, unit);
+    __syncthreads();
+    pair_points(threadIdx.x, S, n, [&](int i, int slot) {
+        if (i >= 1) WX[i] = make_double2(ws[slot], ws[plane + slot]);
+    });
 }
 
 // Shared memory of the warp-per-line x kernels (two line buffers per warp).
 constexpr int XW_WARPS = 2;
 size_t xw_smem(int nx) { return (size_t)XW_WARPS * 64 * WarpLine::padded(nx) * sizeof(cplx); }
-size_t xw_smem1(int nx) { return (size_t)XW_WARPS * 32 * WarpLine::padded(nx) * sizeof(cplx); }   // in-place lines
+
+// A run of lines per block (k_penta_x), as many blocks as the SMs hold, with up to
+// 8 lines at a time.  Blocks of two lines that read the tables from global memory
+// where an SM has fewer than 8 lines, which the copy to shared memory would hold up
+// (257 x 97 x 8: 44 us with it, 27 without), and where the tables leave no room for two.
+int launch_penta(tb_ctx* c, const cplx* D, const cplx* W, cplx* out, double g) {
+    PentaArgs A{D, W, out, c->px.tab, c->g.nx, c->g.ny, c->g.K, c->px.S, 0, g, c->cfg.beta, c->px.unit};
+    const size_t tab = (size_t)penta_table_size(A.S) * sizeof(double), line = (size_t)penta_line_size(A.S) * sizeof(double);
+    const size_t room = (size_t)226 * 1024, sms = c->sm_count > 0 ? c->sm_count : 148;
+    const size_t lines = (size_t)(A.ny - 1) * (A.K - 1);
+    if (line > room) { tb_set_error("x-line of %d points exceeds shared memory", A.nx); return TB_ERR_ARG; }
+    A.staged = tab + 2 * line <= room && lines >= 8 * sms;
+    const size_t t0 = A.staged ? tab : 0;
+    size_t w = std::min<size_t>(A.staged ? PENTA_MAX : 2, (room - t0) / line);
+    if (w >= 4) w &= ~(size_t)3;   // the SM's four sub-partitions
+    const size_t per = std::max<size_t>(1, std::min<size_t>(A.staged ? 3 : 16, room / (t0 + w * line + 1024)));
+    const size_t nb = std::min((lines + w - 1) / w, per * sms);
+    cudaEvent_t ps = nullptr;
+    int r;
+    if ((r = tb_prof_begin(c, PROF_PENTA, &ps))) return r;
+    TB_CUDA(cudaFuncSetAttribute(k_penta_x, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    k_penta_x<<<(unsigned)nb, (unsigned)(64 * w), t0 + w * line, c->stream>>>(A);
+    TB_CHECK_LAUNCH(c);
+    return tb_prof_end(c, PROF_PENTA, ps);
+}
 
 // ts2d_pert / ts3d_pert (main_par.f:1613-1685) for each forced mode.
 struct PertArgs {
@@ -578,14 +670,7 @@ int tb_poi_ux_k(tb_ctx* c, cplx* duydy) {
     cplx* d2 = c->tmp[13];
     XJob xj[1] = {{duydy, d2, XOP_D1}};
     if ((r = tb_launch_xlines(c, xj, 1))) return r;
-    PentaArgs A{d2, c->wy, c->ux, c->px.lu, c->g.nx, c->g.ny, c->g.K, 0, c->cfg.dx * c->cfg.dx, c->cfg.beta};
-    cudaEvent_t ps = nullptr;
-    if ((r = tb_prof_begin(c, PROF_PENTA, &ps))) return r;
-    const size_t sp = xw_smem1(c->g.nx);
-    TB_CUDA(cudaFuncSetAttribute(k_penta_x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp));
-    k_penta_x<<<tb_blocks((size_t)(c->g.ny - 1) * (c->g.K - 1), XW_WARPS), 32 * XW_WARPS, sp, c->stream>>>(A);
-    TB_CHECK_LAUNCH(c);
-    return tb_prof_end(c, PROF_PENTA, ps);
+    return launch_penta(c, d2, c->wy, c->ux, -1.0);
 }
 int tb_poi_uz_k(tb_ctx* c, const cplx* duydy) {
     if (c->g.K < 2) return TB_OK;
@@ -593,14 +678,7 @@ int tb_poi_uz_k(tb_ctx* c, const cplx* duydy) {
     cplx* dwydx = c->tmp[14];
     XJob xj[1] = {{c->wy, dwydx, XOP_D1}};
     if ((r = tb_launch_xlines(c, xj, 1))) return r;
-    PentaArgs A{dwydx, duydy, c->uz, c->px.lu, c->g.nx, c->g.ny, c->g.K, 1, c->cfg.dx * c->cfg.dx, c->cfg.beta};
-    cudaEvent_t ps = nullptr;
-    if ((r = tb_prof_begin(c, PROF_PENTA, &ps))) return r;
-    const size_t sp = xw_smem1(c->g.nx);
-    TB_CUDA(cudaFuncSetAttribute(k_penta_x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp));
-    k_penta_x<<<tb_blocks((size_t)(c->g.ny - 1) * (c->g.K - 1), XW_WARPS), 32 * XW_WARPS, sp, c->stream>>>(A);
-    TB_CHECK_LAUNCH(c);
-    return tb_prof_end(c, PROF_PENTA, ps);
+    return launch_penta(c, dwydx, duydy, c->uz, 1.0);
 }
 int tb_wx_wall_k(tb_ctx* c, cplx* lapv) {
     const double* wat = c->coefs.data() + 100 + 24 * c->g.msh - 17;  // w_at_w_coef(9) on the host
@@ -614,11 +692,10 @@ int tb_wx_wall_k(tb_ctx* c, cplx* lapv) {
     cplx* dw = c->tmp[15];
     k_dwydy_wall<<<nb, 128, 0, c->stream>>>(dw, c->wy, dcoef + 9, c->g.nx, c->g.ny, c->g.K, 1.0 / c->cfg.dy);
     TB_CHECK_LAUNCH(c);
-    size_t sm = xw_smem1(c->g.nx);
-    TB_CUDA(cudaFuncSetAttribute(k_wx_wall, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_wx_wall<<<tb_blocks(c->g.K - 1, XW_WARPS), 32 * XW_WARPS, sm, c->stream>>>(c->wx, dw, lapv, c->px.lu, c->g.nx, c->g.ny,
-                                                                                 c->g.K, c->cfg.dx, c->cfg.dx * c->cfg.dx,
-                                                                                 c->cfg.beta);
+    const size_t sm = (size_t)penta_line_size(c->px.S) * sizeof(double);
+    TB_CUDA(cudaFuncSetAttribute(k_wx_wall, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    k_wx_wall<<<c->g.K - 1, 64, sm, c->stream>>>(c->wx, dw, lapv, c->px.tab, c->g.nx, c->g.ny, c->px.S, c->cfg.dx, c->px.unit,
+                                                 c->cfg.beta);
     TB_CHECK_LAUNCH(c);
     return TB_OK;
 }

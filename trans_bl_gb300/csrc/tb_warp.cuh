@@ -1,9 +1,8 @@
 // tb_warp.cuh -- second-order linear recurrences along a line shared by the
 // 32 lanes of a warp.
 //
-// The x-direction solves of the stage (pentadiagonal LU sweeps, the 4th-order
-// implicit x integrations of continuity and of the wall vorticity) are
-// recurrences y_i = f(y_{i-1}, y_{i-2}) along lines of ~1000 points.  One
+// The 4th-order implicit x integrations of the stage (continuity, the wall
+// vorticity) are recurrences y_i = f(y_{i-1}, y_{i-2}) along lines of ~1000 points.  One
 // thread per line leaves most of the GPU idle (a few hundred lines); here a
 // warp owns a line and lane t owns rows [r0, r1) = [tS, min(n, tS + S)).  A
 // recurrence runs in three passes:
@@ -69,50 +68,5 @@ __device__ __forceinline__ void warp_rec2_fwd(cplx* Bl, int r0, int r1, int lane
         c2 = c1; c1 = z;
         cplx y = Bl[i - r0];
         Bl[i - r0] = make_double2(y.x + z.x, y.y + z.y);
-    }
-}
-
-// Backward: x_i = (y_i - c(i) x_{i+1} - d(i) x_{i+2}) * s(i) for all rows,
-// x_n = x_{n+1} = 0.  Bl holds this lane's rows (y on entry, x on exit).
-template <class FC, class FD, class FS>
-__device__ __forceinline__ void warp_rec2_bwd(cplx* Bl, int r0, int r1, int lane, FC c, FD d, FS s) {
-    cplx x1 = make_double2(0.0, 0.0), x2 = make_double2(0.0, 0.0);
-    double p1 = 1.0, p2 = 0.0, q1 = 0.0, q2 = 1.0;   // responses to (x_{r1}, x_{r1+1})
-    for (int i = r1 - 1; i >= r0; i--) {
-        double ci = c(i), di = d(i), si = s(i);
-        cplx y = Bl[i - r0];
-        cplx x = make_double2((y.x - ci * x1.x - di * x2.x) * si, (y.y - ci * x1.y - di * x2.y) * si);
-        Bl[i - r0] = x;
-        x2 = x1; x1 = x;
-        double p = (-ci * p1 - di * p2) * si; p2 = p1; p1 = p;
-        double q = (-ci * q1 - di * q2) * si; q2 = q1; q1 = q;
-    }
-    double m00 = p1, m01 = q1, m10 = p2, m11 = q2;
-    cplx e0 = x1, e1 = x2;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        double n00 = __shfl_down_sync(0xffffffffu, m00, off), n01 = __shfl_down_sync(0xffffffffu, m01, off);
-        double n10 = __shfl_down_sync(0xffffffffu, m10, off), n11 = __shfl_down_sync(0xffffffffu, m11, off);
-        cplx f0, f1;
-        f0.x = __shfl_down_sync(0xffffffffu, e0.x, off); f0.y = __shfl_down_sync(0xffffffffu, e0.y, off);
-        f1.x = __shfl_down_sync(0xffffffffu, e1.x, off); f1.y = __shfl_down_sync(0xffffffffu, e1.y, off);
-        if (lane + off < 32) {
-            e0 = make_double2(e0.x + m00 * f0.x + m01 * f1.x, e0.y + m00 * f0.y + m01 * f1.y);
-            e1 = make_double2(e1.x + m10 * f0.x + m11 * f1.x, e1.y + m10 * f0.y + m11 * f1.y);
-            double t00 = m00 * n00 + m01 * n10, t01 = m00 * n01 + m01 * n11;
-            double t10 = m10 * n00 + m11 * n10, t11 = m10 * n01 + m11 * n11;
-            m00 = t00; m01 = t01; m10 = t10; m11 = t11;
-        }
-    }
-    cplx c1, c2;   // true x_{r1}, x_{r1+1}
-    c1.x = __shfl_down_sync(0xffffffffu, e0.x, 1); c1.y = __shfl_down_sync(0xffffffffu, e0.y, 1);
-    c2.x = __shfl_down_sync(0xffffffffu, e1.x, 1); c2.y = __shfl_down_sync(0xffffffffu, e1.y, 1);
-    if (lane == 31) { c1 = make_double2(0.0, 0.0); c2 = c1; }
-    for (int i = r1 - 1; i >= r0; i--) {
-        double ci = c(i), di = d(i), si = s(i);
-        cplx z = make_double2((-ci * c1.x - di * c2.x) * si, (-ci * c1.y - di * c2.y) * si);
-        c2 = c1; c1 = z;
-        cplx x = Bl[i - r0];
-        Bl[i - r0] = make_double2(x.x + z.x, x.y + z.y);
     }
 }
