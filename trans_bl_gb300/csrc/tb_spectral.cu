@@ -7,9 +7,15 @@
 // and the forward transform returns c_0 = (1/P) sum p_n, c_k = (2/P) sum p_n
 // e^{+2 pi i k n / P}, zeroes components below 1e-14 and forces Im c_0 = 0.
 // Both directions are computed here as a length-P/2 complex FFT plus the
-// real-to-complex split, one thread per (i, j) grid line, with exact
-// twiddles from a constant table instead of the reference's rotation
-// recurrence.
+// real-to-complex split, with exact twiddles from constant tables instead of
+// the reference's rotation recurrence: one thread per (i, j) grid line, and in
+// FP64 two at P = 128, where one line's values are more than a thread's registers.
+//
+// An FP64 warp instruction (comparisons included) holds its pipe for 64
+// cycles, so the FP64 transforms are written for their number: a butterfly is
+// six fused multiply-adds (twiddle w = m (1 + i r) or m (r + i), |r| <= 1), the
+// split takes the modes k and P/2 - k together (12 in place of 28), its halves and
+// the 1/P are left to the caller's factors, and values are compared as integers.
 #include "tb_internal.h"
 #include "tb_tc.cuh"
 #include <cuda_bf16.h>
@@ -19,18 +25,15 @@
 
 #define TW_N 512
 __constant__ double c_twr[TW_N], c_twi[TW_N];  // e^{-2 pi i t / TW_N}
+__constant__ double c_lfm[TW_N / 2], c_lfr[TW_N / 2];   // the same as m (1 + i r) or m (r + i), see fft
 __constant__ float c_twrf[TW_N], c_twif[TW_N]; // the same, rounded to FP32
 
 namespace {
 
 __device__ __forceinline__ double twr(int t) { return c_twr[t & (TW_N - 1)]; }
 __device__ __forceinline__ double twi(int t) { return c_twi[t & (TW_N - 1)]; }
-template <class R> __device__ __forceinline__ R tw_r(int t);
-template <class R> __device__ __forceinline__ R tw_i(int t);
-template <> __device__ __forceinline__ double tw_r<double>(int t) { return c_twr[t & (TW_N - 1)]; }
-template <> __device__ __forceinline__ double tw_i<double>(int t) { return c_twi[t & (TW_N - 1)]; }
-template <> __device__ __forceinline__ float tw_r<float>(int t) { return c_twrf[t & (TW_N - 1)]; }
-template <> __device__ __forceinline__ float tw_i<float>(int t) { return c_twif[t & (TW_N - 1)]; }
+__device__ __forceinline__ float twr_f(int t) { return c_twrf[t & (TW_N - 1)]; }
+__device__ __forceinline__ float twi_f(int t) { return c_twif[t & (TW_N - 1)]; }
 
 template <int N>
 __device__ __forceinline__ int brev(int i) {
@@ -40,15 +43,15 @@ __device__ __forceinline__ int brev(int i) {
     return r;
 }
 
-// In-place radix-2 complex FFT of length N. SIGN = -1: sum X_k e^{-2 pi i km/N};
+// In-place radix-2 complex FFT of length N in FP32. SIGN = -1: sum X_k e^{-2 pi i km/N};
 // SIGN = +1: sum X_k e^{+2 pi i km/N}.
-template <int N, int SIGN, class R = double>
-__device__ __forceinline__ void cfft(R* re, R* im) {
+template <int N, int SIGN>
+__device__ __forceinline__ void cfft(float* re, float* im) {
 #pragma unroll
     for (int i = 0; i < N; i++) {
         int j = brev<N>(i);
         if (j > i) {
-            R t = re[i]; re[i] = re[j]; re[j] = t;
+            float t = re[i]; re[i] = re[j]; re[j] = t;
             t = im[i]; im[i] = im[j]; im[j] = t;
         }
     }
@@ -60,15 +63,15 @@ __device__ __forceinline__ void cfft(R* re, R* im) {
 #pragma unroll
             for (int q = 0; q < h; q++) {
                 int a = s + q, b = a + h;
-                R tr, ti;
+                float tr, ti;
                 if (q == 0) {
                     tr = re[b]; ti = im[b];
                 } else if (4 * q == len) {  // twiddle -SIGN*i ... e^{SIGN*i*pi/2} = SIGN*i
                     tr = (SIGN < 0) ? im[b] : -im[b];
                     ti = (SIGN < 0) ? -re[b] : re[b];
                 } else {
-                    R wr = tw_r<R>(q * (TW_N / len));
-                    R wi = (SIGN < 0) ? tw_i<R>(q * (TW_N / len)) : -tw_i<R>(q * (TW_N / len));
+                    float wr = twr_f(q * (TW_N / len));
+                    float wi = (SIGN < 0) ? twi_f(q * (TW_N / len)) : -twi_f(q * (TW_N / len));
                     tr = wr * re[b] - wi * im[b];
                     ti = wr * im[b] + wi * re[b];
                 }
@@ -79,52 +82,208 @@ __device__ __forceinline__ void cfft(R* re, R* im) {
     }
 }
 
-// Fourier (K modes at stride cs) -> physical p[0..P-1].
-template <int P>
-__device__ __forceinline__ void to_phys(const cplx* __restrict__ cf, size_t cs, int K, double* p) {
+// |cos| >= |sin| of the angle 2 pi t / TW_N, 0 <= t < TW_N / 2.
+__host__ __device__ constexpr bool lf_big(int t) { return t <= TW_N / 8 || t >= 3 * TW_N / 8; }
+
+// The same in FP64, six fused multiply-adds a butterfly: w b = m u with
+// u = (1 + i r) b or (r + i) b, and a +- m u.
+template <int N, int SIGN>
+__device__ __forceinline__ void fft(double* re, double* im) {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        int j = brev<N>(i);
+        if (j > i) {
+            double t = re[i]; re[i] = re[j]; re[j] = t;
+            t = im[i]; im[i] = im[j]; im[j] = t;
+        }
+    }
+#pragma unroll
+    for (int len = 2; len <= N; len <<= 1) {
+        const int h = len / 2;
+#pragma unroll
+        for (int s = 0; s < N; s += len) {
+#pragma unroll
+            for (int q = 0; q < h; q++) {
+                const int a = s + q, b = a + h;
+                const double ar = re[a], ai = im[a], br = re[b], bi = im[b];
+                if (q == 0) {
+                    re[b] = ar - br; im[b] = ai - bi;
+                    re[a] = ar + br; im[a] = ai + bi;
+                } else if (4 * q == len) {   // w = SIGN i
+                    const double tr = (SIGN < 0) ? bi : -bi, ti = (SIGN < 0) ? -br : br;
+                    re[b] = ar - tr; im[b] = ai - ti;
+                    re[a] = ar + tr; im[a] = ai + ti;
+                } else {
+                    const int t = q * (TW_N / len);
+                    const double m = c_lfm[t], r = c_lfr[t];
+                    double ur, ui;
+                    if (lf_big(t)) {
+                        ur = fma(SIGN < 0 ? -r : r, bi, br);
+                        ui = fma(SIGN < 0 ? r : -r, br, bi);
+                    } else {   // SIGN > 0: conj(w) = m (r + i) with m -> -m, r -> -r
+                        ur = fma(r, br, SIGN < 0 ? -bi : bi);
+                        ui = fma(r, bi, SIGN < 0 ? br : -br);
+                    }
+                    re[b] = fma(-m, ur, ar); im[b] = fma(-m, ui, ai);
+                    re[a] = fma(m, ur, ar); im[a] = fma(m, ui, ai);
+                }
+            }
+        }
+    }
+}
+
+// Components below 1e-14 -> 0, compared by their bits.
+__device__ __forceinline__ double zap(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+    return b < 0x3d06849b86a12b9bull ? 0.0 : v;   // 1e-14
+}
+
+// The K modes of a grid line at stride cs, zero beyond.
+struct Modes {
+    const cplx* f;
+    size_t cs;
+    int K;
+    __device__ __forceinline__ cplx operator()(int k) const { return k < K ? f[(size_t)k * cs] : make_double2(0.0, 0.0); }
+};
+
+// Inverse split of the modes k and N - k, twice its value: Z_k and Z_{N-k} of
+// the length-N transform; (wr, wi) = e^{-2 pi i k / P}.
+__device__ __forceinline__ void split_in(cplx A, cplx B, double wr, double wi, double& zr, double& zi, double& yr, double& yi) {
+    const double sr = A.x + B.x, si = A.y - B.y, dr = A.x - B.x, di = A.y + B.y;
+    const double t1 = fma(wr, di, wi * dr), t2 = fma(wr, dr, -(wi * di));
+    zr = sr - t1; zi = si + t2;
+    yr = sr + t1; yi = t2 - si;
+}
+// Forward split: the modes k (a) and N - k (b), times P, of F_k and F_{N-k};
+// (vr, vi) = e^{+2 pi i k / P}.
+__device__ __forceinline__ void split_out(double fr, double fi, double gr, double gi, double vr, double vi, cplx& a, cplx& b) {
+    const double sr = fr + gr, si = fi - gi, dr = fr - gr, di = fi + gi;
+    const double t1 = fma(vr, di, vi * dr), t2 = fma(vi, di, -(vr * dr));
+    a = make_double2(zap(sr + t1), zap(si + t2));
+    b = make_double2(zap(sr - t1), zap(t2 - si));
+}
+
+// Fourier (load(k) gives mode k) -> twice the physical values p[0..P-1].
+template <int P, class Load>
+__device__ __forceinline__ void to_phys2(const Load& load, double* p) {
     constexpr int N = P / 2;
     double re[N], im[N];
-    cplx c0 = cf[0];
-    double C0 = c0.x, CN = 0.5 * c0.y;
-    re[0] = C0 + CN; im[0] = C0 - CN;
+    const cplx c0 = load(0);
+    re[0] = fma(2.0, c0.x, c0.y); im[0] = fma(2.0, c0.x, -c0.y);
 #pragma unroll
-    for (int k = 1; k < N; k++) {
-        cplx A = (k < K) ? cf[(size_t)k * cs] : make_double2(0.0, 0.0);
-        cplx Bc = (N - k < K) ? cf[(size_t)(N - k) * cs] : make_double2(0.0, 0.0);
-        double Br = Bc.x, Bi = -Bc.y;  // conj
-        double sr = 0.5 * (A.x + Br), si = 0.5 * (A.y + Bi);
-        double dr = 0.5 * (A.x - Br), di = 0.5 * (A.y - Bi);
-        double wr = twr(k * (TW_N / P)), wi = twi(k * (TW_N / P));  // e^{-2 pi i k / P}
-        re[k] = sr - (wr * di + wi * dr);
-        im[k] = si + (wr * dr - wi * di);
+    for (int k = 1; 2 * k < N; k++)
+        split_in(load(k), load(N - k), twr(k * (TW_N / P)), twi(k * (TW_N / P)), re[k], im[k], re[N - k], im[N - k]);
+    if (N > 1) {
+        const cplx c = load(N / 2);
+        re[N / 2] = 2.0 * c.x; im[N / 2] = 2.0 * c.y;
     }
-    cfft<N, -1>(re, im);
+    fft<N, -1>(re, im);
 #pragma unroll
     for (int m = 0; m < N; m++) { p[2 * m] = re[m]; p[2 * m + 1] = im[m]; }
 }
 
-__device__ __forceinline__ double zap(double v) { return fabs(v) < 1e-14 ? 0.0 : v; }
-
-// physical p[0..P-1] -> Fourier (K modes at stride cs).
-template <int P>
-__device__ __forceinline__ void to_four(const double* p, int K, cplx* __restrict__ cf, size_t cs) {
+// P^-1 times the physical values p[0..P-1] -> Fourier, store(k, mode k) for
+// every k < P/2.
+template <int P, class Store>
+__device__ __forceinline__ void to_four(const double* p, const Store& store) {
     constexpr int N = P / 2;
     double re[N], im[N];
 #pragma unroll
     for (int m = 0; m < N; m++) { re[m] = p[2 * m]; im[m] = p[2 * m + 1]; }
-    cfft<N, +1>(re, im);
-    const double invP = 1.0 / (double)P, two_P = 2.0 / (double)P;
-    cf[0] = make_double2(zap((re[0] + im[0]) * invP), 0.0);
+    fft<N, +1>(re, im);
+    store(0, make_double2(zap(re[0] + im[0]), 0.0));
 #pragma unroll
-    for (int k = 1; k < N; k++) {
-        if (k >= K) continue;
-        double Fr = re[k], Fi = im[k], Gr = re[N - k], Gi = -im[N - k];  // conj(F_{N-k})
-        double Er = 0.5 * (Fr + Gr), Ei = 0.5 * (Fi + Gi);
-        double gr = Fr - Gr, gi = Fi - Gi;
-        double Or = 0.5 * gi, Oi = -0.5 * gr;  // g / (2i)
-        double vr = twr(k * (TW_N / P)), vi = -twi(k * (TW_N / P));  // e^{+2 pi i k / P}
-        double Hr = Er + (vr * Or - vi * Oi), Hi = Ei + (vr * Oi + vi * Or);
-        cf[(size_t)k * cs] = make_double2(zap(two_P * Hr), zap(two_P * Hi));
+    for (int k = 1; 2 * k < N; k++) {
+        cplx a, b;
+        split_out(re[k], im[k], re[N - k], im[N - k], twr(k * (TW_N / P)), -twi(k * (TW_N / P)), a, b);
+        store(k, a);
+        store(N - k, b);
+    }
+    if (N > 1) store(N / 2, make_double2(zap(2.0 * re[N / 2]), zap(2.0 * im[N / 2])));
+}
+
+// A grid line on TP threads (lanes l and l ^ 16): thread p holds the values
+// m = j TP + p, j < M, of the length-N transform, that is the physical points
+// 2m and 2m + 1, and on the Fourier side the modes k of parity p.
+template <int P>
+struct Col {
+    static constexpr int N = P / 2, TP = P >= 128 ? 2 : 1, M = N / TP;
+    static constexpr int VAL = 2 * M, PER_BLOCK = 128 / TP;   // physical values of a thread; lines of a block
+};
+// The last stage over both threads' length-M transforms, thread p for the
+// outputs k and k + M, k = 2i + p (positions i and M/2 + i).
+template <int P, int SIGN>
+__device__ __forceinline__ void join(int p, double* re, double* im) {
+    constexpr int N = Col<P>::N, M = Col<P>::M;
+    double xr[M], xi[M];
+#pragma unroll
+    for (int i = 0; i < M; i++) { xr[i] = re[i]; xi[i] = im[i]; }
+#pragma unroll
+    for (int i = 0; i < M / 2; i++) {
+        const double sr = __shfl_xor_sync(0xffffffffu, p ? xr[2 * i] : xr[2 * i + 1], 16);
+        const double si = __shfl_xor_sync(0xffffffffu, p ? xi[2 * i] : xi[2 * i + 1], 16);
+        const double wr_ = p ? xr[2 * i + 1] : xr[2 * i], wi_ = p ? xi[2 * i + 1] : xi[2 * i];   // own
+        const double er = p ? sr : wr_, ei = p ? si : wi_, orr = p ? wr_ : sr, oi = p ? wi_ : si;
+        const int t = (2 * i + p) * (TW_N / N);
+        const double c = twr(t), s = SIGN < 0 ? twi(t) : -twi(t);
+        const double tr = fma(c, orr, -(s * oi)), ti = fma(c, oi, s * orr);
+        re[i] = er + tr; im[i] = ei + ti;
+        re[M / 2 + i] = er - tr; im[M / 2 + i] = ei - ti;
+    }
+}
+template <int P, class Load>
+__device__ __forceinline__ void col_phys2(const Load& load, int p, double* re, double* im) {
+    constexpr int N = Col<P>::N, M = Col<P>::M;
+    if constexpr (Col<P>::TP == 1) {
+        double v[P];
+        to_phys2<P>(load, v);
+#pragma unroll
+        for (int m = 0; m < N; m++) { re[m] = v[2 * m]; im[m] = v[2 * m + 1]; }
+    } else {
+        double yr[M / 2 + 1], yi[M / 2 + 1];   // Z_{N-k}
+#pragma unroll
+        for (int i = 0; i < M / 2; i++) {
+            const int k = 2 * i + p, t = k * (TW_N / P);
+            split_in(load(k), load(k ? N - k : 0), twr(t), twi(t), re[i], im[i], yr[i], yi[i]);
+        }
+        const cplx c0 = load(0), cm = load(N / 2);
+        if (p == 0) { re[0] = fma(2.0, c0.x, c0.y); im[0] = fma(2.0, c0.x, -c0.y); }
+        yr[M / 2] = 2.0 * cm.x; yi[M / 2] = 2.0 * cm.y;
+#pragma unroll
+        for (int q = M / 2; q < M; q++) {
+            re[q] = p ? yr[M - 1 - q] : yr[M - q];
+            im[q] = p ? yi[M - 1 - q] : yi[M - q];
+        }
+        fft<M, -1>(re, im);
+        join<P, -1>(p, re, im);
+    }
+}
+template <int P, class Store>
+__device__ __forceinline__ void col_four(double* re, double* im, int p, const Store& store) {
+    constexpr int N = Col<P>::N, M = Col<P>::M;
+    if constexpr (Col<P>::TP == 1) {
+        double v[P];
+#pragma unroll
+        for (int m = 0; m < N; m++) { v[2 * m] = re[m]; v[2 * m + 1] = im[m]; }
+        to_four<P>(v, store);
+    } else {
+        fft<M, +1>(re, im);
+        join<P, +1>(p, re, im);
+#pragma unroll
+        for (int i = 0; i < M / 2; i++) {
+            const int k = 2 * i + p, t = k * (TW_N / P);
+            const double gr = p ? re[M - 1 - i] : re[i ? M - i : 0], gi = p ? im[M - 1 - i] : im[i ? M - i : 0];
+            cplx a, b;
+            split_out(re[i], im[i], gr, gi, twr(t), -twi(t), a, b);
+            if (k) {
+                store(k, a);
+                store(N - k, b);
+            }
+        }
+        if (p == 0) {
+            store(0, make_double2(zap(re[0] + im[0]), 0.0));
+            store(N / 2, make_double2(zap(2.0 * re[M / 2]), zap(2.0 * im[M / 2])));
+        }
     }
 }
 
@@ -134,9 +293,9 @@ __global__ void __launch_bounds__(128) k_f_to_p(double* phys, const cplx* four, 
     int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n2) return;
     double p[P];
-    to_phys<P>(four + q, n2, K, p);
+    to_phys2<P>(Modes{four + q, (size_t)n2, K}, p);
 #pragma unroll
-    for (int z = 0; z < P; z++) phys[(size_t)q + (size_t)n2 * z] = p[z];
+    for (int z = 0; z < P; z++) phys[(size_t)q + (size_t)n2 * z] = 0.5 * p[z];
 }
 template <int P>
 __global__ void __launch_bounds__(128) k_p_to_f(cplx* four, const double* phys, int n2, int K) {
@@ -144,8 +303,8 @@ __global__ void __launch_bounds__(128) k_p_to_f(cplx* four, const double* phys, 
     if (q >= n2) return;
     double p[P];
 #pragma unroll
-    for (int z = 0; z < P; z++) p[z] = phys[(size_t)q + (size_t)n2 * z];
-    to_four<P>(p, K, four + q, n2);
+    for (int z = 0; z < P; z++) p[z] = (1.0 / (double)P) * phys[(size_t)q + (size_t)n2 * z];
+    to_four<P>(p, [&](int k, cplx v) { if (k < K) four[(size_t)q + (size_t)n2 * k] = v; });
 }
 
 // nlterms_fi (nlterms_par.f:41-86): a = uy wx - ux wy, b = ux wz - uz wx, c = uz wy - uy wz.
@@ -159,23 +318,21 @@ __global__ void __launch_bounds__(128) k_nlterms(NlArgs A) {
     int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= A.n2) return;
     size_t cs = A.n2;
+    const cplx* fs[6] = {A.ux, A.uy, A.uz, A.wx, A.wy, A.wz};
     double ph[6][P];
-    to_phys<P>(A.ux + q, cs, A.K, ph[0]);
-    to_phys<P>(A.uy + q, cs, A.K, ph[1]);
-    to_phys<P>(A.uz + q, cs, A.K, ph[2]);
-    to_phys<P>(A.wx + q, cs, A.K, ph[3]);
-    to_phys<P>(A.wy + q, cs, A.K, ph[4]);
-    to_phys<P>(A.wz + q, cs, A.K, ph[5]);
+#pragma unroll
+    for (int f = 0; f < 6; f++) to_phys2<P>(Modes{fs[f] + q, cs, A.K}, ph[f]);
+    constexpr double sc = 0.25 / (double)P;   // the fields' factors 2 and the forward transform's 1 / P
 #pragma unroll
     for (int z = 0; z < P; z++) {
-        double ux = ph[0][z], uy = ph[1][z], uz = ph[2][z], wx = ph[3][z], wy = ph[4][z], wz = ph[5][z];
+        double ux = sc * ph[0][z], uy = sc * ph[1][z], uz = sc * ph[2][z], wx = ph[3][z], wy = ph[4][z], wz = ph[5][z];
         ph[0][z] = uy * wx - ux * wy;
         ph[1][z] = ux * wz - uz * wx;
         ph[2][z] = uz * wy - uy * wz;
     }
-    to_four<P>(ph[0], A.K, A.a + q, cs);
-    to_four<P>(ph[1], A.K, A.b + q, cs);
-    to_four<P>(ph[2], A.K, A.c + q, cs);
+    cplx* outs[3] = {A.a, A.b, A.c};
+#pragma unroll
+    for (int f = 0; f < 3; f++) to_four<P>(ph[f], [&](int k, cplx v) { if (k < A.K) outs[f][q + cs * k] = v; });
 }
 
 // ---------------------------------------------------------------------------
@@ -204,11 +361,11 @@ __device__ __forceinline__ void to_phys_dist(const cplx* __restrict__ cf, size_t
         float Ar = (float)A.x, Ai = (float)A.y, Br = (float)Bc.x, Bi = -(float)Bc.y;
         float sr = 0.5f * (Ar + Br), si = 0.5f * (Ai + Bi);
         float dr = 0.5f * (Ar - Br), di = 0.5f * (Ai - Bi);
-        float wr = tw_r<float>(k * (TW_N / P)), wi = tw_i<float>(k * (TW_N / P));
+        float wr = twr_f(k * (TW_N / P)), wi = twi_f(k * (TW_N / P));
         re[k] = sr - (wr * di + wi * dr);
         im[k] = si + (wr * dr - wi * di);
     }
-    cfft<N, -1, float>(re, im);
+    cfft<N, -1>(re, im);
 #pragma unroll
     for (int m = 0; m < N; m++) { p[2 * m] = re[m]; p[2 * m + 1] = im[m]; }
 }
@@ -220,7 +377,7 @@ __device__ __forceinline__ void to_four_f(const float* p, float* cr, float* ci) 
     float re[N], im[N];
 #pragma unroll
     for (int m = 0; m < N; m++) { re[m] = p[2 * m]; im[m] = p[2 * m + 1]; }
-    cfft<N, +1, float>(re, im);
+    cfft<N, +1>(re, im);
     const float invP = 1.0f / (float)P, two_P = 2.0f / (float)P;
     cr[0] = (re[0] + im[0]) * invP; ci[0] = 0.0f;
 #pragma unroll
@@ -229,7 +386,7 @@ __device__ __forceinline__ void to_four_f(const float* p, float* cr, float* ci) 
         float Er = 0.5f * (Fr + Gr), Ei = 0.5f * (Fi + Gi);
         float gr = Fr - Gr, gi = Fi - Gi;
         float Or = 0.5f * gi, Oi = -0.5f * gr;
-        float vr = tw_r<float>(k * (TW_N / P)), vi = -tw_i<float>(k * (TW_N / P));
+        float vr = twr_f(k * (TW_N / P)), vi = -twi_f(k * (TW_N / P));
         cr[k] = two_P * (Er + (vr * Or - vi * Oi));
         ci[k] = two_P * (Ei + (vr * Oi + vi * Or));
     }
@@ -559,29 +716,23 @@ struct LesArgs {
     int nx, ny, n2, K, damping;
     double beta, Re, fac_y, dy, stf, Cs, Aplus, delta_les;
 };
+// Eddy viscosity and force of one grid line on Col<P>::TP threads, each with
+// its share of the strain in shared memory.  The six distinct strain
+// components are summed before their transforms: six of these, three of the
+// Laplacian and three back, where the nine velocity gradients took fifteen.
+// Bound by the FP64 pipe: 19.6 ms at 1025 x 193 x 64 (P = 128) with one thread a
+// line and its arrays in local memory, 10.3 ms now.
 template <int P>
-__device__ __forceinline__ void to_phys_dz(const cplx* __restrict__ u, size_t cs, int K, double beta, double* p) {
-    // z-derivative in Fourier space: v_kb(k) u = -i (k-1) beta u  (main_par.f:1888)
-    constexpr int N = P / 2;
-    cplx tmp[N];
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-        if (k < K) {
-            cplx v = u[(size_t)k * cs];
-            double kb = -(double)k * beta;
-            tmp[k] = make_double2(-kb * v.y, kb * v.x);
-        } else {
-            tmp[k] = make_double2(0.0, 0.0);
-        }
-    }
-    to_phys<P>(tmp, 1, K < N ? K : N, p);
-}
-template <int P>
-__global__ void __launch_bounds__(128) k_les(LesArgs A) {
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= A.n2) return;
-    size_t cs = A.n2;
-    int i = q % A.nx, j = q / A.nx;
+__global__ void __launch_bounds__(128, 2) k_les(LesArgs A) {
+    using CP = Col<P>;
+    constexpr int M = CP::M;
+    extern __shared__ double strain[];
+    const int tid = threadIdx.x, p = CP::TP == 2 ? (tid >> 4) & 1 : 0;
+    const int col = blockIdx.x * CP::PER_BLOCK + (CP::TP == 2 ? (tid >> 5) * 16 + (tid & 15) : tid);
+    const bool in = col < A.n2;
+    const int q = in ? col : A.n2 - 1;   // both threads of a line take part in its shuffles
+    const size_t cs = A.n2;
+    const int i = q % A.nx, j = q / A.nx;
     double y = (A.stf == 1.0) ? (double)j * A.dy : A.dy * (pow(A.stf, (double)j) - 1.0) / (A.stf - 1.0);
     double wz0 = (A.damping & 2) ? fabs(A.wz[i].x) : A.wz[i].x;
     double yplus = sqrt(A.Re * wz0 / sqrt(A.fac_y)) * y;
@@ -594,53 +745,50 @@ __global__ void __launch_bounds__(128) k_les(LesArgs A) {
         ratio = ratio * ratio * ratio;
         damp = 1.0 - exp(-ratio);
     }
-    double cte = A.Cs * A.Cs * A.delta_les * A.delta_les * damp;
-    double dg[P], of[P], t1[P], t2[P];
-    to_phys<P>(A.dudx + q, cs, A.K, t1);
-#pragma unroll
-    for (int z = 0; z < P; z++) dg[z] = t1[z] * t1[z];
-    to_phys<P>(A.dvdy + q, cs, A.K, t1);
-#pragma unroll
-    for (int z = 0; z < P; z++) dg[z] += t1[z] * t1[z];
-    to_phys_dz<P>(A.uz + q, cs, A.K, A.beta, t1);
-#pragma unroll
-    for (int z = 0; z < P; z++) dg[z] += t1[z] * t1[z];
-    to_phys<P>(A.dudy + q, cs, A.K, t1);
-    to_phys<P>(A.dvdx + q, cs, A.K, t2);
-#pragma unroll
-    for (int z = 0; z < P; z++) { double s = 0.5 * (t1[z] + t2[z]); of[z] = s * s; }
-    to_phys_dz<P>(A.ux + q, cs, A.K, A.beta, t1);
-    to_phys<P>(A.dwdx + q, cs, A.K, t2);
-#pragma unroll
-    for (int z = 0; z < P; z++) { double s = 0.5 * (t1[z] + t2[z]); of[z] += s * s; }
-    to_phys_dz<P>(A.uy + q, cs, A.K, A.beta, t1);
-    to_phys<P>(A.dwdy + q, cs, A.K, t2);
-#pragma unroll
-    for (int z = 0; z < P; z++) {
-        double s = 0.5 * (t1[z] + t2[z]);
-        of[z] += s * s;
-        dg[z] = cte * sqrt(2.0 * (dg[z] + 2.0 * of[z]));  // nu_t
-    }
-    const cplx* us[3] = {A.ux, A.uy, A.uz};
-    cplx* outs[3] = {A.fx, A.fy, A.fz};
-    constexpr int N = P / 2;
-    for (int f = 0; f < 3; f++) {
-        cplx lap[N];
-#pragma unroll
-        for (int k = 0; k < N; k++) {
-            if (k < A.K) {
-                size_t o = (size_t)q + cs * k;
-                cplx a = A.d2x[f][o], b = A.d2y[f][o], u = us[f][o];
-                double kk = A.k2b2[k];
-                lap[k] = make_double2(a.x + b.x + kk * u.x, a.y + b.y + kk * u.y);
-            } else {
-                lap[k] = make_double2(0.0, 0.0);
+    const double cte = A.Cs * A.Cs * A.delta_les * A.delta_les * damp;
+    double re[M], im[M];
+    double* S = strain + tid;   // value v at v * 128
+    // s_xx, s_yy, s_zz and twice s_xy, s_xz, s_yz: fields a (of 3: its z-derivative) + b
+    for (int t = 0; t < 6; t++) {
+        const cplx* a = (t == 0 ? A.dudx : t == 1 ? A.dvdy : t == 2 ? A.uz : t == 3 ? A.dudy : t == 4 ? A.ux : A.uy) + q;
+        const cplx* b = t < 3 ? nullptr : (t == 3 ? A.dvdx : t == 4 ? A.dwdx : A.dwdy) + q;
+        const bool dz = t == 2 || t > 3;
+        col_phys2<P>([&](int k) {
+            if (k >= A.K) return make_double2(0.0, 0.0);
+            cplx v = a[(size_t)k * cs];
+            if (dz) {   // -i (k-1) beta u  (main_par.f:1888)
+                const double kb = -(double)k * A.beta;
+                v = make_double2(-kb * v.y, kb * v.x);
             }
-        }
-        to_phys<P>(lap, 1, A.K < N ? A.K : N, t1);
+            if (b) { const cplx w = b[(size_t)k * cs]; v.x += w.x; v.y += w.y; }
+            return v;
+        }, p, re, im);
+        const double f = t < 3 ? 1.0 : 0.5;
 #pragma unroll
-        for (int z = 0; z < P; z++) t1[z] = dg[z] * t1[z];
-        to_four<P>(t1, A.K, outs[f] + q, cs);
+        for (int m = 0; m < M; m++) {
+            const double u = f * re[m], w = f * im[m];
+            S[(2 * m) * 128] = t ? fma(u, re[m], S[(2 * m) * 128]) : u * re[m];
+            S[(2 * m + 1) * 128] = t ? fma(w, im[m], S[(2 * m + 1) * 128]) : w * im[m];
+        }
+    }
+    // nu_t = cte sqrt(2 S); S is four times the sum of squares here, and the
+    // factors 2 of the Laplacian and 1 / P of the transform back are taken along
+    for (int v = 0; v < 2 * M; v++) S[v * 128] = (cte * (0.5 / (double)P)) * sqrt(0.5 * S[v * 128]);
+    for (int f = 0; f < 3; f++) {
+        const cplx* d2x = A.d2x[f] + q;
+        const cplx* d2y = A.d2y[f] + q;
+        const cplx* us = (f == 0 ? A.ux : f == 1 ? A.uy : A.uz) + q;
+        cplx* out = (f == 0 ? A.fx : f == 1 ? A.fy : A.fz) + q;
+        col_phys2<P>([&](int k) {
+            if (k >= A.K) return make_double2(0.0, 0.0);
+            const size_t o = (size_t)k * cs;
+            const cplx a = d2x[o], b = d2y[o], u = us[o];
+            const double kk = A.k2b2[k];
+            return make_double2(fma(kk, u.x, a.x + b.x), fma(kk, u.y, a.y + b.y));
+        }, p, re, im);
+#pragma unroll
+        for (int m = 0; m < M; m++) { re[m] *= S[(2 * m) * 128]; im[m] *= S[(2 * m + 1) * 128]; }
+        col_four<P>(re, im, p, [&](int k, cplx v) { if (in && k < A.K) out[(size_t)k * cs] = v; });
     }
 }
 
@@ -654,27 +802,57 @@ struct IbmArgs {
     int n2, K, accumulate;
     double irf;
 };
+// The roughness touches few grid lines: a warp whose lines have delta = 0
+// everywhere and finite velocities (which a NaN would have to reach) writes
+// the zero force, or leaves what it would be added to, after one pass over
+// delta and u: 0.36 ms at 1025 x 193 x 64, 6.3 ms with every line transformed.
 template <int P>
 __global__ void __launch_bounds__(128) k_cvirt(IbmArgs A) {
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= A.n2) return;
-    size_t cs = A.n2;
-    const cplx* us[3] = {A.ux, A.uy, A.uz};
-    cplx* outs[3] = {A.fx, A.fy, A.fz};
-    double p[P];
-    constexpr int N = P / 2;
-    for (int f = 0; f < 3; f++) {
-        to_phys<P>(us[f] + q, cs, A.K, p);
-#pragma unroll
-        for (int z = 0; z < P; z++) p[z] = A.irf * A.delta[(size_t)q + cs * z] * p[z];
-        cplx tmp[N];
-        to_four<P>(p, A.K, tmp, 1);
-        for (int k = 0; k < A.K && k < N; k++) {
-            size_t o = (size_t)q + cs * k;
-            cplx v = make_double2(A.gibbs[k] * tmp[k].x, A.gibbs[k] * tmp[k].y);
-            if (A.accumulate) { cplx w = outs[f][o]; v.x += w.x; v.y += w.y; }
-            outs[f][o] = v;
+    using CP = Col<P>;
+    constexpr int M = CP::M;
+    const int tid = threadIdx.x, p = CP::TP == 2 ? (tid >> 4) & 1 : 0;
+    const int col = blockIdx.x * CP::PER_BLOCK + (CP::TP == 2 ? (tid >> 5) * 16 + (tid & 15) : tid);
+    const bool in = col < A.n2;
+    const int q = in ? col : A.n2 - 1;
+    const size_t cs = A.n2;
+    const cplx* us[3] = {A.ux + q, A.uy + q, A.uz + q};
+    cplx* outs[3] = {A.fx + q, A.fy + q, A.fz + q};
+    const double* delta = A.delta + q;
+    auto finite = [](double v) { return ((unsigned)__double2hiint(v) & 0x7ff00000u) != 0x7ff00000u; };
+    bool work = !finite(A.irf);
+#pragma unroll 8
+    for (int z = p; z < P; z += CP::TP) work |= delta[cs * z] != 0.0;
+    if (!__any_sync(0xffffffffu, work)) {
+        for (int f = 0; f < 3; f++)
+#pragma unroll 8
+            for (int k = p; k < A.K; k += CP::TP) {
+                const cplx v = us[f][cs * k];
+                work |= !finite(v.x) || !finite(v.y);
+            }
+        if (!__any_sync(0xffffffffu, work)) {
+            if (!A.accumulate && in)
+                for (int f = 0; f < 3; f++)
+                    for (int k = p; k < A.K && k < P / 2; k += CP::TP) outs[f][cs * k] = make_double2(0.0, 0.0);
+            return;
         }
+    }
+    double re[M], im[M];
+    const double sc = A.irf * (0.5 / (double)P);
+    for (int f = 0; f < 3; f++) {
+        col_phys2<P>(Modes{us[f], cs, A.K}, p, re, im);
+#pragma unroll
+        for (int m = 0; m < M; m++) {
+            const size_t z = 2 * (size_t)(m * CP::TP + p);
+            re[m] = sc * delta[cs * z] * re[m];
+            im[m] = sc * delta[cs * (z + 1)] * im[m];
+        }
+        col_four<P>(re, im, p, [&](int k, cplx v) {
+            if (!in || k >= A.K) return;
+            v.x *= A.gibbs[k]; v.y *= A.gibbs[k];
+            cplx* o = outs[f] + cs * k;
+            if (A.accumulate) { const cplx w = *o; v.x += w.x; v.y += w.y; }
+            *o = v;
+        });
     }
 }
 
@@ -688,15 +866,11 @@ __global__ void k_delta_filter(double* delta, const double* gibbs, int n2, int K
     double p[P];
     cplx tmp[N];
 #pragma unroll
-    for (int z = 0; z < P; z++) p[z] = delta[(size_t)q + (size_t)n2 * z];
-    to_four<P>(p, K, tmp, 1);
-    for (int k = 0; k < N; k++) {
-        if (k < K) tmp[k] = make_double2(gibbs[k] * tmp[k].x, gibbs[k] * tmp[k].y);
-        else tmp[k] = make_double2(0.0, 0.0);
-    }
-    to_phys<P>(tmp, 1, K < N ? K : N, p);
+    for (int z = 0; z < P; z++) p[z] = delta[(size_t)q + (size_t)n2 * z] * (1.0 / (double)P);
+    to_four<P>(p, [&](int k, cplx v) { tmp[k] = k < K ? make_double2(gibbs[k] * v.x, gibbs[k] * v.y) : make_double2(0.0, 0.0); });
+    to_phys2<P>([&](int k) { return tmp[k]; }, p);
 #pragma unroll
-    for (int z = 0; z < P; z++) delta[(size_t)q + (size_t)n2 * z] = p[z];
+    for (int z = 0; z < P; z++) delta[(size_t)q + (size_t)n2 * z] = 0.5 * p[z];
 }
 
 bool g_tw_ready[64] = {false};
@@ -704,7 +878,7 @@ bool g_tw_ready[64] = {false};
 int ensure_twiddles(tb_ctx* c) {
     int dev = c->device;
     if (dev >= 0 && dev < 64 && g_tw_ready[dev]) return TB_OK;
-    double hr[TW_N], hi[TW_N];
+    double hr[TW_N], hi[TW_N], lm[TW_N / 2], lr[TW_N / 2];
     for (int t = 0; t < TW_N; t++) {
         long double ang = -2.0L * 3.141592653589793238462643383279502884L * (long double)t / (long double)TW_N;
         hr[t] = (double)cosl(ang);
@@ -712,6 +886,15 @@ int ensure_twiddles(tb_ctx* c) {
     }
     TB_CUDA(cudaMemcpyToSymbol(c_twr, hr, sizeof hr));
     TB_CUDA(cudaMemcpyToSymbol(c_twi, hi, sizeof hi));
+    for (int t = 0; t < TW_N / 2; t++) {
+        const long double ang = -2.0L * 3.141592653589793238462643383279502884L * (long double)t / (long double)TW_N;
+        const long double wr = cosl(ang), wi = sinl(ang);
+        const bool big = lf_big(t);
+        lm[t] = (double)(big ? wr : wi);
+        lr[t] = (double)(big ? wi / wr : wr / wi);
+    }
+    TB_CUDA(cudaMemcpyToSymbol(c_lfm, lm, sizeof lm));
+    TB_CUDA(cudaMemcpyToSymbol(c_lfr, lr, sizeof lr));
     float fr[TW_N], fi[TW_N];
     for (int t = 0; t < TW_N; t++) { fr[t] = (float)hr[t]; fi[t] = (float)hi[t]; }
     TB_CUDA(cudaMemcpyToSymbol(c_twrf, fr, sizeof fr));
@@ -720,15 +903,15 @@ int ensure_twiddles(tb_ctx* c) {
     return TB_OK;
 }
 
-#define TB_DISPATCH_P(P, STMT)                                           \
+#define TB_DISPATCH_P(P, ...)                                            \
     switch (P) {                                                         \
-        case 2: { constexpr int PP = 2; STMT; } break;                   \
-        case 4: { constexpr int PP = 4; STMT; } break;                   \
-        case 8: { constexpr int PP = 8; STMT; } break;                   \
-        case 16: { constexpr int PP = 16; STMT; } break;                 \
-        case 32: { constexpr int PP = 32; STMT; } break;                 \
-        case 64: { constexpr int PP = 64; STMT; } break;                 \
-        case 128: { constexpr int PP = 128; STMT; } break;               \
+        case 2: { constexpr int PP = 2; __VA_ARGS__; } break;                   \
+        case 4: { constexpr int PP = 4; __VA_ARGS__; } break;                   \
+        case 8: { constexpr int PP = 8; __VA_ARGS__; } break;                   \
+        case 16: { constexpr int PP = 16; __VA_ARGS__; } break;                 \
+        case 32: { constexpr int PP = 32; __VA_ARGS__; } break;                 \
+        case 64: { constexpr int PP = 64; __VA_ARGS__; } break;                 \
+        case 128: { constexpr int PP = 128; __VA_ARGS__; } break;               \
         default: tb_set_error("kphys %d not supported", P); return TB_ERR_ARG; \
     }
 
@@ -985,8 +1168,8 @@ int tb_launch_les(tb_ctx* c, cplx* fx, cplx* fy, cplx* fz) {
     A.beta = c->cfg.beta; A.Re = c->cfg.Re; A.fac_y = c->cfg.fac_y; A.dy = c->cfg.dy; A.stf = c->cfg.stf;
     A.Cs = c->cfg.C_s; A.Aplus = c->cfg.A_plus;
     A.delta_les = std::pow(c->cfg.dx * c->cfg.dy * c->dz, 1.0 / 3.0);
-    unsigned nb = tb_blocks(A.n2, 128);
-    TB_DISPATCH_P(c->g.P, (k_les<PP><<<nb, 128, 0, c->stream>>>(A)));
+    TB_DISPATCH_P(c->g.P, TB_CUDA(cudaFuncSetAttribute(k_les<PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Col<PP>::VAL * 128 * 8));
+                          (k_les<PP><<<tb_blocks(A.n2, Col<PP>::PER_BLOCK), 128, Col<PP>::VAL * 128 * 8, c->stream>>>(A)));
     TB_CHECK_LAUNCH(c);
     return TB_OK;
 }
@@ -996,8 +1179,7 @@ int tb_launch_cvirt(tb_ctx* c, cplx* fx, cplx* fy, cplx* fz, bool accumulate) {
     if (r) return r;
     IbmArgs A{c->ux, c->uy, c->uz, c->delta_no, c->gibbs, fx, fy, fz, (int)tb_n2(c), c->g.K, accumulate ? 1 : 0,
               c->cfg.irf};
-    unsigned nb = tb_blocks(A.n2, 128);
-    TB_DISPATCH_P(c->g.P, (k_cvirt<PP><<<nb, 128, 0, c->stream>>>(A)));
+    TB_DISPATCH_P(c->g.P, (k_cvirt<PP><<<tb_blocks(A.n2, Col<PP>::PER_BLOCK), 128, 0, c->stream>>>(A)));
     TB_CHECK_LAUNCH(c);
     return TB_OK;
 }
