@@ -493,12 +493,12 @@ __device__ __forceinline__ void split_bf16(float x, unsigned short* p) {
     }
 }
 
-// Row `row` of the A operand (P values) into its BF16 parts.
+// Values 8 g0 .. 8 g0 + P/2 - 1 of row `row` of the A operand into its BF16 parts.
 template <int P>
-__device__ __forceinline__ void stage_row(unsigned char* sm, int row, const float* v) {
+__device__ __forceinline__ void stage_row(unsigned char* sm, int row, int g0, const float* v) {
     using Lt = TcLayout<P>;
 #pragma unroll
-    for (int g = 0; g < P / 8; g++) {
+    for (int g = 0; g < P / 16; g++) {
         unsigned short h[TC_PARTS][8];
 #pragma unroll
         for (int e = 0; e < 8; e++) {
@@ -512,7 +512,7 @@ __device__ __forceinline__ void stage_row(unsigned char* sm, int row, const floa
             uint4 H;
             H.x = h[q][0] | ((uint32_t)h[q][1] << 16); H.y = h[q][2] | ((uint32_t)h[q][3] << 16);
             H.z = h[q][4] | ((uint32_t)h[q][5] << 16); H.w = h[q][6] | ((uint32_t)h[q][7] << 16);
-            *reinterpret_cast<uint4*>(sm + Lt::A0 + q * Lt::AB + g * 2048 + row * 16) = H;
+            *reinterpret_cast<uint4*>(sm + Lt::A0 + q * Lt::AB + (g0 + g) * 2048 + row * 16) = H;
         }
     }
 }
@@ -607,14 +607,38 @@ __device__ __forceinline__ const cplx* nl_field(const NlArgs& A, int f) {
     return (f == 0) ? A.ux : (f == 1) ? A.uy : (f == 2) ? A.uz : (f == 3) ? A.wx : (f == 4) ? A.wy : A.wz;
 }
 
+// Both passes take a tile of 128 points with two threads a point, one for the
+// lower and one for the upper half of its slots or physical points: what they wait
+// for is their loads, and shared memory holds few tiles per SM (one at P = 128).
+// One thread a point took 4.3 ms (P = 128) and 1.01 ms (P = 64) for both passes at
+// 1025 x 193 points; two take 2.57 and 0.81.
+constexpr int TC_THREADS = 256;
+
+// Columns of this thread's half of its point's row of tensor memory, with 8 of them (P =
+// 16) out of the 16 that one load gives.
+template <int P>
+__device__ __forceinline__ void tmem_half(uint32_t tmem, int warp, int half, float* v) {
+    constexpr int H = P / 2;
+    const uint32_t lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    if constexpr (H < 16) {
+        float w[16];
+        tbtc::tmem_ld16(lane, w);
+#pragma unroll
+        for (int i = 0; i < H; i++) v[i] = half ? w[H + i] : w[i];
+    } else {
+#pragma unroll
+        for (int c = 0; c < H; c += 16) tbtc::tmem_ld16(lane + half * H + c, v + c);
+    }
+}
+
 // Pass 1 on the tensor cores: tile = (field f, 128 points) -> ph[(f P + z) n2 + q].
 template <int P>
-__global__ void __launch_bounds__(128) k_nl_phys_tc(NlArgs A, float* __restrict__ ph, const uint16_t* __restrict__ mats,
-                                                    int* err, TcCtl ctl) {
-    constexpr int N = P / 2;
+__global__ void __launch_bounds__(TC_THREADS) k_nl_phys_tc(NlArgs A, float* __restrict__ ph, const uint16_t* __restrict__ mats,
+                                                           int* err, TcCtl ctl) {
+    constexpr int H = P / 2;
     extern __shared__ __align__(1024) unsigned char sm[];
     const uint32_t tmem = tc_setup<P>(sm, mats);
-    const int t = threadIdx.x, warp = t >> 5;
+    const int t = threadIdx.x & 127, half = threadIdx.x >> 7, warp = threadIdx.x >> 5;
     const size_t n2 = A.n2;
     const int tpf = (int)((n2 + 127) / 128), ntiles = 6 * tpf;
     uint32_t phase = 0;
@@ -622,27 +646,23 @@ __global__ void __launch_bounds__(128) k_nl_phys_tc(NlArgs A, float* __restrict_
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int f = tile / tpf;
         const size_t q = (size_t)(tile % tpf) * 128 + t;
-        const cplx* F = nl_field(A, f);
-        float v[P];
-        v[0] = 0.f;
-        v[1] = q < n2 ? (float)F[q].y : 0.f;
+        const cplx* F = nl_field(A, f) + q;
+        float v[H];
 #pragma unroll
-        for (int k = 1; k < N; k++) {
+        for (int i = 0; i < H / 2; i++) {
+            const int k = half * (H / 2) + i;
             cplx c = make_double2(0.0, 0.0);
-            if (k < A.K && q < n2) c = F[(size_t)k * n2 + q];
-            v[2 * k] = (float)c.x;
-            v[2 * k + 1] = (float)c.y;
+            if (k < A.K && q < n2) c = F[(size_t)k * n2];
+            v[2 * i] = k ? (float)c.x : 0.f;
+            v[2 * i + 1] = (float)c.y;
         }
-        stage_row<P>(sm, t, v);
+        stage_row<P>(sm, t, half * (H / 8), v);
         if (!(ok = tc_run<P>(sm, tmem, phase, ctl))) break;
+        tmem_half<P>(tmem, warp, half, v);
+        if (q < n2) {
+            float* o = ph + ((size_t)f * P + half * H) * n2 + q;
 #pragma unroll
-        for (int c0 = 0; c0 < P; c0 += 16) {
-            float w[16];
-            tbtc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + c0, w);
-            if (q < n2) {
-#pragma unroll
-                for (int i = 0; i < 16; i++) ph[((size_t)f * P + c0 + i) * n2 + q] = w[i];
-            }
+            for (int i = 0; i < H; i++) o[(size_t)i * n2] = v[i];
         }
         tbtc::fence_before_sync();
         __syncthreads();
@@ -653,12 +673,12 @@ __global__ void __launch_bounds__(128) k_nl_phys_tc(NlArgs A, float* __restrict_
 // Pass 2 on the tensor cores: tile = (output o, 128 points); the quadratic
 // disturbance term's slots plus the FP64 mean terms, as k_nl_four.
 template <int P>
-__global__ void __launch_bounds__(128) k_nl_four_tc(NlArgs A, const float* __restrict__ ph,
-                                                    const uint16_t* __restrict__ mats, int* err, TcCtl ctl) {
-    constexpr int N = P / 2;
+__global__ void __launch_bounds__(TC_THREADS) k_nl_four_tc(NlArgs A, const float* __restrict__ ph,
+                                                           const uint16_t* __restrict__ mats, int* err, TcCtl ctl) {
+    constexpr int H = P / 2;
     extern __shared__ __align__(1024) unsigned char sm[];
     const uint32_t tmem = tc_setup<P>(sm, mats);
-    const int t = threadIdx.x, warp = t >> 5;
+    const int t = threadIdx.x & 127, half = threadIdx.x >> 7, warp = threadIdx.x >> 5;
     const size_t n2 = A.n2;
     const int tpf = (int)((n2 + 127) / 128), ntiles = 3 * tpf;
     uint32_t phase = 0;
@@ -668,34 +688,35 @@ __global__ void __launch_bounds__(128) k_nl_four_tc(NlArgs A, const float* __res
         const size_t q = (size_t)(tile % tpf) * 128 + t;
         const int p1 = (o == 0) ? 1 : (o == 1) ? 0 : 2, q1 = (o == 0) ? 3 : (o == 1) ? 5 : 4;
         const int p2 = (o == 0) ? 0 : (o == 1) ? 2 : 1, q2 = (o == 0) ? 4 : (o == 1) ? 3 : 5;
-        float v[P];
+        float v[H];
 #pragma unroll
-        for (int z = 0; z < P; z++) v[z] = 0.f;
+        for (int i = 0; i < H; i++) v[i] = 0.f;
         if (q < n2) {
-            const float *a1 = ph + (size_t)p1 * P * n2 + q, *b1 = ph + (size_t)q1 * P * n2 + q;
-            const float *a2 = ph + (size_t)p2 * P * n2 + q, *b2 = ph + (size_t)q2 * P * n2 + q;
+            const size_t z0 = (size_t)half * H * n2 + q;
+            const float *a1 = ph + (size_t)p1 * P * n2 + z0, *b1 = ph + (size_t)q1 * P * n2 + z0;
+            const float *a2 = ph + (size_t)p2 * P * n2 + z0, *b2 = ph + (size_t)q2 * P * n2 + z0;
 #pragma unroll
-            for (int z = 0; z < P; z++) {
-                const size_t zz = (size_t)z * n2;
-                v[z] = a1[zz] * b1[zz] - a2[zz] * b2[zz];
+            for (int i = 0; i < H; i++) {
+                const size_t zz = (size_t)i * n2;
+                v[i] = a1[zz] * b1[zz] - a2[zz] * b2[zz];
             }
         }
-        stage_row<P>(sm, t, v);
+        stage_row<P>(sm, t, half * (H / 8), v);
         if (!(ok = tc_run<P>(sm, tmem, phase, ctl))) break;
-#pragma unroll
-        for (int c0 = 0; c0 < P; c0 += 16) tbtc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + c0, v + c0);
+        tmem_half<P>(tmem, warp, half, v);
         if (q < n2) {
             const cplx *P1 = nl_field(A, p1) + q, *Q1 = nl_field(A, q1) + q, *P2 = nl_field(A, p2) + q, *Q2 = nl_field(A, q2) + q;
             const double m1 = P1[0].x, n1 = Q1[0].x, m2 = P2[0].x, n2v = Q2[0].x;
             cplx* out = ((o == 0) ? A.a : (o == 1) ? A.b : A.c) + q;
-            out[0] = make_double2(zap(m1 * n1 - m2 * n2v + (double)v[0]), 0.0);
+            if (half == 0) out[0] = make_double2(zap(m1 * n1 - m2 * n2v + (double)v[0]), 0.0);
 #pragma unroll
-            for (int k = 1; k < N; k++) {
-                if (k >= A.K) continue;
+            for (int i = 0; i < H / 2; i++) {
+                const int k = half * (H / 2) + i;
+                if (k == 0 || k >= A.K) continue;
                 const size_t kk = (size_t)k * n2;
                 const cplx aq1 = Q1[kk], ap1 = P1[kk], aq2 = Q2[kk], ap2 = P2[kk];
-                const double vr = m1 * aq1.x + n1 * ap1.x - m2 * aq2.x - n2v * ap2.x + (double)v[2 * k];
-                const double vi = m1 * aq1.y + n1 * ap1.y - m2 * aq2.y - n2v * ap2.y + (double)v[2 * k + 1];
+                const double vr = m1 * aq1.x + n1 * ap1.x - m2 * aq2.x - n2v * ap2.x + (double)v[2 * i];
+                const double vi = m1 * aq1.y + n1 * ap1.y - m2 * aq2.y - n2v * ap2.y + (double)v[2 * i + 1];
                 out[kk] = make_double2(zap(vr), zap(vi));
             }
         }
@@ -1121,9 +1142,9 @@ int tb_launch_nlterms(tb_ctx* c, cplx* a, cplx* b, cplx* cc) {
         const int per = (c->tune_nl >= 1 && c->tune_nl <= TcLayout<PP>::PER_SM) ? c->tune_nl : TcLayout<PP>::PER_SM; \
         const size_t cap = (size_t)per * sms;                                                                  \
         const unsigned g1 = (unsigned)std::min<size_t>(6 * tiles, cap), g2 = (unsigned)std::min<size_t>(3 * tiles, cap); \
-        k_nl_phys_tc<PP><<<g1, 128, TcLayout<PP>::BYTES, c->stream>>>(A, c->nl_phys, c->dft_tc, c->tc_err, ctl);   \
+        k_nl_phys_tc<PP><<<g1, TC_THREADS, TcLayout<PP>::BYTES, c->stream>>>(A, c->nl_phys, c->dft_tc, c->tc_err, ctl);   \
         TB_CHECK_LAUNCH(c);                                                                                    \
-        k_nl_four_tc<PP><<<g2, 128, TcLayout<PP>::BYTES, c->stream>>>(A, c->nl_phys, c->dft_tc + TC_PARTS * PP * PP, \
+        k_nl_four_tc<PP><<<g2, TC_THREADS, TcLayout<PP>::BYTES, c->stream>>>(A, c->nl_phys, c->dft_tc + TC_PARTS * PP * PP, \
                                                                       c->tc_err, ctl);                         \
         break;                                                                                                 \
     }
