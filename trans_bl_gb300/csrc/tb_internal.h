@@ -225,7 +225,15 @@ int tb_plain_setup(tb_ctx* c);
 int tb_plain_tune(tb_ctx* c, int l, int itera, const int* gis, int ngis, int* best, float* best_ms);
 int tb_poisson_setup(tb_ctx* c);
 int tb_poisson_begin(tb_ctx* c, const cplx* dwzdx);
-int tb_poisson_defect_f32(tb_ctx* c, const double* rows, float2* r32, size_t elems32, int T, int np, unsigned long long* maxsq);
+// Device tables of the mixed form's FP64 defect.  Row j of rows (ny, DEFECT_ROW):
+// weights of the x-stencil sums of rows j-1 .. j+1 over -12 dx^2 fac_y, of the
+// values of rows j-2 .. j+2 in the y-derivative, -1/dy^2.  modes (K, 2): the k^2
+// term in units of the x-stencil sums, the top row's boundary term.
+constexpr int DEFECT_ROW = 9;
+struct DefectRows {
+    const double *rows, *modes;
+};
+int tb_poisson_defect_f32(tb_ctx* c, const DefectRows& D, float2* r32, size_t elems32, int T, int np, unsigned long long* maxsq);
 int tb_poisson_end(tb_ctx* c);
 int tb_poi_uy_mixed(tb_ctx* c, const cplx* dwzdx, double erro);
 // Learned first correction of the mixed solve (tb_learn.cu owns the network

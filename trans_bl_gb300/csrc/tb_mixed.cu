@@ -56,7 +56,7 @@ constexpr int DIRECT_MAX = 400;      // unknowns per mode below which coarsening
 struct Mixed {
     float2 *ea = nullptr, *eb = nullptr, *r = nullptr;   // per mode blocks of `elems` (layout: tb_cycle.cuh)
     float4* tab = nullptr;    // per mode: line-solve and residual rows of every level (mg::Cycle::tab)
-    double* drow = nullptr;   // (K, ny, 8) rows of the FP64 defect: -w1[-1..1], -w2[-2..2] (residual_row)
+    double* drow = nullptr;   // rows and modes of the FP64 defect (DefectRows)
     float* coef = nullptr;    // sp(7) cp(8) pp(4) lp(5) per reference level
     float* qdy2 = nullptr;    // (ny, msh)
     float* ainv = nullptr;    // (K, N, N) inverse of the coarsest operator per mode
@@ -539,7 +539,7 @@ int apply(tb_ctx* c, const FineDev& M) {
 
 int defect(tb_ctx* c) {
     Mixed* m = get(c);
-    return tb_poisson_defect_f32(c, m->drow, m->r, m->elems, m->cyc.lv[0].T, m->cyc.lv[0].np, m->maxsq);
+    return tb_poisson_defect_f32(c, DefectRows{m->drow, m->drow + (size_t)DEFECT_ROW * c->g.ny}, m->r, m->elems, m->cyc.lv[0].T, m->cyc.lv[0].np, m->maxsq);
 }
 
 template <int S>
@@ -666,37 +666,50 @@ void line_tables(int n, int S, double unit, double qx, const double* cf, const d
     }
 }
 
-// The operator's row j (1 <= j < n) of one level and mode as weights of the
-// x-stencil sums of rows j-1 .. j+1 (w[0..2]) and of the values of rows
-// j-2 .. j+2 (w[3..7]), the centre stencil's diagonal (-30) folded into the
-// latter: L u = sum_q w1[q] X(j+q) + sum_q w2[q] u(j+q).
+// The operator's row j (1 <= j < n) of one level: weights w1 of the x-stencil sums
+// (and of the k^2 term) of rows j-1 .. j+1, w2 of the values of rows j-2 .. j+2
+// in the y-derivative, whose factor q2 is returned (defect, poisson_par.f:543-793).
+double operator_row(int j, int n, const double* cf, const double* Q2, double* w1, double* w2) {
+    const double *SP = cf, *CP = cf + 7, *PP = cf + 15, *LP = cf + 19;
+    std::fill(w1, w1 + 3, 0.0);
+    std::fill(w2, w2 + 5, 0.0);
+    if (j == 1) {
+        w1[1] = SP[1]; w1[2] = SP[2];
+        for (int q = 0; q < 4; q++) w2[1 + q] = SP[3 + q];
+        return Q2[0];
+    }
+    if (j <= n - 3) {
+        for (int q = 0; q < 3; q++) w1[q] = CP[q];
+        for (int q = 0; q < 5; q++) w2[q] = CP[3 + q];
+        return Q2[j - 2];
+    }
+    w1[1] = 1.0;
+    if (j == n - 2) {
+        w2[3] = PP[3]; w2[2] = PP[2]; w2[1] = PP[1];
+        return Q2[j - 1];
+    }
+    w2[2] = LP[2]; w2[1] = LP[3]; w2[0] = LP[4];
+    return Q2[j - 2];
+}
+// The boundary term of the top row: its multiple of the value there is subtracted.
+double top_term(int n, double ify, double k2b2, double alpha2, const double* cf, const double* Q2) {
+    return cf[20] * std::sqrt((alpha2 - k2b2) * ify) * std::sqrt(Q2[n - 3]);
+}
+
+// The row as weights of the x-stencil sums of rows j-1 .. j+1 (w[0..2]) and of
+// the values of rows j-2 .. j+2 (w[3..7]), the centre stencil's diagonal (-30)
+// folded into the latter: L u = sum_q w1[q] X(j+q) + sum_q w2[q] u(j+q).
 void residual_row(int j, int n, double den, double ify, double k2b2, double alpha2, const double* cf, const double* Q2,
                   double* w) {
-    const double *SP = cf, *CP = cf + 7, *PP = cf + 15, *LP = cf + 19;
     double *w1 = w, *w2 = w + 3;
-    std::fill(w, w + 8, 0.0);
-    const double kk = k2b2 * ify;
-    if (j == 1) {
-        const double q2 = Q2[0];
-        w1[1] = den * SP[1]; w1[2] = den * SP[2];
-        for (int q = 0; q < 4; q++) w2[1 + q] = q2 * SP[3 + q];
-        w2[2] += kk * SP[1]; w2[3] += kk * SP[2];
-    } else if (j <= n - 3) {
-        const double q2 = Q2[j - 2];
-        for (int q = 0; q < 3; q++) w1[q] = den * CP[q];
-        for (int q = 0; q < 5; q++) w2[q] = q2 * CP[3 + q];
-        for (int q = 0; q < 3; q++) w2[1 + q] += kk * CP[q];
-    } else if (j == n - 2) {
-        const double q2 = Q2[j - 1];
-        w1[1] = den;
-        w2[3] = q2 * PP[3]; w2[2] = q2 * PP[2] + kk; w2[1] = q2 * PP[1];
-    } else {
-        const double q2 = Q2[j - 2];
-        w1[1] = den;
-        w2[2] = q2 * LP[2] + kk - LP[1] * std::sqrt((alpha2 - k2b2) * ify) * std::sqrt(q2);
-        w2[1] = q2 * LP[3]; w2[0] = q2 * LP[4];
+    const double q2 = operator_row(j, n, cf, Q2, w1, w2), kk = k2b2 * ify;
+    for (int q = 0; q < 5; q++) w2[q] *= q2;
+    for (int q = 0; q < 3; q++) w2[1 + q] += kk * w1[q];
+    if (j == n - 1) w2[2] -= top_term(n, ify, k2b2, alpha2, cf, Q2);
+    for (int q = 0; q < 3; q++) {
+        w1[q] *= den;
+        w2[1 + q] -= 30.0 * w1[q];
     }
-    for (int q = 0; q < 3; q++) w2[1 + q] -= 30.0 * w1[q];
 }
 
 // FP32 residual rows of one level and mode, negated, the sums in units of 16.
@@ -826,14 +839,20 @@ int tb_mixed_setup(tb_ctx* c) {
         }
     if ((r = upl(&m->tab, t32))) return r;
     cy.tab = m->tab;
-    std::vector<double> drow((size_t)K * ny * 8, 0.0);
-    for (int k = 0; k < K; k++)
+    std::vector<double> drow((size_t)DEFECT_ROW * ny + 2 * K, 0.0);
+    {
+        const double den = 1.0 / (12.0 * c->h_dx2[0] * c->cfg.fac_y), ify = 1.0 / c->cfg.fac_y;
         for (int j = 1; j < ny; j++) {
-            double* w = &drow[((size_t)k * ny + j) * 8];
-            residual_row(j, ny, 1.0 / (12.0 * c->h_dx2[0] * c->cfg.fac_y), 1.0 / c->cfg.fac_y, c->h_k2b2[k],
-                         c->cfg.alpha * c->cfg.alpha, &cf64[0], &c->h_qdy2[0], w);
-            for (int q = 0; q < 8; q++) w[q] = -w[q];
+            double* w = &drow[(size_t)DEFECT_ROW * j];
+            w[8] = -operator_row(j, ny, &cf64[0], &c->h_qdy2[0], w, w + 3);
+            for (int q = 0; q < 3; q++) w[q] *= -den;
         }
+        for (int k = 0; k < K; k++) {
+            double* md = &drow[(size_t)DEFECT_ROW * ny + 2 * k];
+            md[0] = c->h_k2b2[k] * ify / den;
+            md[1] = top_term(ny, ify, c->h_k2b2[k], c->cfg.alpha * c->cfg.alpha, &cf64[0], &c->h_qdy2[0]);
+        }
+    }
     if ((r = upl(&m->drow, drow))) return r;
     std::vector<float> cf(cf64.begin(), cf64.end());
     if ((r = upl(&m->coef, cf))) return r;

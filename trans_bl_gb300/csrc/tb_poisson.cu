@@ -76,15 +76,20 @@ __global__ void k_source(PoiDev P, const cplx* wx, const cplx* dwzdx, const cplx
 // defect records +inf).
 //
 // An FP64 warp instruction holds its pipe for 64 cycles, so their number is
-// what the kernel costs.  L fc is the sum of three x-stencil sums and five
-// values with weights that depend on the row and the mode only (rows, set up
-// once: -w1[-1..1], -w2[-2..2] with every constant factor and the stencil's
-// diagonal folded in), and a thread marches down a column with both windows
-// in registers, so a stencil sum is formed once: 24 FP64 instructions a complex
-// point instead of 46 with the operator's terms formed one by one (all modes
-// active, 1025 x 193 x 64: 975 -> 530 us).  The maximum is compared as integer bit patterns.
-constexpr int DEF_ROWS = 24;   // rows per thread: two more stencil sums per chunk
-__global__ void __launch_bounds__(128) k_defect_f32(PoiDev P, const double* __restrict__ rows, float2* r32, size_t elems32, int T,
+// what the kernel costs.  A thread marches down a column with the values and
+// the x-stencil sums of its rows in registers, so a sum is formed once, and the k^2
+// term rides on the sums as one more centre term: 28 FP64 instructions a complex
+// point (46 with the operator's terms formed one by one).  This defect stops the
+// solve, so its rounding must stay that of those terms: the sums cancel
+// before they meet 1/(12 dx^2), the y-derivative before it meets 1/dy^2.  With all
+// constants and the diagonal folded into row weights it takes 24, but leaves 2.5 to
+// 5 times the error (rms against 80-bit sums, 65 to 257 rows); this order has that of the
+// terms one by one.
+// Rows per thread, with two more stencil sums a chunk: 16 and 24 rows leave small grids
+// idle (257 x 97 x 8: 37 and 52 us, 31 with 8 rows) and gain nothing on large ones
+// (1025 x 193 x 32: 425, 430 and 428 us).
+constexpr int DEF_ROWS = 8;
+__global__ void __launch_bounds__(128) k_defect_f32(PoiDev P, DefectRows D, float2* r32, size_t elems32, int T,
                                                     int np, unsigned long long* maxsq) {
     __shared__ unsigned long long wmax[4];
     const int k = blockIdx.z;
@@ -96,25 +101,28 @@ __global__ void __launch_bounds__(128) k_defect_f32(PoiDev P, const double* __re
     if (i <= nx - 2) {
         const cplx* F = P.fc + (size_t)k * P.elems + i;
         const cplx* SC = P.sc + (size_t)k * P.elems + i;
-        const double* W = rows + (size_t)k * ny * 8;
+        const double kd = D.modes[2 * k], top = D.modes[2 * k + 1];
         const int iq = i + 1;
         float2* out = r32 + (size_t)k * elems32 + ((size_t)(iq % 3) * np + 1) * T + iq / 3;   // row 0 of this line
         const bool border = i == 1 || i == nx - 2;
         const int e = (i == 1) ? 1 : -1;
         const cplx z = make_double2(0.0, 0.0);
         auto val = [&](int j) -> cplx { return (j >= 0 && j < ny) ? F[(size_t)nx * j] : z; };
-        // x-stencil sum of row j without its centre term -30 f; a border line
-        // (one-sided, centre term -15 f) adds the 15 f that the folded weight has too much
+        // x-stencil sum of row j (rhs_center, rhs_border; one-sided on a border line) and its k^2 term
         auto sum = [&](int j, cplx f) -> cplx {
             if (j < 1 || j >= ny) return z;   // weight 0
             const cplx* R = F + (size_t)nx * j;
+            cplx s;
             if (border) {
                 const cplx a = R[-e], b = R[e], c = R[2 * e], d = R[3 * e], g = R[4 * e];
-                return make_double2(fma(15.0, f.x, fma(10.0, a.x, fma(-4.0, b.x, fma(14.0, c.x, fma(-6.0, d.x, g.x))))),
-                                    fma(15.0, f.y, fma(10.0, a.y, fma(-4.0, b.y, fma(14.0, c.y, fma(-6.0, d.y, g.y))))));
+                s = make_double2(fma(-6.0, d.x, fma(14.0, c.x, fma(-4.0, b.x, fma(-15.0, f.x, 10.0 * a.x)))) + g.x,
+                                 fma(-6.0, d.y, fma(14.0, c.y, fma(-4.0, b.y, fma(-15.0, f.y, 10.0 * a.y)))) + g.y);
+            } else {
+                const cplx a = R[-2], b = R[-1], c = R[1], d = R[2];
+                s = make_double2(fma(16.0, c.x, fma(-30.0, f.x, fma(16.0, b.x, -a.x))) - d.x,
+                                 fma(16.0, c.y, fma(-30.0, f.y, fma(16.0, b.y, -a.y))) - d.y);
             }
-            const cplx a = R[-2], b = R[-1], c = R[1], d = R[2];
-            return make_double2(fma(16.0, b.x + c.x, -(a.x + d.x)), fma(16.0, b.y + c.y, -(a.y + d.y)));
+            return make_double2(fma(kd, f.x, s.x), fma(kd, f.y, s.y));
         };
         cplx f0 = val(j0 - 2), f1 = val(j0 - 1), f2 = val(j0), f3 = val(j0 + 1);
         cplx x0 = sum(j0 - 1, f1), x1 = sum(j0, f2);
@@ -122,14 +130,16 @@ __global__ void __launch_bounds__(128) k_defect_f32(PoiDev P, const double* __re
 #pragma unroll 2
         for (int j = j0; j < j1; j++) {
             const cplx f4 = val(j + 2), x2 = sum(j + 1, f3);
-            const double* w = W + 8 * j;
-            cplx v = SC[(size_t)nx * j];
-            const cplx t[8] = {x0, x1, x2, f0, f1, f2, f3, f4};
+            const double* w = D.rows + DEFECT_ROW * j;
+            const cplx t[5] = {f0, f1, f2, f3, f4}, X[3] = {x0, x1, x2};
+            cplx cc = make_double2(w[3] * f0.x, w[3] * f0.y);
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const double c = w[q];
-                v = make_double2(fma(c, t[q].x, v.x), fma(c, t[q].y, v.y));
-            }
+            for (int q = 1; q < 5; q++) cc = make_double2(fma(w[3 + q], t[q].x, cc.x), fma(w[3 + q], t[q].y, cc.y));
+            cplx v = SC[(size_t)nx * j];
+            v = make_double2(fma(w[8], cc.x, v.x), fma(w[8], cc.y, v.y));
+#pragma unroll
+            for (int q = 0; q < 3; q++) v = make_double2(fma(w[q], X[q].x, v.x), fma(w[q], X[q].y, v.y));
+            if (j == ny - 1) v = make_double2(fma(top, f2.x, v.x), fma(top, f2.y, v.y));
             const unsigned long long a = (unsigned long long)__double_as_longlong(fma(v.x, v.x, v.y * v.y));
             m = max(m, a > largest ? 0x7ff0000000000000ull : a);
             out[(size_t)j * T] = make_float2((float)v.x, (float)v.y);
@@ -213,12 +223,12 @@ int tb_poisson_end(tb_ctx* c) {
     return TB_OK;
 }
 
-int tb_poisson_defect_f32(tb_ctx* c, const double* rows, float2* r32, size_t elems32, int T, int np, unsigned long long* maxsq) {
+int tb_poisson_defect_f32(tb_ctx* c, const DefectRows& D, float2* r32, size_t elems32, int T, int np, unsigned long long* maxsq) {
     PoiDev P = make_dev(c);
     dim3 grid(tb_blocks(c->g.nx - 2, 128), tb_blocks(c->g.ny - 1, DEF_ROWS), c->g.K);
     cudaEvent_t ps = nullptr;
     if (tb_prof_begin(c, PROF_DEFECT, &ps)) return TB_ERR_CUDA;
-    k_defect_f32<<<grid, 128, 0, c->stream>>>(P, rows, r32, elems32, T, np, maxsq);
+    k_defect_f32<<<grid, 128, 0, c->stream>>>(P, D, r32, elems32, T, np, maxsq);
     TB_CHECK_LAUNCH(c);
     return tb_prof_end(c, PROF_DEFECT, ps);
 }
