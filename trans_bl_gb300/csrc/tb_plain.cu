@@ -50,19 +50,18 @@ __host__ __device__ inline int rows_per_lane(int n, int G) {
 //   per row s, from 8 s: weights WL WC WR of the x-stencil sums of rows j-1, j,
 //     j+1 in the right-hand side (negative), L1 L2, U1 U2 (times ID), ID
 //   WZ  -L times the fixed value of row 0, rows 1 and 2 (entries of rows s < 2)
-//   S > 2: per row the responses H1 H2 (forward) and K1 K2 (backward) to the
-//     states entering the chunk
+//   per row the responses H1 H2 (forward) and K1 K2 (backward) to the states
+//     entering the chunk
 //   PF, PB  5 x 4: Kogge-Stone matrices of the chunk propagators in a warp
-//   CF, CB  3 x (4; S = 1: 2): response of the chunk's rows (S <= 2) or of the state
-//     entering it (S > 2) to the state leaving warp w of those before (after) it
+//   CF, CB  3 x 4: response of the state entering the chunk to the state
+//     leaving warp w of those before (after) it
 __host__ __device__ constexpr int tab_wz(int S) { return 8 * S; }
 __host__ __device__ constexpr int tab_h(int S) { return 8 * S + (S < 2 ? 1 : 2); }
-__host__ __device__ constexpr int tab_pf(int S) { return tab_h(S) + (S > 2 ? 4 * S : 0); }
+__host__ __device__ constexpr int tab_pf(int S) { return tab_h(S) + 4 * S; }
 __host__ __device__ constexpr int tab_pb(int S) { return tab_pf(S) + 20; }
-__host__ __device__ constexpr int tab_cw(int S) { return S == 1 ? 2 : 4; }
 __host__ __device__ constexpr int tab_cf(int S) { return tab_pb(S) + 20; }
-__host__ __device__ constexpr int tab_cb(int S) { return tab_cf(S) + 3 * tab_cw(S); }
-__host__ __device__ constexpr int tab_entries(int S) { return tab_cb(S) + 3 * tab_cw(S); }
+__host__ __device__ constexpr int tab_cb(int S) { return tab_cf(S) + 12; }
+__host__ __device__ constexpr int tab_entries(int S) { return tab_cb(S) + 12; }
 __host__ __device__ inline int tab_size(int n, int G) { return tab_entries(rows_per_lane(n, G)) * 32 * G; }
 __host__ __device__ inline size_t tab_block(int ny) {
     const int a = tab_size(ny, 1), b = tab_size(ny, 2), c = tab_size(ny, 4), m = a > b ? a : b;
@@ -109,14 +108,19 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // rhs_border2 (poisson_par.f:343-540), banbk5_poi (penta_par.f:367-404) and
 // fc + rf (x - fc) for the rows j >= 1 (0-based), S rows a lane.  Each chunk
 // runs its local recurrences with zero carry, the chunk-end 2x2 propagators
-// are scanned within each warp (Kogge-Stone, `lv` levels), and the states
-// leaving the other warps enter through precomputed responses.  With one or
-// two rows a lane the scanned state is the rows themselves.  Row 0 keeps its
-// value f0, which enters rows 1 and 2.  Rows past the line have zero tables.
+// are scanned within each warp (Kogge-Stone, `lv` levels), the states leaving the
+// other warps enter through precomputed responses, and the rows follow from the
+// state that enters their chunk.  Row 0 keeps its value f0, which enters rows 1
+// and 2.  Rows past the line have zero tables.
+//
+// With one or two rows a lane the scanned states are the rows themselves, but a row
+// taken from there carries the rounding of every level: the defect that three sweeps
+// leave of a solved problem on 129 rows is 1.4 times that of sequential sweeps, 1.05 times
+// with the rows formed from the entering state.
 //
 // FP64 instructions a warp, four warps of one row a lane: 3 stencil, 3 weights,
-// 1 + 16 scan and up to 6 for the other warps in each direction, 1 scaling, 2
-// update: 55 of ~64 cycles.  The x-stencil lines come as pointers to the
+// twice 1 + 16 scan and 2 for the rows, 12 for the three other warps, 1 scaling, 2
+// update: 59 of ~64 cycles.  The x-stencil lines come as pointers to the
 // chunk's rows (stride NC = 32 G): for a centre line (i-2, i-1, i+1, i+2), for
 // a border line the four inner lines in order of distance and the outer line.
 template <int S>
@@ -178,27 +182,19 @@ __device__ __forceinline__ void line_solve(bool border, const double* T, int G, 
         if (lane == 31) { xf[2 * g] = b0; xf[2 * g + 1] = b1; }
         group_barrier(bar, 32 * G);
     }
-    constexpr int CW = tab_cw(S);
-    if (S > 2) {
-        b0 = __shfl_up_sync(0xffffffffu, b0, 1);
-        b1 = __shfl_up_sync(0xffffffffu, b1, 1);
-        if (lane == 0) { b0 = 0.0; b1 = 0.0; }
-    }
+    b0 = __shfl_up_sync(0xffffffffu, b0, 1);
+    b1 = __shfl_up_sync(0xffffffffu, b1, 1);
+    if (lane == 0) { b0 = 0.0; b1 = 0.0; }
 #pragma unroll
     for (int w = 0; w < 3; w++)
         if (w < g) {
             const double z0 = xf[2 * w], z1 = xf[2 * w + 1];
-            const int e = tab_cf(S) + CW * w;
+            const int e = tab_cf(S) + 4 * w;
             b0 = fma(tab(e), z0, fma(tab(e + 1), z1, b0));
-            if (S > 1) b1 = fma(tab(e + (S > 1 ? 2 : 0)), z0, fma(tab(e + (S > 1 ? 3 : 0)), z1, b1));
+            b1 = fma(tab(e + 2), z0, fma(tab(e + 3), z1, b1));
         }
-    if (S <= 2) {
-        y[S - 1] = b0;
-        if (S == 2) y[0] = b1;
-    } else {
 #pragma unroll
-        for (int s = 0; s < S; s++) y[s] = fma(tab(tab_h(S) + 4 * s), b0, fma(tab(tab_h(S) + 4 * s + 1), b1, y[s]));
-    }
+    for (int s = 0; s < S; s++) y[s] = fma(tab(tab_h(S) + 4 * s), b0, fma(tab(tab_h(S) + 4 * s + 1), b1, y[s]));
     // backward, likewise from the high lanes
 #pragma unroll
     for (int s = S - 1; s >= 0; s--) {
@@ -228,26 +224,19 @@ __device__ __forceinline__ void line_solve(bool border, const double* T, int G, 
         if (lane == 0) { xb[2 * g] = b0; xb[2 * g + 1] = b1; }
         group_barrier(bar, 32 * G);
     }
-    if (S > 2) {
-        b0 = __shfl_down_sync(0xffffffffu, b0, 1);
-        b1 = __shfl_down_sync(0xffffffffu, b1, 1);
-        if (lane == 31) { b0 = 0.0; b1 = 0.0; }
-    }
+    b0 = __shfl_down_sync(0xffffffffu, b0, 1);
+    b1 = __shfl_down_sync(0xffffffffu, b1, 1);
+    if (lane == 31) { b0 = 0.0; b1 = 0.0; }
 #pragma unroll
     for (int w = 0; w < 3; w++)
         if (g + 1 + w < G) {   // the warps after this one
             const double z0 = xb[2 * (g + 1 + w)], z1 = xb[2 * (g + 1 + w) + 1];
-            const int e = tab_cb(S) + CW * w;
+            const int e = tab_cb(S) + 4 * w;
             b0 = fma(tab(e), z0, fma(tab(e + 1), z1, b0));
-            if (S > 1) b1 = fma(tab(e + (S > 1 ? 2 : 0)), z0, fma(tab(e + (S > 1 ? 3 : 0)), z1, b1));
+            b1 = fma(tab(e + 2), z0, fma(tab(e + 3), z1, b1));
         }
-    if (S <= 2) {
-        y[0] = b0;
-        if (S == 2) y[S - 1] = b1;
-    } else {
 #pragma unroll
-        for (int s = 0; s < S; s++) y[s] = fma(tab(tab_h(S) + 4 * s + 2), b0, fma(tab(tab_h(S) + 4 * s + 3), b1, y[s]));
-    }
+    for (int s = 0; s < S; s++) y[s] = fma(tab(tab_h(S) + 4 * s + 2), b0, fma(tab(tab_h(S) + 4 * s + 3), b1, y[s]));
 #pragma unroll
     for (int s = 0; s < S; s++) {
         out[s] = y[s];
@@ -283,8 +272,8 @@ __host__ __device__ inline size_t wave_lines(const Wave& v, int NC, int S) {
 // between two rings.
 //
 // One CTA per (mode, part), two warps a line and all sweeps of a wavefront on
-// the SM's four FP64 pipes took 361 ms a step at 385 x 129 x 1 and 450 ms at
-// 513 x 129 x 8; this takes 134 and 180 ms, 3.4 us a step of the wavefront of four
+// the SM's four FP64 pipes took 411 ms a step at 385 x 129 x 1 and 450 ms at
+// 513 x 129 x 8; this takes 149 and 204 ms, 3.8 us a step of the wavefront of four
 // sweeps on 129 rows.
 // STAGED: both types' tables fit shared memory beside the rings, and every load
 // of a solve is one from shared memory.
@@ -752,14 +741,14 @@ void group_tables(int n, int S, int G, const double* L1, const double* L2, const
             double p1 = u == 0, p2 = u == 1;
             for (int s = 0; s < S; s++) {
                 const double y = -l1[s] * p1 - l2[s] * p2;
-                if (S > 2) at(tab_h(S) + 4 * s + u) = y;
+                at(tab_h(S) + 4 * s + u) = y;
                 p2 = p1; p1 = y;
             }
             Mf[c][u] = p1; Mf[c][2 + u] = p2;
             p1 = u == 0; p2 = u == 1;
             for (int s = S - 1; s >= 0; s--) {
                 const double x = -u1[s] * p1 - u2[s] * p2;
-                if (S > 2) at(tab_h(S) + 4 * s + 2 + u) = x;
+                at(tab_h(S) + 4 * s + 2 + u) = x;
                 p2 = p1; p1 = x;
             }
             Mb[c][u] = p1; Mb[c][2 + u] = p2;
@@ -786,22 +775,21 @@ void group_tables(int n, int S, int G, const double* L1, const double* L2, const
             }
             a = na; b = nb;
         }
-        const int CW = tab_cw(S);
         M2 f = I, r = I;   // from the warp's start (end) to the chunk's
         for (int t = 0; t < 32; t++) {
             const int cf_ = 32 * g + t, cb_ = 32 * g + 31 - t;
-            if (S <= 2) { f = mul(Mf[cf_], f); r = mul(Mb[cb_], r); }
             M2 x = f;
             for (int w = g - 1; w >= 0; w--) {   // from warp w's end to this warp's start
-                for (int q = 0; q < CW; q++) out[(size_t)(tab_cf(S) + CW * w + q) * NC + cf_] = x[q];
+                for (int q = 0; q < 4; q++) out[(size_t)(tab_cf(S) + 4 * w + q) * NC + cf_] = x[q];
                 x = mul(x, A[w]);
             }
             x = r;
             for (int w = g + 1; w < G; w++) {
-                for (int q = 0; q < CW; q++) out[(size_t)(tab_cb(S) + CW * (w - g - 1) + q) * NC + cb_] = x[q];
+                for (int q = 0; q < 4; q++) out[(size_t)(tab_cb(S) + 4 * (w - g - 1) + q) * NC + cb_] = x[q];
                 x = mul(x, B[w]);
             }
-            if (S > 2) { f = mul(Mf[cf_], f); r = mul(Mb[cb_], r); }
+            f = mul(Mf[cf_], f);
+            r = mul(Mb[cb_], r);
         }
     }
 }
