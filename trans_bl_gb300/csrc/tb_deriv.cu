@@ -69,13 +69,17 @@ struct YArgs {
 };
 
 // One real line a thread: the real and the imaginary parts of a field are
-// lines of their own, neighbours in memory.  The rows' 1/pivot is folded into the
-// right-hand side's weights and the sub-diagonal, so an interior row takes 5
-// instructions for its right-hand side and one for each sweep.  All jobs run in
-// one launch, blockIdx.y the job.  Bound by the FP64 pipe on large grids and by the
-// chain of rows on small ones: a step's 8 launches take 0.62 ms at 257 x 97 x 8 and
-// 4.3 ms at 1025 x 193 x 32; a launch per operator with a complex line a thread and
-// one instruction more a row took 1.30 and 6.3 ms.
+// lines of their own, neighbours in memory.  The right-hand side is formed with the
+// scheme's weights as they are, in units of the row's 1/dy or 1/dy^2, which together
+// with 1/pivot enters the backward sweep beside its chain: an interior row takes 5
+// instructions for its right-hand side and 1 and 2 for the sweeps, and its weights
+// stay in registers.  (All factors folded into the weights take one less, but each weight
+// is then rounded for itself and the derivative no longer cancels: 1.3 to 5 times the
+// error on 33 to 257 rows.)  All jobs run in one launch, blockIdx.y the job.  Bound by
+// the FP64 pipe on large grids and by the chain of rows on small ones: dery and deryfv
+// of a field, a launch each, take 0.10 ms at 257 x 97 x 8 and 0.48 ms at 1025 x 193 x 32;
+// a complex line a thread, which reads a row's five weights and takes one instruction
+// more a row on its chain, took 0.20 and 0.61 ms.
 __global__ void __launch_bounds__(128) k_ylines(YArgs A) {
     const int line = blockIdx.x * blockDim.x + threadIdx.x, ny = A.ny;
     if (line >= A.nx2 * A.K) return;
@@ -86,6 +90,7 @@ __global__ void __launch_bounds__(128) k_ylines(YArgs A) {
     double* __restrict__ o = reinterpret_cast<double*>(J.dst) + base;
     const double* __restrict__ ta = A.t[J.op].a;
     const double* __restrict__ tg = A.t[J.op].g;
+    const double* __restrict__ tib = A.t[J.op].ib;
     const YRhs& R = A.r[J.op];
     const double* __restrict__ wr = R.w;
     double u = 0.0;
@@ -105,6 +110,7 @@ __global__ void __launch_bounds__(128) k_ylines(YArgs A) {
     generic(0);
     generic(1);
     {
+        const double c0 = wr[14], c1 = wr[15], c2 = wr[16], c3 = wr[17], c4 = wr[18];
         double w0 = f[0], w1 = f[s], w2 = f[2 * s], w3 = f[3 * s];
         double pre[YPD];
 #pragma unroll
@@ -117,12 +123,11 @@ __global__ void __launch_bounds__(128) k_ylines(YArgs A) {
                     const double w4 = pre[q];   // row j + 2
                     const int nr = j + 2 + YPD;
                     if (nr < ny) pre[q] = f[(size_t)nr * s];
-                    const double* w = wr + 7 * j;
-                    double r = w[0] * w0;
-                    r = fma(w[1], w1, r);
-                    r = fma(w[2], w2, r);
-                    r = fma(w[3], w3, r);
-                    r = fma(w[4], w4, r);
+                    double r = c0 * w0;
+                    r = fma(c1, w1, r);
+                    r = fma(c2, w2, r);
+                    r = fma(c3, w3, r);
+                    r = fma(c4, w4, r);
                     u = fma(-ta[j], u, r);
                     o[(size_t)j * s] = u;
                     w0 = w1; w1 = w2; w2 = w3; w3 = w4;
@@ -133,6 +138,8 @@ __global__ void __launch_bounds__(128) k_ylines(YArgs A) {
     generic(ny - 2);
     generic(ny - 1);
     // backward sweep, rows ny-2 .. 0, the forward values read YPD rows ahead
+    u *= tib[ny - 1];
+    o[(size_t)(ny - 1) * s] = u;
     {
         double pre[YPD];
 #pragma unroll
@@ -145,7 +152,7 @@ __global__ void __launch_bounds__(128) k_ylines(YArgs A) {
                     const double v = pre[q];
                     const int nr = j - YPD;
                     if (nr >= 0) pre[q] = o[(size_t)nr * s];
-                    u = fma(-tg[j + 1], u, v);
+                    u = fma(-tg[j + 1], u, tib[j] * v);
                     o[(size_t)j * s] = u;
                 }
             }

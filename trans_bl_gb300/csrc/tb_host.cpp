@@ -121,15 +121,16 @@ int upload(T** dst, const std::vector<T>& src) {
     return TB_OK;
 }
 
-// y-line LHS: the sub-diagonal over the row's pivot and gam; ib returns the
-// pivots' inverses, which the right-hand side's weights take.
+// y-line LHS (TriLHS) for right-hand sides in units s.
 int upload_tri(TriLHS& t, std::vector<double> a, const std::vector<double>& b, const std::vector<double>& c,
-               std::vector<double>& ib) {
-    std::vector<double> g;
+               const std::vector<double>& s) {
+    std::vector<double> g, ib;
     thomas_factors(a, b, c, g, ib);
-    for (size_t j = 0; j < a.size(); j++) a[j] *= ib[j];
-    int r = upload(&t.a, a);
-    return r ? r : upload(&t.g, g);
+    for (size_t j = a.size() - 1; j > 0; j--) a[j] *= ib[j - 1] * (s[j - 1] / s[j]);
+    for (size_t j = 0; j < a.size(); j++) ib[j] *= s[j];
+    int r;
+    if ((r = upload(&t.a, a)) || (r = upload(&t.g, g))) return r;
+    return upload(&t.ib, ib);
 }
 
 // Row tables of an x-line operator (tb_xline.cuh) with right-hand sides in
@@ -360,34 +361,25 @@ int tb_host_build_tables(tb_ctx* c) {
     // y compact LHS (coefy/coefy_fv/coeffy derivs_par.f:1040-1142) and RHS row weights
     {
         auto lhs = [&](const double* first3, const double* sp, const double* cp, const double* pp, const double* lp,
-                       TriLHS& t, std::vector<double>& ib) {
+                       const std::vector<double>& s, TriLHS& t) {
             std::vector<double> a(ny), b(ny), cc(ny);
             a[0] = first3[0]; b[0] = first3[1]; cc[0] = first3[2];
             a[1] = sp[0]; b[1] = sp[1]; cc[1] = sp[2];
             for (int j = 2; j < ny - 2; j++) { a[j] = cp[0]; b[j] = cp[1]; cc[j] = cp[2]; }
             a[ny - 2] = pp[2]; b[ny - 2] = pp[1]; cc[ny - 2] = pp[0];
             a[ny - 1] = lp[1]; b[ny - 1] = lp[0]; cc[ny - 1] = 0.0;
-            return upload_tri(t, a, b, cc, ib);
+            return upload_tri(t, a, b, cc, s);
         };
-        std::vector<double> ib1, ibfv, ib2;
         double f1[3] = {0.0, co.fp_fd_e[0], 0.0}, ffv[3] = {0.0, 1.0, 0.0}, f2[3] = {0.0, co.fp_sd[0], co.fp_sd[1]};
-        if ((r = lhs(f1, co.sp_fd, co.cp_fd, co.pp_fd, co.lp_fd, c->ty1, ib1))) return r;
-        if ((r = lhs(ffv, co.sp_fd, co.cp_fd, co.pp_fd, co.lp_fd, c->tyfv, ibfv))) return r;
-        if ((r = lhs(f2, co.sp_sd, co.cp_sd, co.pp_sd, co.lp_sd, c->ty2, ib2))) return r;
         // RHS weights (rhsy derivs_par.f:400-449, rhsyfv 504, rhsyy 552): row j uses
-        // f[j + off .. j + off + cnt - 1] with weights scaled by v_qdy / v_qdy2
-        // (and by the LHS's 1 / pivot, fold).
+        // f[j + off .. j + off + cnt - 1], the row's v_qdy / v_qdy2 kept apart in s.
         auto q1 = [&](int j1) { return c->h_qdy[j1 - 1]; };
         auto q2 = [&](int j1) { return c->h_qdy2[j1 - 1]; };
-        std::vector<double> w((size_t)ny * 7, 0.0);
+        std::vector<double> w((size_t)ny * 7, 0.0), s(ny, 1.0);
         std::vector<int> off(ny), cnt(ny);
-        auto row = [&](int j0, int o, const double* src, int n, double s, bool rev) {
-            off[j0] = o; cnt[j0] = n;
-            for (int m = 0; m < n; m++) w[(size_t)j0 * 7 + m] = (rev ? src[n - 1 - m] : src[m]) * s;
-        };
-        auto fold = [&](const std::vector<double>& ib) {
-            for (int j = 0; j < ny; j++)
-                for (int m = 0; m < 7; m++) w[(size_t)j * 7 + m] *= ib[j];
+        auto row = [&](int j0, int o, const double* src, int n, double scale, bool rev) {
+            off[j0] = o; cnt[j0] = n; s[j0] = scale;
+            for (int m = 0; m < n; m++) w[(size_t)j0 * 7 + m] = rev ? src[n - 1 - m] : src[m];
         };
         // first derivative
         auto build1 = [&](bool fv, YRhs& out) {
@@ -398,21 +390,21 @@ int tb_host_build_tables(tb_ctx* c) {
             // rhs(jmax-1) = q(jmax-5) * (pp4 f(J) + pp5 f(J-1) + ... + pp9 f(J-5)): stored ascending from f(J-5)
             row(ny - 2, -4, co.pp_fd + 3, 6, q1(ny - 5), true);
             row(ny - 1, -4, co.lp_fd + 2, 5, q1(ny - 4), true);
-            fold(fv ? ibfv : ib1);
             int rr;
             if ((rr = upload(&out.w, w))) return rr;
             if ((rr = upload(&out.off, off))) return rr;
             return upload(&out.cnt, cnt);
         };
-        if ((r = build1(false, c->ry1))) return r;
-        if ((r = build1(true, c->ryfv))) return r;
+        if ((r = build1(false, c->ry1)) || (r = lhs(f1, co.sp_fd, co.cp_fd, co.pp_fd, co.lp_fd, s, c->ty1))) return r;
+        s[0] = 1.0;   // the boundary row 0 = 0
+        if ((r = build1(true, c->ryfv)) || (r = lhs(ffv, co.sp_fd, co.cp_fd, co.pp_fd, co.lp_fd, s, c->tyfv))) return r;
         std::fill(w.begin(), w.end(), 0.0);
         row(0, 0, co.fp_sd + 2, 6, q2(1), false);
         row(1, -1, co.sp_sd + 3, 7, q2(1), false);
         for (int j = 2; j < ny - 2; j++) row(j, -2, co.cp_sd + 3, 5, q2(j + 1 - 2), false);
         row(ny - 2, -5, co.pp_sd + 3, 7, q2(ny - 6), true);
         row(ny - 1, -5, co.lp_sd + 2, 6, q2(ny - 5), true);
-        fold(ib2);
+        if ((r = lhs(f2, co.sp_sd, co.cp_sd, co.pp_sd, co.lp_sd, s, c->ty2))) return r;
         if ((r = upload(&c->ry2.w, w))) return r;
         if ((r = upload(&c->ry2.off, off))) return r;
         if ((r = upload(&c->ry2.cnt, cnt))) return r;

@@ -34,19 +34,22 @@ void tb_set_error(const char* fmt, ...);
 
 // Device-side line operator tables ----------------------------------------
 // Thomas factors of a constant tridiagonal LHS (tridparx/tridy,
-// derivs_par.f:775-975).  y-lines: forward u_j = r_j - a_j u_{j-1} with a_j and the
-// weights of r_j over the pivot, backward u_j -= g_{j+1} u_{j+1}.  x-lines, S rows
+// derivs_par.f:775-975).  y-lines, the right-hand side's row j in units s_j (1/dy or
+// 1/dy^2 there): forward v_j = r_j - a_j v_{j-1} with a_j over the pivot before and
+// times s_{j-1} / s_j, backward u_j = ib_j v_j - g_{j+1} u_{j+1}.  x-lines, S rows
 // per lane: the row tables of tb_xline.cuh, and their FP32 copy (lines of
 // the mixed form's modes k >= 1).
 struct TriLHS {
     double* a = nullptr;   // (n)
     double* g = nullptr;   // (n) gam
+    double* ib = nullptr;  // (n) s_j / pivot
     double* xt = nullptr;
     float* xtf = nullptr;
     int S = 0;
 };
-// Row weights of the stretched-y compact RHS: row j (0-based) is
-// sum_m w[7*j+m] * f[j + off[j] + m], m < cnt[j], over the LHS's pivot.
+// Row weights of the stretched-y compact RHS, without 1/dy or 1/dy^2: row j
+// (0-based) is sum_m w[7*j+m] * f[j + off[j] + m], m < cnt[j]; the rows
+// 2 .. ny-3 have the same five.
 struct YRhs {
     double* w;   // (ny*7)
     int* off;    // (ny)
