@@ -24,7 +24,9 @@
 // two other planes, in the same lane or one aside, so the x-stencils are
 // shuffles.  A sweep spoils the strip's outer lanes (one on the left, two on
 // the right), which the adjoining strips compute as their own: strips overlap
-// instead of exchanging values, and e goes from one buffer to another.
+// instead of exchanging values, and e goes from one buffer to another.  Up to 7
+// rows a warp the registers hold it all; k_down spills 0.4, 0.5 and 1.0 KB a thread
+// at 9, 13 and 17 rows, and beyond (272 rows in all) tb_tall.cuh takes over.
 //
 // Line solves.  The NW warps own NW row chunks of S rows each.  Local
 // recurrences with zero carry in registers, chunk-end states exchanged through
@@ -97,12 +99,13 @@ inline int strips(int T, int nu, int more) {
     return q;
 }
 
-// Rows per chunk: the smallest instantiated S with NW * S >= n.
+// Rows per chunk: the smallest instantiated S with NW * S >= n (n <= 272:
+// taller levels are those of tb_tall.cuh).
 inline int pick_rows(int n) {
-    static const int opts[] = {2, 4, 5, 7, 9, 13, 17, 33};
+    static const int opts[] = {2, 4, 5, 7, 9, 13};
     for (int s : opts)
         if (NW * s >= n) return s;
-    return 33;
+    return 17;
 }
 
 #ifdef __CUDACC__

@@ -23,12 +23,15 @@
 // groups: the two border lines, then the centre lines by colour i mod 3.  The
 // centre stencil reaches i+-2 and the border stencil reaches 4 lines inwards,
 // so the lines of one group never read each other and a whole group is solved
-// at once (tb_cycle.cuh: the V-cycle's kernels and the layout of its levels).
+// at once (tb_cycle.cuh: the V-cycle's kernels and the layout of its levels;
+// tb_tall.cuh: levels of more than 272 rows).
 #include "tb_internal.h"
 #include "tb_cycle.cuh"
+#include "tb_tall.cuh"
+#include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
-#include <algorithm>
 #include <thread>
 
 namespace {
@@ -74,7 +77,8 @@ struct Mixed {
     int ptsx[MG_MAX], ptsy[MG_MAX], ylvl[MG_MAX], semi[MG_MAX];
     double dx2[MG_MAX];
     size_t elems = 0;
-    mg::Cycle cyc;            // launch arguments of the V-cycle kernel
+    mg::Cycle cyc;            // launch arguments of the V-cycle kernels
+    tall::Levels tl;          // the levels above the strips (NL of them: 0 on most grids)
 };
 
 // The finest FP32 level for the kernels outside the V-cycle.
@@ -93,63 +97,14 @@ struct FineDev {
 
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 
-// FP32 residual r - L e at the interior point (i, j) of the finest level: the
-// operator of defect (poisson_par.f:543-793) point by point (the learned
-// correction's judge and its tests; the V-cycle has its own fused form).
+// FP32 residual r - L e at the interior point (i, j) of the finest level, point
+// by point (the learned correction's judge and its tests; the V-cycle's strips have
+// their own fused form).
 __device__ __forceinline__ float2 fine_resid(const FineDev& M, int k, int i, int j) {
-    const int nxl = M.nx, n = M.ny;
-    const float* cf = M.coef;
-    const float *SP = cf, *CP = cf + 7, *PP = cf + 15, *LP = cf + 19;
-    const float* Q2 = M.qdy2;
-    const float k2b2 = (float)M.k2b2[k];
-    const float den = M.den;
     const float2* E = M.e + (size_t)k * M.elems;
-    auto f = [&](int ii, int jj) -> float2 { return E[mg::el(M.L, ii, jj)]; };
-    auto bx = [&](int jj) -> float2 {
-        if (i == 1 || i == nxl - 2) {
-            int e = (i == 1) ? 1 : -1;
-            float2 a = f(i - e, jj), c0 = f(i, jj), b = f(i + e, jj), c = f(i + 2 * e, jj), d = f(i + 3 * e, jj), g = f(i + 4 * e, jj);
-            return f2(10.f * a.x - 15.f * c0.x - 4.f * b.x + 14.f * c.x - 6.f * d.x + g.x,
-                      10.f * a.y - 15.f * c0.y - 4.f * b.y + 14.f * c.y - 6.f * d.y + g.y);
-        }
-        float2 a = f(i - 2, jj), b = f(i - 1, jj), c0 = f(i, jj), c = f(i + 1, jj), d = f(i + 2, jj);
-        return f2(-a.x + 16.f * b.x - 30.f * c0.x + 16.f * c.x - d.x, -a.y + 16.f * b.y - 30.f * c0.y + 16.f * c.y - d.y);
-    };
-    float2 b, cc, d;
-    float q2, top = 0.f;
-    if (j == 1) {
-        float2 b1 = bx(1), b2 = bx(2);
-        b = f2(SP[2] * b2.x + SP[1] * b1.x, SP[2] * b2.y + SP[1] * b1.y);
-        float2 g0 = f(i, 0), g1 = f(i, 1), g2 = f(i, 2), g3 = f(i, 3);
-        cc = f2(SP[3] * g0.x + SP[4] * g1.x + SP[5] * g2.x + SP[6] * g3.x, SP[3] * g0.y + SP[4] * g1.y + SP[5] * g2.y + SP[6] * g3.y);
-        d = f2(k2b2 * (SP[1] * g1.x + SP[2] * g2.x), k2b2 * (SP[1] * g1.y + SP[2] * g2.y));
-        q2 = Q2[0];
-    } else if (j <= n - 3) {
-        float2 ba = bx(j - 1), bb = bx(j), bc = bx(j + 1);
-        b = f2(CP[0] * ba.x + CP[1] * bb.x + CP[2] * bc.x, CP[0] * ba.y + CP[1] * bb.y + CP[2] * bc.y);
-        float2 fm2 = f(i, j - 2), fm1 = f(i, j - 1), g0 = f(i, j), fp1 = f(i, j + 1), fp2 = f(i, j + 2);
-        cc = f2(CP[3] * fm2.x + CP[4] * fm1.x + CP[5] * g0.x + CP[6] * fp1.x + CP[7] * fp2.x,
-                CP[3] * fm2.y + CP[4] * fm1.y + CP[5] * g0.y + CP[6] * fp1.y + CP[7] * fp2.y);
-        d = f2(k2b2 * (CP[0] * fm1.x + CP[1] * g0.x + CP[2] * fp1.x), k2b2 * (CP[0] * fm1.y + CP[1] * g0.y + CP[2] * fp1.y));
-        q2 = Q2[j - 2];
-    } else if (j == n - 2) {
-        b = bx(j);
-        float2 fm1 = f(i, j - 1), g0 = f(i, j), fp1 = f(i, j + 1);
-        cc = f2(PP[3] * fp1.x + PP[2] * g0.x + PP[1] * fm1.x, PP[3] * fp1.y + PP[2] * g0.y + PP[1] * fm1.y);
-        d = f2(k2b2 * g0.x, k2b2 * g0.y);
-        q2 = Q2[j - 1];
-    } else {
-        b = bx(j);
-        float2 fm2 = f(i, j - 2), fm1 = f(i, j - 1), g0 = f(i, j);
-        cc = f2(LP[2] * g0.x + LP[3] * fm1.x + LP[4] * fm2.x, LP[2] * g0.y + LP[3] * fm1.y + LP[4] * fm2.y);
-        d = f2(k2b2 * g0.x, k2b2 * g0.y);
-        q2 = Q2[j - 2];
-        top = LP[1] * sqrtf((M.alpha2 - k2b2) * M.ify) * sqrtf(q2);
-    }
-    float2 fij = f(i, j);
-    float2 s = M.r[(size_t)k * M.elems + mg::el(M.L, i, j)];
-    return f2(s.x - (b.x * den + cc.x * q2 + d.x * M.ify - top * fij.x),
-              s.y - (b.y * den + cc.y * q2 + d.y * M.ify - top * fij.y));
+    const tall::PointOp O{M.nx, M.ny, M.coef, M.qdy2, (float)M.k2b2[k], M.den, M.ify, M.alpha2};
+    return tall::point_resid(O, i, j, M.r[(size_t)k * M.elems + mg::el(M.L, i, j)],
+                             [&](int ii, int jj) { return E[mg::el(M.L, ii, jj)]; });
 }
 
 // The residual of one mode into out, line-contiguous (nx, ny).
@@ -563,8 +518,7 @@ int strip(tb_ctx* c, const mg::Cycle& M, int l, int up, int from) {
         case 7: r = launch_strip<7>(c, M, l, up, from); break;
         case 9: r = launch_strip<9>(c, M, l, up, from); break;
         case 13: r = launch_strip<13>(c, M, l, up, from); break;
-        case 17: r = launch_strip<17>(c, M, l, up, from); break;
-        default: r = launch_strip<33>(c, M, l, up, from); break;
+        default: r = launch_strip<17>(c, M, l, up, from); break;
     }
     if (r) return r;
     return l == 0 && up ? tb_prof_end(c, PROF_RELAX0, p0) : TB_OK;
@@ -579,9 +533,61 @@ int strip_attr() {
 int cycle_attrs() {
     int r;
     if ((r = strip_attr<2>()) || (r = strip_attr<4>()) || (r = strip_attr<5>()) || (r = strip_attr<7>()) || (r = strip_attr<9>()) ||
-        (r = strip_attr<13>()) || (r = strip_attr<17>()) || (r = strip_attr<33>()))
+        (r = strip_attr<13>()) || (r = strip_attr<17>()))
         return r;
     return TB_OK;
+}
+
+// One relaxation sweep of a tall level: border lines, then centre colours 0, 1, 2.
+int tall_sweep(tb_ctx* c, const tall::Levels& T, int l) {
+    const size_t smem = (size_t)(tall::THREADS / 32) * 2 * T.n * sizeof(float2);
+    auto relax = [&](int first, int step, int nlines) -> int {
+        const unsigned nb = tb_blocks((size_t)nlines * T.K, tall::THREADS / 32);
+        switch (tall::pick_rows(T.n)) {
+            case 9: tall::k_relax<9><<<nb, tall::THREADS, smem, c->stream>>>(T, l, first, step, nlines); break;
+            case 11: tall::k_relax<11><<<nb, tall::THREADS, smem, c->stream>>>(T, l, first, step, nlines); break;
+            case 13: tall::k_relax<13><<<nb, tall::THREADS, smem, c->stream>>>(T, l, first, step, nlines); break;
+            case 15: tall::k_relax<15><<<nb, tall::THREADS, smem, c->stream>>>(T, l, first, step, nlines); break;
+            default: tall::k_relax<17><<<nb, tall::THREADS, smem, c->stream>>>(T, l, first, step, nlines); break;
+        }
+        TB_CHECK_LAUNCH(c);
+        return TB_OK;
+    };
+    const int nxl = T.nx[l];
+    int r = relax(1, nxl - 3, 2);
+    for (int first = 2; !r && first < 5 && first <= nxl - 3; first++) r = relax(first, 3, (nxl - 3 - first) / 3 + 1);
+    return r;
+}
+// The tall levels on the way down, from e of the finest one, and on the way up.
+int tall_down(tb_ctx* c, const tall::Levels& T, const mg::Cycle& M) {
+    int r;
+    for (int l = 0; l < T.NL; l++) {
+        for (int s = 0; s < NU_PRE; s++)
+            if ((r = tall_sweep(c, T, l))) return r;
+        tall::k_resid<<<tb_blocks((size_t)T.nx[l] * T.n * T.K, 256), 256, 0, c->stream>>>(T, l);
+        TB_CHECK_LAUNCH(c);
+        if (l + 1 < T.NL) tall::k_restrict_x<<<tb_blocks((size_t)T.nx[l + 1] * T.n * T.K, 256), 256, 0, c->stream>>>(T, l);
+        else {
+            const mg::Level& N = M.lv[T.NL];
+            tall::k_restrict_out<<<dim3(tb_blocks(N.nx - 2, 128), N.n - 1, T.K), 128, 0, c->stream>>>(T, M);
+        }
+        TB_CHECK_LAUNCH(c);
+    }
+    return TB_OK;
+}
+int tall_up(tb_ctx* c, const tall::Levels& T, const mg::Cycle& M) {
+    cudaEvent_t p0 = nullptr;
+    int r;
+    for (int l = T.NL - 1; l >= 0; l--) {
+        if (l == 0 && (r = tb_prof_begin(c, PROF_RELAX0, &p0))) return r;
+        const unsigned nb = tb_blocks((size_t)T.nx[l] * T.n * T.K, 256);
+        if (l + 1 < T.NL) tall::k_prolong_x<<<nb, 256, 0, c->stream>>>(T, l + 1);
+        else tall::k_prolong_in<<<nb, 256, 0, c->stream>>>(T, M);
+        TB_CHECK_LAUNCH(c);
+        for (int s = 0; s < NU_POST; s++)
+            if ((r = tall_sweep(c, T, l))) return r;
+    }
+    return tb_prof_end(c, PROF_RELAX0, p0);
 }
 
 // The V-cycles of one correction.
@@ -592,15 +598,23 @@ int vcycles(tb_ctx* c) {
     if ((r = tb_prof_begin(c, PROF_SOR, &ps))) return r;
     mg::Cycle M = m->cyc;
     M.state = c->pstate;
+    tall::Levels T = m->tl;
+    T.state = c->pstate;
+    T.k2b2 = c->k2b2;
     const int bot = M.NL - 1;
+    const dim3 tiles(tb_blocks(c->g.nx, 32), tb_blocks(c->g.ny, 32), M.K), tile(32, 8);
+    if (T.NL) { tall::k_cross<false><<<tiles, tile, 0, c->stream>>>(T, M); TB_CHECK_LAUNCH(c); }
     for (int v = 0; v < INNER_VCYCLES; v++) {
-        for (int l = 0; l < bot; l++)
+        if (T.NL && (r = tall_down(c, T, M))) return r;
+        for (int l = T.NL; l < bot; l++)
             if ((r = strip(c, M, l, 0, v > 0 && l == 0))) return r;
         mg::k_direct<<<dim3(tb_blocks(M.N, 4 * mg::NW), M.K), mg::NT, 0, c->stream>>>(M);
         TB_CHECK_LAUNCH(c);
-        for (int l = bot - 1; l >= 0; l--)
+        for (int l = bot - 1; l >= T.NL; l--)
             if ((r = strip(c, M, l, 1, 0))) return r;
+        if (T.NL && (r = tall_up(c, T, M))) return r;
     }
+    if (T.NL) { tall::k_cross<true><<<tiles, tile, 0, c->stream>>>(T, M); TB_CHECK_LAUNCH(c); }
     return tb_prof_end(c, PROF_SOR, ps);
 }
 
@@ -663,6 +677,50 @@ void line_tables(int n, int S, double unit, double qx, const double* cf, const d
         const double row[12] = {unit * w[0], unit * w[1], unit * w[2], -L1[j], -L2[j], ID[j] * h1[j], ID[j] * h2[j],
                                 -U1[j] * ID[j], -U2[j] * ID[j], ID[j], k1[j], k2[j]};
         put_pairs(out + (size_t)mg::ROW4 * j, row, 12);
+    }
+}
+
+// Line tables of a tall level, type and mode (tall::tab_size): the band LU rows,
+// the responses h1 h2 (k1 k2) of a lane's S rows to the states entering them
+// forward (backward), and the Kogge-Stone matrices of the lanes' propagators.
+void tall_tables(int n, int S, const double* L1, const double* L2, const double* U1, const double* U2, const double* ID, float* out) {
+    using M2 = std::array<double, 4>;
+    auto mul = [](const M2& A, const M2& B) {
+        return M2{A[0] * B[0] + A[1] * B[2], A[0] * B[1] + A[1] * B[3], A[2] * B[0] + A[3] * B[2], A[2] * B[1] + A[3] * B[3]};
+    };
+    const double* lu[5] = {L1, L2, U1, U2, ID};
+    for (int q = 0; q < 5; q++)
+        for (int j = 0; j < n; j++) out[(size_t)q * n + j] = (float)lu[q][j];
+    float *h = out + 5 * (size_t)n, *kk = h + 2 * (size_t)n, *Pf = kk + 2 * (size_t)n, *Pb = Pf + 640;
+    M2 Mf[32], Mb[32];
+    for (int t = 0; t < 32; t++) {
+        const int r0 = std::min(n, t * S), r1 = std::min(n, r0 + S);
+        for (int u = 0; u < 2; u++) {
+            double p1 = u == 0, p2 = u == 1;
+            for (int j = r0; j < r1; j++) {
+                const double y = -L2[j] * p2 - L1[j] * p1;
+                h[(size_t)u * n + j] = (float)y;
+                p2 = p1; p1 = y;
+            }
+            Mf[t][u] = p1; Mf[t][2 + u] = p2;
+            p1 = u == 0; p2 = u == 1;
+            for (int j = r1 - 1; j >= r0; j--) {
+                const double x = (-U1[j] * p1 - U2[j] * p2) * ID[j];
+                kk[(size_t)u * n + j] = (float)x;
+                p2 = p1; p1 = x;
+            }
+            Mb[t][u] = p1; Mb[t][2 + u] = p2;
+        }
+    }
+    for (int d = 0, off = 1; d < 5; d++, off <<= 1) {
+        M2 nf[32], nb[32];
+        for (int t = 0; t < 32; t++) {
+            for (int q = 0; q < 4; q++) { Pf[(d * 32 + t) * 4 + q] = (float)Mf[t][q]; Pb[(d * 32 + t) * 4 + q] = (float)Mb[t][q]; }
+            nf[t] = t >= off ? mul(Mf[t], Mf[t - off]) : Mf[t];
+            nb[t] = t + off < 32 ? mul(Mb[t], Mb[t + off]) : Mb[t];
+        }
+        std::copy(nf, nf + 32, Mf);
+        std::copy(nb, nb + 32, Mb);
     }
 }
 
@@ -770,22 +828,30 @@ int tb_mixed_setup(tb_ctx* c) {
         return TB_ERR_ARG;
     }
     mg::Cycle& cy = m->cyc;
+    tall::Levels& tl = m->tl;
     std::memset(&cy, 0, sizeof cy);
+    std::memset(&tl, 0, sizeof tl);
+    while (m->ptsy[tl.NL] > tall::STRIP_ROWS) tl.NL++;   // at least one level has half the rows
     cy.nu_pre = NU_PRE; cy.nu_post = NU_POST;
     size_t off = 0;
     int t4 = 0;   // tables per mode
     for (int l = 0; l < NL; l++) {
         mg::Level& L = cy.lv[l];
         L.nx = m->ptsx[l]; L.n = m->ptsy[l]; L.semi = m->semi[l];
-        L.S = mg::pick_rows(L.n);
         const int Tn = L.nx / 3 + 1;   // elements of a colour plane
         L.T = (Tn + 3) & ~3;
-        L.np = mg::NW * L.S + 2;
+        if (l < tl.NL) {   // of these levels only the finest has colour planes
+            L.np = L.n + 2;
+            if (l > 0) continue;
+        } else {
+            L.S = mg::pick_rows(L.n);
+            L.np = mg::NW * L.S + 2;
+            L.down = mg::strips(Tn, NU_PRE, 1);
+            L.up = mg::strips(Tn, NU_POST, 0);
+            if (l < NL - 1) { L.tab = t4; t4 += mg::level4(L); }
+        }
         L.off = (int)off;
         off += (size_t)3 * L.np * L.T;
-        L.down = mg::strips(Tn, NU_PRE, 1);
-        L.up = mg::strips(Tn, NU_POST, 0);
-        if (l < NL - 1) { L.tab = t4; t4 += mg::level4(L); }
         if (off > 0x7fffffffu) { tb_set_error("mixed form: grid too large for the FP32 hierarchy"); return TB_ERR_ARG; }
     }
     cy.tab4 = t4;
@@ -799,6 +865,22 @@ int tb_mixed_setup(tb_ctx* c) {
         TB_CUDA(cudaMemset(*p, 0, w * sizeof(float2)));
     }
     cy.ea = m->ea; cy.eb = m->eb; cy.r = m->r;
+    if (tl.NL) {
+        tl.K = K; tl.n = ny;
+        tl.ify = (float)(1.0 / c->cfg.fac_y);
+        tl.alpha2 = (float)(c->cfg.alpha * c->cfg.alpha);
+        for (int l = 0; l < tl.NL; l++) {
+            tl.nx[l] = m->ptsx[l];
+            tl.qx[l] = (float)(1.0 / (12.0 * m->dx2[l] * c->cfg.fac_y));
+            tl.off[l] = tl.elems;
+            tl.elems += (size_t)m->ptsx[l] * ny;
+        }
+        const size_t te = (size_t)K * tl.elems, tr = (size_t)K * c->g.nx * ny;
+        for (const auto& p : {std::make_pair(&tl.e, te), std::make_pair(&tl.r, te), std::make_pair(&tl.rr, tr)}) {
+            TB_CUDA(cudaMalloc(p.first, p.second * sizeof(float2)));
+            TB_CUDA(cudaMemset(*p.first, 0, p.second * sizeof(float2)));
+        }
+    }
     TB_CUDA(cudaMalloc(&m->maxsq, K * sizeof(unsigned long long)));
     TB_CUDA(cudaMemset(m->maxsq, 0, K * sizeof(unsigned long long)));
     TB_CUDA(cudaMalloc(&m->hvalid, 4 * sizeof(int)));
@@ -822,8 +904,17 @@ int tb_mixed_setup(tb_ctx* c) {
     // level's y-line matrix and chunk tables) and residual rows, in FP32
     std::vector<float4> t32((size_t)K * cy.tab4, make_float4(0.f, 0.f, 0.f, 0.f));
     std::vector<double> a, L1(ny), L2(ny), U1(ny), U2(ny), ID(ny);
+    std::vector<float> ttall((size_t)2 * tl.NL * K * tall::tab_size(ny), 0.f);
+    for (int type = 0; type < 2; type++)
+        for (int l = 0; l < tl.NL; l++)
+            for (int k = 0; k < K; k++) {
+                tb_poisson_band_matrix_dx(c, type, 1, k + 1, m->dx2[l], a);
+                tb_band5_factor(ny, a, L1.data(), L2.data(), U1.data(), U2.data(), ID.data());
+                tall_tables(ny, tall::pick_rows(ny), L1.data(), L2.data(), U1.data(), U2.data(), ID.data(),
+                            &ttall[(((size_t)type * tl.NL + l) * K + k) * tall::tab_size(ny)]);
+            }
     for (int k = 0; k < K; k++)
-        for (int l = 0; l < NL - 1; l++) {
+        for (int l = tl.NL; l < NL - 1; l++) {
             const mg::Level& L = cy.lv[l];
             const double* cfl = &cf64[24 * m->ylvl[l]];
             const double qx = 1.0 / (12.0 * m->dx2[l] * c->cfg.fac_y);
@@ -858,6 +949,14 @@ int tb_mixed_setup(tb_ctx* c) {
     if ((r = upl(&m->coef, cf))) return r;
     std::vector<float> q2(c->h_qdy2.begin(), c->h_qdy2.end());
     if ((r = upl(&m->qdy2, q2))) return r;
+    if (tl.NL) {
+        float* t = nullptr;
+        r = upl(&t, ttall);
+        tl.tab = t;
+        if (r) return r;
+        tl.coef = m->coef;
+        tl.qdy2 = m->qdy2;
+    }
     // exact inverse of the coarsest operator per mode (modes in parallel)
     const int N = m->N;
     std::vector<float> ainv((size_t)K * N * N);
@@ -918,7 +1017,8 @@ void tb_mixed_free(tb_ctx* c) {
         for (cplx* p : h)
             if (p) cudaFree(p);
     for (void* p : {(void*)m->ea, (void*)m->eb, (void*)m->r, (void*)m->tab, (void*)m->drow, (void*)m->coef, (void*)m->qdy2, (void*)m->ainv,
-                    (void*)m->maxsq, (void*)m->hvalid, (void*)m->iter, (void*)m->lkeep})
+                    (void*)m->maxsq, (void*)m->hvalid, (void*)m->iter, (void*)m->lkeep, (void*)m->tl.e, (void*)m->tl.r,
+                    (void*)m->tl.rr, (void*)m->tl.tab})
         if (p) cudaFree(p);
     delete m;
     c->mixed = nullptr;
