@@ -97,3 +97,21 @@ def test_defect_rounds_no_more_than_its_terms(nx, ny):
     got = np.array(ctx.poisson_stats()["residual"])
     rms = [float(np.sqrt(np.mean(v[1:] ** 2))) for v in (got, host)]
     assert rms[0] <= rms[1], rms
+
+
+@pytest.mark.parametrize("n_lambda,counts", [(6.0, [7, 6, 6, 6]), (3.0, [7, 7, 7, 6])])
+def test_257_rows_converge_at_1e_8(n_lambda, counts):
+    """The 257-row grid of the roughness runs (first cell 0.005 delta*) at their
+    tolerance, not far above the defect's rounding there, with their x spacing and
+    half of it: every mode converges, with the corrections of a defect that forms
+    the operator's terms one by one."""
+    kw = dict(amp2d=3e-3, amp3d=3e-3, strip=(0.5, 1.0), n_lambda=n_lambda)
+    cfg = configs.blasius_ts_config(513, 257, 4, 8, 4, max_vcycles=11, precision=api.FORM_MIXED, **kw)
+    # the base flow of 17 stations, repeated
+    base = [np.ascontiguousarray(np.resize(b.T, (513, 257)).T)
+            for b in api.baseflow_fs(configs.blasius_ts_config(17, 257, 4, 8, 2, **kw), 0.0)]
+    ctx = api.Context(cfg, api.generate_coefs(cfg.stf, cfg.msh), base)
+    ctx.put_state(configs.disturbed_state(cfg, base, np.random.default_rng(23), 1e-3))
+    ctx.poi_uy(ctx.outuy(), 1e-8)
+    ps = ctx.poisson_stats()
+    assert ps["noconv"] == 0 and ps["vcycles"] == counts
