@@ -373,7 +373,7 @@ int tb_profile_read(tb_ctx* ctx, int family, double* ms, long long* launches);
    not allocate GPU memory after start-up (a memory manager that owns all free
    device memory, or a real-time section).  Needs no context and
    allocates nothing: the lines are filtered in place, the operator's tables
-   kept in a 32 MiB array built into the library; one call takes nx*ny*kfour <= 2^21 - 4096 points and
+   kept in a 197 KB array built into the library; one call takes nx*ny*kfour <= 2^21 - 4096 points and
    nx <= 4096 (filter larger grids one slice of Fourier modes per call) and
    returns TB_ERR_ARG beyond that.  The first call on a device sets up the
    array's address and must precede any stream capture (after cudaDeviceReset

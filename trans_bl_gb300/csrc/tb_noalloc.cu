@@ -10,12 +10,12 @@
 // allocation.
 //
 //  - The lines are filtered in place, two warps per x-line staged in shared
-//    memory (tb_xline.cuh), with the operator's row tables built at every call
-//    in a fixed 32 MiB scratch array, a file-scope __device__ array.  One call
-//    filters at most nx*ny*kfour = 2^21 - 4096 points with nx <= 4096 (larger
-//    grids: call once per slice of Fourier modes, which the filter treats
-//    independently).  Every GPU that loads this library keeps the array
-//    resident until the process exits.
+//    memory (tb_xline.cuh).  The operator's row tables, built at every call, and
+//    the pivots of lines where they do not settle sit in a file-scope __device__
+//    array of 197 KB, which every GPU that loads this library keeps until the
+//    process exits.  One call filters at most nx*ny*kfour = 2^21 - 4096 points
+//    with nx <= 4096, the entry point's documented limits (larger grids: call once
+//    per slice of Fourier modes, which the filter treats independently).
 //  - The first call on a device (with that device current) looks up the
 //    array's device address with cudaGetSymbolAddress and keeps it for the
 //    device; make that first call before any stream capture.  The kept
@@ -33,17 +33,18 @@
 #include <algorithm>
 #include <atomic>
 
-#define TB_NOALLOC_FILTER_MAX (1u << 21)      // complex*16 elements in the scratch (32 MiB)
-#define TB_NOALLOC_PIVOTS 4096                 // longest line; the last elements hold the Thomas pivots
-#define TB_NOALLOC_FIELD_MAX (TB_NOALLOC_FILTER_MAX - TB_NOALLOC_PIVOTS)
+#define TB_NOALLOC_LINE_MAX 4096                                // longest line
+#define TB_NOALLOC_FIELD_MAX ((1u << 21) - TB_NOALLOC_LINE_MAX)  // points per call
 
-static __device__ __align__(256) double2 g_filter_scratch[TB_NOALLOC_FILTER_MAX];
+// the row tables of the longest line (xl::table_size), then its pivots
+constexpr int TB_NOALLOC_TABLES = 5 * TB_NOALLOC_LINE_MAX + 320 + 256;
+static __device__ __align__(256) double g_filter_scratch[TB_NOALLOC_TABLES + TB_NOALLOC_LINE_MAX];
 
 namespace {
 
 // Device address of the scratch per device ordinal, set by the first call on
 // that device (concurrent first calls store the same value).
-std::atomic<double2*> g_scratch_addr[64];
+std::atomic<double*> g_scratch_addr[64];
 
 // 1 / pivot of the Thomas factors of the filter's LHS (lhs_tridf
 // filter_par.f:181), computed on the host and passed by value: rows first ..
@@ -140,15 +141,15 @@ __global__ void __launch_bounds__(64 * FILTER_LINES) k_filter_lines(FilterArgs A
     }
 }
 
-int scratch_address(double2** out) {
+int scratch_address(double** out) {
     int dev = 0;
     TB_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) { tb_set_error("device ordinal %d out of range", dev); return TB_ERR_ARG; }
-    double2* a = g_scratch_addr[dev].load(std::memory_order_acquire);
+    double* a = g_scratch_addr[dev].load(std::memory_order_acquire);
     if (!a) {
         void* p = nullptr;
         TB_CUDA(cudaGetSymbolAddress(&p, g_filter_scratch));
-        a = static_cast<double2*>(p);
+        a = static_cast<double*>(p);
         g_scratch_addr[dev].store(a, std::memory_order_release);
     }
     *out = a;
@@ -160,22 +161,21 @@ int scratch_address(double2** out) {
 extern "C" int tb_filter_trid_noalloc(double* wx, double* wy, double* wz, int nx, int ny, int kfour, double alphaf,
                                       void* stream) {
     if (!wx || !wy || !wz) { tb_set_error("tb_filter_trid_noalloc: null field pointer"); return TB_ERR_ARG; }
-    if (nx < 8 || nx > TB_NOALLOC_PIVOTS || ny < 2 || kfour < 1) {
-        tb_set_error("tb_filter_trid_noalloc: need 8 <= nx <= %d, ny >= 2, kfour >= 1", TB_NOALLOC_PIVOTS);
+    if (nx < 8 || nx > TB_NOALLOC_LINE_MAX || ny < 2 || kfour < 1) {
+        tb_set_error("tb_filter_trid_noalloc: need 8 <= nx <= %d, ny >= 2, kfour >= 1", TB_NOALLOC_LINE_MAX);
         return TB_ERR_ARG;
     }
     size_t n3 = (size_t)nx * ny * kfour;
     if (n3 > TB_NOALLOC_FIELD_MAX) {
-        tb_set_error("tb_filter_trid_noalloc: nx*ny*kfour = %zu exceeds the %u-element scratch (32 MiB); "
+        tb_set_error("tb_filter_trid_noalloc: nx*ny*kfour = %zu exceeds the %u points of one call; "
                      "filter fewer Fourier modes per call", n3, (unsigned)TB_NOALLOC_FIELD_MAX);
         return TB_ERR_ARG;
     }
-    double2* s = nullptr;
-    int r = scratch_address(&s);
+    double* T = nullptr;
+    int r = scratch_address(&T);
     if (r) return r;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    double* piv = reinterpret_cast<double*>(s + TB_NOALLOC_FIELD_MAX);
-    double* T = reinterpret_cast<double*>(s);
+    double* piv = T + TB_NOALLOC_TABLES;
     auto off = [&](int i) { return (i >= 3 && i <= nx - 4) ? alphaf : 0.0; };
     Pivots P;
     double bet = 1.0;   // pivot of the row before
