@@ -154,7 +154,7 @@ int tb_destroy(tb_ctx* c) {
                     c->fcx2, c->fcllx2, c->th, c->th1, c->dv1t, c->dv2t, c->thb, c->th_phys, c->gibbs, c->delta_no, c->k2b2,
                     c->tx1.xt, c->tx1.xtf, c->tx2.xt, c->tx2.xtf, c->tfil.xt, c->tfil.xtf, c->ty1.a, c->ty1.g, c->ty1.ib, c->tyfv.a, c->tyfv.g, c->tyfv.ib,
                     c->ty2.a, c->ty2.g, c->ty2.ib, c->ry1.w, c->ry1.off, c->ry1.cnt, c->ryfv.w, c->ryfv.off, c->ryfv.cnt,
-                    c->ry2.w, c->ry2.off, c->ry2.cnt, c->px.tab, c->pfc, c->psc, c->pfct, c->pdef,
+                    c->ry2.w, c->ry2.off, c->ry2.cnt, c->px.tab, c->pfc, c->psc,
                     c->pl_fc, c->pl_sc, c->pl_fct, c->pl_def, c->pl_tab, c->pl_maxsq, c->pstate, c->perr, c->pqdy2, c->pcoef, c->wcoef};
     for (void* p : ptrs) if (p) cudaFree(p);
     tb_graph_free(c);

@@ -110,7 +110,7 @@ struct tb_ctx {
     YRhs ry1, ryfv, ry2;
     PentaX px;
     // Poisson work (per mode blocks of lvl_elems complex): fc, sc, fct
-    cplx *pfc = nullptr, *psc = nullptr, *pfct = nullptr, *pdef = nullptr;
+    cplx *pfc = nullptr, *psc = nullptr;
     // plain form: line-contiguous real/imaginary planes per (mode, part) of
     // the multigrid arrays (element (i, j) of level l at lvl_off[l] + i*ptsy[l] + j)
     double *pl_fc = nullptr, *pl_sc = nullptr, *pl_fct = nullptr, *pl_def = nullptr;

@@ -12,22 +12,16 @@
 namespace {
 
 struct PoiDev {
-    cplx *fc, *sc, *fct, *def;    // per-mode blocks
-    const double* coef;           // sp(7) cp(8) pp(4) lp(5) per level
-    const double* qdy2;           // (ny, msh)
-    const double* k2b2;
-    int* state;                   // per mode: [2k] active, [2k+1] vcycles done
-    double* err;
-    int nx, ny, K, msh;
-    int ptsx[TB_MAX_MSH], ptsy[TB_MAX_MSH];
-    size_t off[TB_MAX_MSH], elems, dstride;
-    double dx2[TB_MAX_MSH];
-    double den[TB_MAX_MSH];       // 1 / (12 dx2 fac_y)
-    double fac_y, alpha, ify;
+    cplx *fc, *sc;         // blocks of elems per mode, x-contiguous
+    const double* coef;    // sp(7) cp(8) pp(4) lp(5) of the fine level
+    const int* state;      // per mode: [2k] active, [2k+1] corrections done
+    int nx, ny, K;
+    size_t elems;
+    double fac_y, alpha;
 };
 
-__device__ __forceinline__ cplx& AT(cplx* base, const PoiDev& P, int k, int l, int i, int j) {
-    return base[(size_t)k * P.elems + P.off[l] + (size_t)i + (size_t)P.ptsx[l] * j];
+__device__ __forceinline__ cplx& AT(cplx* base, const PoiDev& P, int k, int i, int j) {
+    return base[(size_t)k * P.elems + (size_t)i + (size_t)P.nx * j];
 }
 
 // ---------------------------------------------------------------------------
@@ -63,8 +57,8 @@ __global__ void k_source(PoiDev P, const cplx* wx, const cplx* dwzdx, const cplx
                              -(lp1 * dwzdx[o].y));
         }
     }
-    AT(P.sc, P, k, 0, i, j) = s;
-    AT(P.fc, P, k, 0, i, j) = uy[q];
+    AT(P.sc, P, k, i, j) = s;
+    AT(P.fc, P, k, i, j) = uy[q];
 }
 
 // ---------------------------------------------------------------------------
@@ -161,7 +155,7 @@ __global__ void k_write_uy(PoiDev P, cplx* uy) {
     if (q >= n) return;
     int i = (int)(q % P.nx), j = (int)((q / P.nx) % P.ny), k = (int)(q / ((size_t)P.nx * P.ny));
     if (j < 1 || i < 1 || i > P.nx - 2) return;
-    uy[q] = AT(P.fc, P, k, 0, i, j);
+    uy[q] = AT(P.fc, P, k, i, j);
 }
 
 __global__ void k_activate(int* state, int K) {
@@ -172,15 +166,9 @@ __global__ void k_activate(int* state, int K) {
 PoiDev make_dev(tb_ctx* c) {
     PoiDev P;
     std::memset(&P, 0, sizeof P);
-    P.fc = c->pfc; P.sc = c->psc; P.fct = c->pfct; P.def = c->pdef; P.coef = c->pcoef;
-    P.qdy2 = c->pqdy2; P.k2b2 = c->k2b2; P.state = c->pstate; P.err = c->perr;
-    P.nx = c->g.nx; P.ny = c->g.ny; P.K = c->g.K; P.msh = c->g.msh;
-    for (int l = 0; l < c->g.msh; l++) {
-        P.ptsx[l] = c->g.ptsx[l]; P.ptsy[l] = c->g.ptsy[l]; P.off[l] = c->g.lvl_off[l]; P.dx2[l] = c->h_dx2[l];
-        P.den[l] = 1.0 / (12.0 * c->h_dx2[l] * c->cfg.fac_y);
-    }
-    P.ify = 1.0 / c->cfg.fac_y;
-    P.elems = c->g.lvl_elems; P.dstride = (size_t)c->g.nx * c->g.ny;
+    P.fc = c->pfc; P.sc = c->psc; P.coef = c->pcoef; P.state = c->pstate;
+    P.nx = c->g.nx; P.ny = c->g.ny; P.K = c->g.K;
+    P.elems = c->g.lvl_elems;
     P.fac_y = c->cfg.fac_y; P.alpha = c->cfg.alpha;
     return P;
 }
@@ -188,16 +176,13 @@ PoiDev make_dev(tb_ctx* c) {
 }  // namespace
 
 int tb_poisson_setup(tb_ctx* c) {
-    int ny = c->g.ny, K = c->g.K;
-    size_t w = (size_t)K * c->g.lvl_elems;
-    for (cplx** p : {&c->pfc, &c->psc, &c->pfct}) {
+    const int K = c->g.K;
+    const size_t w = (size_t)K * c->g.lvl_elems;
+    for (cplx** p : {&c->pfc, &c->psc}) {
         if (*p) cudaFree(*p);
         TB_CUDA(cudaMalloc(p, w * sizeof(cplx)));
         TB_CUDA(cudaMemset(*p, 0, w * sizeof(cplx)));
     }
-    if (c->pdef) cudaFree(c->pdef);
-    TB_CUDA(cudaMalloc(&c->pdef, (size_t)K * c->g.nx * ny * sizeof(cplx)));
-    TB_CUDA(cudaMemset(c->pdef, 0, (size_t)K * c->g.nx * ny * sizeof(cplx)));
     if (!c->pstate) TB_CUDA(cudaMalloc(&c->pstate, 2 * K * sizeof(int)));
     if (!c->perr) TB_CUDA(cudaMalloc(&c->perr, K * sizeof(double)));
     return TB_OK;
