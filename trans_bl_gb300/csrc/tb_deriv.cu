@@ -166,7 +166,8 @@ __global__ void __launch_bounds__(128) k_ylines(YArgs A) {
 // where the tuner found that faster.  Where every pair of warps has one line at
 // most, or a line is so long that the tables leave no room for two, the tables are read
 // from global memory by blocks of two lines, without the copy to shared memory
-// (D1 of 33 lines of 1025 points: 33 us, 49 with it; of 129 lines of 385: 20 and 28).
+// (D1 of 33 lines of 1025 points: 33 us, 49 with it; of 129 lines of 385: 20 and 28;
+// near the line the two meet: of 1032 lines of 385, one a pair, 29 and 28).
 template <int OP>
 int launch_xop(tb_ctx* c, XArgs& A, const TriLHS& t) {
     A.S = t.S; A.tab = t.xt; A.tabf = t.xtf;

@@ -161,7 +161,7 @@ struct tb_ctx {
     int sm_count = 0;
     int fp32_lines = 0;                    // mixed form: line operators of modes k >= 1 in FP32 (opt-in)
     // launch shapes chosen by tb_autotune (0: the built-in defaults)
-    int tune_xw = 0;                       // warps per block of the x-line kernel (1 or 2)
+    int tune_xw = 0;                       // lines per block of the x-line kernel: 1 half of what fits, 2 all
     int tune_yt = 0;                       // threads per block of the y-line kernel (32, 64 or 128)
     int tune_nl = 0;                       // resident blocks per SM of the tensor-core passes
     int tune_pg3 = 0, tune_pg1 = 0;        // plain form: 1 + log2 warps per line of multi- / single-sweep launches

@@ -446,8 +446,11 @@ size_t xw_smem(int nx) { return (size_t)XW_WARPS * 64 * WarpLine::padded(nx) * s
 
 // A run of lines per block (k_penta_x), as many blocks as the SMs hold, with up to
 // 8 lines at a time.  Blocks of two lines that read the tables from global memory
-// where an SM has fewer than 8 lines, which the copy to shared memory would hold up
-// (257 x 97 x 8: 44 us with it, 27 without), and where the tables leave no room for two.
+// where an SM has fewer than 8 lines, which the copy to shared memory would hold up,
+// and where the tables leave no room for two.  With and without the copy, us:
+// 4.4 lines an SM 31 and 24 (257 points), 78 and 59 (1025 points); 6.9 lines 47 and 45
+// (513), 83 and 82 (1025); 9.3 lines 57 and 46 (257), 64 and 69 (513), 112 and 145
+// (1025); 39 lines 143 and 140 (257), 213 and 233 (513), 366 and 461 (1025).
 int launch_penta(tb_ctx* c, const cplx* D, const cplx* W, cplx* out, double g) {
     PentaArgs A{D, W, out, c->px.tab, c->g.nx, c->g.ny, c->g.K, c->px.S, 0, g, c->cfg.beta, c->px.unit};
     const size_t tab = (size_t)penta_table_size(A.S) * sizeof(double), line = (size_t)penta_line_size(A.S) * sizeof(double);

@@ -797,8 +797,8 @@ void group_tables(int n, int S, int G, const double* L1, const double* L2, const
 // Warps per line (as log2, the table group) of a launch with `slots` sweeps in
 // flight on lines of n points: one row a lane as far as four warps go, for the
 // shortest line solve, and fewer warps where the sub-partitions of all SMs have more
-// than a warp each, for fewer instructions in all (a line takes 4 x 55 on four
-// warps, 2 x 82 on two); or what the tuner chose.  Timed at 385 x 129, three sweeps,
+// than a warp each, for fewer instructions in all (a line takes 4 x 59 on four
+// warps, 2 x 72 on two); or what the tuner chose.  Timed at 385 x 129, three sweeps,
 // the fastest is four warps at 1, 8 and 16 modes, two at 32, one at 64, as here.
 int plain_group(const tb_ctx* c, int n, int itera, int slots) {
     const int tuned = itera == 1 ? c->tune_pg1 : c->tune_pg3;

@@ -8,12 +8,15 @@
 // e^{+2 pi i k n / P}, zeroes components below 1e-14 and forces Im c_0 = 0.
 // Both directions are computed here as a length-P/2 complex FFT plus the
 // real-to-complex split, with exact twiddles from constant tables instead of
-// the reference's rotation recurrence: one thread per (i, j) grid line, and in
-// FP64 two at P = 128, where one line's values are more than a thread's registers.
+// the reference's rotation recurrence: one thread per (i, j) grid line, and two
+// in k_les and k_cvirt at P = 128, where one line's values are more than a thread's
+// registers.
 //
 // An FP64 warp instruction (comparisons included) holds its pipe for 64
 // cycles, so the FP64 transforms are written for their number: a butterfly is
-// six fused multiply-adds (twiddle w = m (1 + i r) or m (r + i), |r| <= 1), the
+// six fused multiply-adds (twiddle w = m (1 + i r) or m (r + i), |r| <= 1: the factored
+// butterfly of Linzer and Feig, "Implementation of efficient FFT algorithms on
+// fused multiply-add architectures", IEEE Trans. Signal Process. 41, 1993), the
 // split takes the modes k and P/2 - k together (12 in place of 28), its halves and
 // the 1/P are left to the caller's factors, and values are compared as integers.
 #include "tb_internal.h"

@@ -1,8 +1,8 @@
 // Launch shapes of the stage's batched kernels, picked per context by
 // timing the candidates on the context's own grid (CUDA events on its
-// stream): warps per block of the x-line solves, threads per block of the
-// y-line solves, and resident blocks per SM of the tensor-core passes of the
-// nonlinear terms.  The timed launches write only the stage's scratch fields
+// stream): lines per block of the x-line solves (half or all that fit), threads
+// per block of the y-line solves, resident blocks per SM of the tensor-core passes
+// of the nonlinear terms, and warps per line of the plain form's sweeps.  The timed launches write only the stage's scratch fields
 // (tmp), so the state is untouched.  Recorded step graphs are dropped, since
 // they hold the previous shapes.
 #include "tb_internal.h"
